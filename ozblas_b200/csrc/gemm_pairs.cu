@@ -18,16 +18,20 @@
 //   * The accumulators are handed over level by level: the last k step of a pair
 //     completes level 0 first, and the first k step of the next pair starts with
 //     level 0, so the epilogue's reads run under the MMAs of both.
-//     What is left is the shared-memory port: a 128 x 96 x 32 MMA reads 7 KB (57
-//     cycles at 128 B a clock, against 48 of math), and the TMA writes share it.
+//     A 128 x 96 x 32 MMA takes 56 cycles (7 KB of operands through the 128 B a
+//     clock shared-memory port; 48 of math), so a k step is 2016 cycles at best.
+//   * FP64 work stands still while MMAs stream, so the epilogue combines levels
+//     as integers (the kernel's epilogue says more).
+//   * The tiles' pairs are cut into equal shares, tiles included (pp_share).
 //   * Where a tile's lines have no slice at a level (the counts are those of the
 //     worst line of the whole operand), its pairs are skipped: they add zero.
-// Product kernel, before (one digit level at a time, pair buffer, 7-bit digits)
-// and now, one B200: 1024^3 plain, 16 pairs, 1076 -> 268 us; 3001 x 1999 x 2500
-// plain, 20 pairs, 4.08 (and 0.15 for the sum) -> 2.33 ms; 2048^3
-// <float,double,double>, 9 pairs, 1.73 (0.10) -> 0.81 ms.  Split to digit
-// planes (count, FP64 slices, digits in three passes before), 3001 lines of
-// 2500: 374 -> 54 us.
+// Product kernel, before (one digit level at a time, 7-bit digits) and now, one
+// B200: 1024^3 plain, 16 pairs, 1076 -> 145 us; 3001 x 1999 x 2500 plain, 20 pairs,
+// 4.08 -> 1.69 ms (and 0.15 for the sum, now inside); 2048^3
+// <float,double,double>, 9 pairs, 1.73 (0.10) -> 0.57 ms: 2.2, 3.0 and 2.6
+// POP/s of digit products, against 3.6 that the power limit leaves N = 96
+// MMAs.  Split to digit planes (count, FP64 slices, digits in three passes
+// before), 3001 lines of 2500: 374 -> 54 us.
 #include <cuda.h>
 
 #include "gemm_pairs.h"
@@ -340,8 +344,8 @@ template int pair_split<float>(cuozblasHandle_t *, int, int, const float *, int,
 
 // ---------------------------------------------------------------------------
 // Product kernel.  Persistent, one CTA per SM: warp 0 lane 0 loads digit
-// stages (digit d of A and of B for one k step) by TMA into a ring, warp 1
-// issues the MMAs, warps 4-11 read the accumulators.  Every wait is bounded.
+// stages (digit d of A and of B for one k step) by TMA into a ring, warps 1
+// and 2 issue the MMAs, warps 4-11 read the accumulators.  Every wait is bounded.
 // ---------------------------------------------------------------------------
 constexpr int kPpThreads = 384;
 constexpr uint32_t kPpRegLo = 40, kPpRegHi = 232;  // 4 x 40 + 8 x 232 = 12 x 168 registers at launch
@@ -352,7 +356,7 @@ struct PpShape {
     static constexpr int LV = 2 * D - 1;                // 5 x 96 = 480 or 7 x 64 = 448 tensor-memory columns
     static constexpr int TILE_A = 128 * 128, TILE_B = BN * 128, STAGE = TILE_A + TILE_B;
     static constexpr int ST = D == 3 ? 7 : 8;
-    static constexpr int SMEM = ST * STAGE + 1024 /*align*/ + 512 /*barriers*/ + 8 * (BN / 2) * 8 /*column scales*/;
+    static constexpr int SMEM = ST * STAGE + 1024 /*align*/ + 512 /*barriers*/ + 8 * (BN / 2) * 4 /*column exponents*/;
     static constexpr int CW = BN / 2;                   // columns per epilogue warp
 };
 
@@ -363,7 +367,8 @@ struct PpParams {
     const short *ea, *eb;
     double alpha, beta;
     void *C;
-    double *pbuf;
+    double *pbuf;        // kPairStore: the pair buffer; else the partial sums handed from one CTA to the next
+    unsigned *handed;    // per CTA and epilogue warp: its partial sums are in pbuf (zeroed before the launch)
     int *err;
 };
 
@@ -384,6 +389,13 @@ struct PairCursor {
         return true;
     }
 };
+// How many there are.
+__device__ __forceinline__ int pair_count(int LA, int LB, int maxlevel) {
+    int n = 0;
+    const int top = LA + LB - 2 < maxlevel ? LA + LB - 2 : maxlevel;
+    for (int ik = 0; ik <= top; ik++) n += min(ik, LA - 1) - max(0, ik - (LB - 1)) + 1;
+    return n;
+}
 __device__ __forceinline__ void pair_at(int p, int nA, int nB, int &a, int &b) {
     for (int ik = 0;; ik++) {
         const int lo = ik - (nB - 1) > 0 ? ik - (nB - 1) : 0, hi = ik < nA - 1 ? ik : nA - 1, c = hi - lo + 1;
@@ -396,38 +408,138 @@ __device__ __forceinline__ void pair_at(int p, int nA, int nB, int &a, int &b) {
     }
 }
 
-// Calls unit(tm, tn, ia, ib, pair) for the CTA's units in order, and
-// tile_end(tm, tn) after the last unit of a tile; both return false to stop.
-// FUSED: all pairs of tiles blockIdx.x, + gridDim.x, ...; else (pair, tile)
-// units dealt round robin, pair by pair, so the CTAs that run together share
-// the planes of one pair.
-template <bool FUSED, typename U, typename E>
-__device__ __forceinline__ void pp_units(const PpParams &p, U unit, E tile_end) {
-    const int ntiles = p.tiles_m * p.tiles_n;
-    auto coords = [&](int tile, int &tm, int &tn) {  // strips of tile rows, column-major inside a strip
-        const int per = p.strip * p.tiles_n, s = tile / per, w = tile - s * per;
-        const int rows = min(p.strip, p.tiles_m - s * p.strip);
-        tm = s * p.strip + w % rows;
-        tn = w / rows;
+// The CTA's share of a fused launch.  All (tile, pair) units in tile order are
+// cut into one equal range per CTA, so the last wave is full; a tile cut in two
+// is summed in order all the same: the CTA that holds its first pairs runs them
+// first and hands its partial sums on, the CTA that holds the rest runs them
+// last.  With ranges of at least a tile's pairs no tile meets three CTAs;
+// otherwise (and in launches of at most one tile per CTA) whole tiles are dealt
+// round robin.  first_tile / skip: where the range begins, last_tile / head:
+// where it ends (head pairs of last_tile; 0: it ends with a tile).
+struct PpShare {
+    int split, first_tile, skip, last_tile, head;
+};
+enum { kWhole = 0, kHead = 1, kTail = 2 };  // what a CTA runs of a tile
+
+__device__ __forceinline__ void pp_coords(const PpParams &p, int tile, int &tm, int &tn) {
+    // strips of tile rows, column-major inside a strip
+    const int per = p.strip * p.tiles_n, s = tile / per, w = tile - s * per;
+    const int rows = min(p.strip, p.tiles_m - s * p.strip);
+    tm = s * p.strip + w % rows;
+    tn = w / rows;
+}
+__device__ __forceinline__ void pp_levels(const PpParams &p, int tm, int tn, int &LA, int &LB) {
+    LA = p.la ? min(__ldg(p.la + tm), p.nA) : p.nA;
+    LB = p.lb ? min(__ldg(p.lb + tn), p.nB) : p.nB;
+}
+
+// Computed by the whole CTA before the roles part (scratch: one int per thread).
+__device__ __forceinline__ void pp_share(const PpParams &p, int *scratch, PpShare *out) {
+    const int ntiles = p.tiles_m * p.tiles_n, nt = blockDim.x, tid = threadIdx.x;
+    const int per = (ntiles + nt - 1) / nt, lo = min(ntiles, tid * per), hi = min(ntiles, lo + per);
+    auto count = [&](int tile) {
+        int tm, tn, LA, LB;
+        pp_coords(p, tile, tm, tn);
+        pp_levels(p, tm, tn, LA, LB);
+        return pair_count(LA, LB, p.maxlevel);
     };
+    int sum = 0, most = 0;
+    for (int t = lo; t < hi; t++) {
+        const int c = count(t);
+        sum += c;
+        most = max(most, c);
+    }
+    scratch[tid] = sum;
+    most = __reduce_max_sync(0xffffffffu, most);
+    __syncthreads();
+    if (tid == 0) {
+        int run = 0;
+        for (int i = 0; i < nt; i++) {
+            const int v = scratch[i];
+            scratch[i] = run;
+            run += v;
+        }
+        scratch[nt] = run;
+        scratch[nt + 1] = 0;
+        out->split = 0;
+    }
+    __syncthreads();
+    if ((tid & 31) == 0) atomicMax(&scratch[nt + 1], most);
+    __syncthreads();
+    const int64_t total = scratch[nt];
+    const int u0 = (int)(total * blockIdx.x / gridDim.x), u1 = (int)(total * (blockIdx.x + 1) / gridDim.x);
+    if (total / gridDim.x < scratch[nt + 1] || gridDim.x == 1) return;
+    int at = scratch[tid];
+    for (int t = lo; t < hi; t++) {
+        const int c = count(t);
+        if (u0 >= at && u0 < at + c) {
+            out->first_tile = t;
+            out->skip = u0 - at;
+        }
+        if (u1 >= at && u1 < at + c) {
+            out->last_tile = t;
+            out->head = u1 - at;
+        }
+        at += c;
+    }
+    if (tid == 0) {
+        out->split = 1;
+        if (u1 == total) {
+            out->last_tile = ntiles;
+            out->head = 0;
+        }
+    }
+}
+
+// Calls begin(kind), unit(tm, tn, ia, ib, pair) for the pairs in order and
+// end(tm, tn, kind) for every (part of a) tile of the CTA; false stops.
+// FUSED: the CTA's share; else (pair, tile) units dealt round robin, pair by
+// pair, so the CTAs that run together share the planes of one pair.
+template <bool FUSED, typename B, typename U, typename E>
+__device__ __forceinline__ void pp_units(const PpParams &p, const PpShare *sh, B begin, U unit, E end) {
+    const int ntiles = p.tiles_m * p.tiles_n;
     int tm, tn, a, b;
     if (FUSED) {
-        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-            coords(tile, tm, tn);
-            PairCursor cur(p.la ? min(__ldg(p.la + tm), p.nA) : p.nA, p.lb ? min(__ldg(p.lb + tn), p.nB) : p.nB, p.maxlevel);
-            int q = 0;
-            while (cur.next(a, b))
-                if (!unit(tm, tn, a, b, q++)) return;
-            if (!tile_end(tm, tn)) return;
+        const bool split = sh->split != 0;
+        const int first = sh->first_tile, last = sh->last_tile, skip = sh->skip, head = sh->head;
+        // split: step 0 the head of last_tile, then the whole tiles, then the tail of first_tile
+        const int whole0 = skip > 0 ? first + 1 : first, wholes = last - whole0;
+        const int steps = split ? wholes + 2 : (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+        for (int st = 0; st < steps; st++) {
+            int tile, kind = kWhole;
+            if (!split) {
+                tile = blockIdx.x + st * gridDim.x;
+            } else if (st == 0) {
+                if (head == 0) continue;
+                tile = last;
+                kind = kHead;
+            } else if (st <= wholes) {
+                tile = whole0 + st - 1;
+            } else {
+                if (skip == 0) continue;
+                tile = first;
+                kind = kTail;
+            }
+            pp_coords(p, tile, tm, tn);
+            int LA, LB;
+            pp_levels(p, tm, tn, LA, LB);
+            PairCursor cur(LA, LB, p.maxlevel);
+            if (!begin(kind)) return;
+            for (int q = 0; cur.next(a, b); q++) {
+                if (kind == kTail && q < skip) continue;
+                if (kind == kHead && q >= head) break;
+                if (!unit(tm, tn, a, b, q)) return;
+            }
+            if (!end(tm, tn, kind)) return;
         }
     } else {
         const int64_t total = (int64_t)ntiles * p.np;
         for (int64_t u = blockIdx.x; u < total; u += gridDim.x) {
             const int pr = (int)(u / ntiles);
-            coords((int)(u - (int64_t)pr * ntiles), tm, tn);
+            pp_coords(p, (int)(u - (int64_t)pr * ntiles), tm, tn);
             pair_at(pr, p.nA, p.nB, a, b);
             if ((p.la && a >= __ldg(p.la + tm)) || (p.lb && b >= __ldg(p.lb + tn))) continue;  // the pair is zero here
-            if (!unit(tm, tn, a, b, pr) || !tile_end(tm, tn)) return;
+            if (!unit(tm, tn, a, b, pr)) return;
         }
     }
 }
@@ -436,10 +548,123 @@ __device__ __forceinline__ double exp_scale(int e) {  // 2^e, or the line's 0 / 
     return e == kExpZero ? 0.0 : (e == kExpNaN ? __longlong_as_double(0x7ff8000000000000LL) : pow2(e));
 }
 
-// INT32 -> FP64 without the conversion unit (a quarter of the FP64 rate):
-// 2^52 + 2^31 + w built from its bits, minus the constant (exact).
-__device__ __forceinline__ double i2d(uint32_t w) {
-    return __hiloint2double(0x43300000, (int)(w ^ 0x80000000u)) - 4503601774854144.0;
+// |v| < 2^53 as a double in two FP64 additions: 2^84 + 2^63 + hi 2^32 and
+// 2^52 + lo built from their bits, minus the constants (every step exact).
+__device__ __forceinline__ double i2d(long long v) {
+    const int hi = (int)(v >> 32), lo = (int)v;
+    return (__hiloint2double(0x45300000, (int)((uint32_t)hi ^ 0x80000000u)) - 0x1.00000801p84) +
+           __hiloint2double(0x43300000, lo);
+}
+// The exact pair product V 2^e of a pair-buffer entry, 0 or NaN where either
+// line's exponent says so, rounded once if it is subnormal.
+__device__ __forceinline__ double pair_value(long long v, int bias, int ea, int eb) {
+    const bool spa = ea == kExpZero || ea == kExpNaN, spb = eb == kExpZero || eb == kExpNaN;
+    const double d = i2d(v);
+    if (spa || spb) return d * (spa ? exp_scale(ea) : 1.0) * (spb ? exp_scale(eb) : 1.0);
+    const int e = bias + ea + eb;
+    return e >= -1022 && e <= 969 ? d * pow2(e) : scale2(d, e);
+}
+
+// The <float,double,double> sum's term of c32, the product rounded to float:
+// (float)scalbn(c32, tauA + tauB).
+__device__ __forceinline__ double pair_term_sd(double c32, int ea, int eb) {
+    const bool spa = ea == kExpZero || ea == kExpNaN, spb = eb == kExpZero || eb == kExpNaN;
+    if (spa || spb) return c32 * (spa ? exp_scale(ea) : 1.0) * (spb ? exp_scale(eb) : 1.0);
+    return (double)__double2float_rn(scale2(c32, ea + eb));
+}
+
+// a[c] for a run-time c without indexing the register array.
+template <int N>
+__device__ __forceinline__ long long pick(const long long (&a)[N], int c) {
+    long long v = 0;
+#pragma unroll
+    for (int j = 0; j < N; j++)
+        if (j == c) v = a[j];
+    return v;
+}
+
+// MMA issuer PAR (0, 1): the digit levels of that parity, in their own
+// accumulators.  The whole warp walks the units and waits, one elected lane's
+// predicate issues: a branch on the lane index costs 80 cycles an MMA (the
+// compiler cannot tell that one thread issues), the predicated form 50; the
+// waits and commits of a k step add 1300 cycles, which two issuers overlap.
+template <int D, bool FUSED, int PAR>
+__device__ __forceinline__ void pp_issue(const PpParams &p, const PpShare *sh, uint8_t *smem, uint64_t *full, uint64_t *empty,
+                                         uint64_t *acc_full, uint64_t *acc_empty, uint64_t *drain, uint32_t tmem_base,
+                                         volatile int *abort_flag, uint64_t wait_ns) {
+    using S = PpShape<D>;
+    const uint32_t idesc = tc::idesc_i8(128, S::BN);
+    const bool lead = tc::elect_one();
+    const uint64_t desc0 = tc::smem_desc_k_sw128(tc::smem_u32(smem));  // + 16-byte units within the ring
+    uint32_t base = 0, bphase = 0;  // ring slot of the k step's first digit stage, and its phase
+    uint32_t units = 0;
+    bool ok = true, issued = false;
+    pp_units<FUSED>(
+        p, sh, [](int) { return true; },
+        [&](int, int, int, int, int) {
+            for (int kb = 0; kb < p.nkb; kb++) {
+                uint32_t sl[D], ph[D];
+                uint64_t ad[D];
+#pragma unroll
+                for (int d = 0; d < D; d++) {
+                    sl[d] = base + d;
+                    ph[d] = bphase;
+                    if (sl[d] >= (uint32_t)S::ST) {
+                        sl[d] -= S::ST;
+                        ph[d] ^= 1u;
+                    }
+                    ad[d] = desc0 + sl[d] * (uint32_t)(S::STAGE / 16);
+                }
+#pragma unroll
+                for (int L = PAR; L < S::LV; L += 2) {
+                    bool w = true;
+                    if (kb == 0 && units > 0)
+                        w = tc::mbar_wait(&acc_empty[L], (units - 1) & 1u, abort_flag, p.err, 2, wait_ns);
+                    // the digit stages that come into use with this level
+#pragma unroll
+                    for (int d = (L - 1 > 0 ? L - 1 : 0); d <= L; d++)
+                        if (d < D) w = w && tc::mbar_wait(&full[sl[d < D ? d : 0]], ph[d < D ? d : 0], abort_flag, p.err, 2, wait_ns);
+                    if (!__all_sync(0xffffffffu, w)) {
+                        ok = false;
+                        return false;
+                    }
+                    tc::fence_after_sync();
+                    const uint32_t tmem_d = tmem_base + (uint32_t)(L * S::BN);
+                    uint32_t accumulate = kb > 0;
+#pragma unroll
+                    for (int d = 0; d < D; d++) {
+                        const int e = L - d;
+                        if (e < 0 || e >= D) continue;
+#pragma unroll
+                        for (int kk = 0; kk < 4; kk++) {
+                            tc::mma_i8_if(lead, tmem_d, ad[d] + 2 * kk, ad[e] + S::TILE_A / 16 + 2 * kk, idesc,
+                                          accumulate);
+                            accumulate = 1;
+                        }
+                    }
+                    issued = true;
+                    // stage d serves levels d .. d + D - 1: released after this issuer's last of them
+#pragma unroll
+                    for (int d = 0; d < D; d++)
+                        if (L <= d + D - 1 && L + 2 > d + D - 1) tc::mma_commit_if(lead, &empty[sl[d]]);
+                    if (kb == p.nkb - 1) tc::mma_commit_if(lead, &acc_full[L]);
+                }
+                base += D;
+                if (base >= (uint32_t)S::ST) {
+                    base -= S::ST;
+                    bphase ^= 1u;
+                }
+            }
+            units++;
+            return true;
+        },
+        [](int, int, int) { return true; });
+    if (!ok && issued) {  // drain MMAs still in flight before tensor memory is released
+        tc::mma_commit_if(lead, drain);
+        const uint64_t t0 = tc::globaltimer();
+        while (!tc::mbar_try_wait(drain, 0) && tc::globaltimer() - t0 < 100000000ull) {
+        }
+    }
 }
 
 template <int D, int EPI>
@@ -452,27 +677,31 @@ __global__ void __launch_bounds__(kPpThreads, 1)
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t *full = (uint64_t *)(smem + S::ST * S::STAGE), *empty = full + S::ST;
     uint64_t *acc_full = empty + S::ST, *acc_empty = acc_full + S::LV, *drain = acc_empty + S::LV;
-    double *sbs = (double *)(smem + S::ST * S::STAGE + 512);
+    int *sbs = (int *)(smem + S::ST * S::STAGE + 512);
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
+    __shared__ PpShare share;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::ST; s++) {
             tc::mbar_init(&full[s], 1);
-            tc::mbar_init(&empty[s], 1);
+            tc::mbar_init(&empty[s], 2);
         }
         for (int l = 0; l < S::LV; l++) {
             tc::mbar_init(&acc_full[l], 1);
             tc::mbar_init(&acc_empty[l], 256);
         }
         tc::mbar_init(drain, 1);
+        tc::mbar_init(drain + 1, 1);
         abort_flag = 0;
         tc::fence_mbar_init();
         tc::prefetch_tmap(&tmA);
         tc::prefetch_tmap(&tmB);
     }
     if (warp == 1) tc::tmem_alloc(&tmem_slot, 512);
+    if (FUSED) pp_share(p, (int *)smem, &share);  // the ring is free until the roles begin
+    tc::fence_proxy_async();                      // and its first copies come after these writes
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -486,7 +715,7 @@ __global__ void __launch_bounds__(kPpThreads, 1)
             bool ok = hold_copies == 0;
             if (ok)
                 pp_units<FUSED>(
-                    p,
+                    p, &share, [](int) { return true; },
                     [&](int tm, int tn, int ia, int ib, int) {
                         for (int kb = 0; kb < p.nkb; kb++)
 #pragma unroll
@@ -508,196 +737,181 @@ __global__ void __launch_bounds__(kPpThreads, 1)
                             }
                         return true;
                     },
-                    [](int, int) { return true; });
+                    [](int, int, int) { return true; });
             if (!ok) tc::drain_copies(full, S::ST, issued, issued_phase);
         } else if (warp == 1) {
-            // ---------------------------------------------------------------- MMA issuer
-            // The whole warp walks the units and waits; one elected lane issues.  (A
-            // branch on the lane index instead costs 80 cycles an MMA against 57: the
-            // compiler then cannot tell that a single thread issues.)
-            const uint32_t idesc = tc::idesc_i8(128, S::BN);
-            uint32_t base = 0, bphase = 0;  // ring slot of the k step's first digit stage, and its phase
-            uint32_t units = 0;
-            bool ok = true, issued = false;
-            pp_units<FUSED>(
-                p,
-                [&](int, int, int, int, int) {
-                    for (int kb = 0; kb < p.nkb; kb++) {
-                        uint32_t sl[D], ph[D];
-#pragma unroll
-                        for (int d = 0; d < D; d++) {
-                            sl[d] = base + d;
-                            ph[d] = bphase;
-                            if (sl[d] >= (uint32_t)S::ST) {
-                                sl[d] -= S::ST;
-                                ph[d] ^= 1u;
-                            }
-                        }
-#pragma unroll
-                        for (int L = 0; L < S::LV; L++) {
-                            bool w = true;
-                            if (kb == 0 && units > 0)
-                                w = tc::mbar_wait(&acc_empty[L], (units - 1) & 1u, &abort_flag, p.err, 2, wait_ns);
-                            if (L < D)  // levels 0 .. D - 1 bring in one digit stage each
-                                w = w && tc::mbar_wait(&full[sl[L < D ? L : 0]], ph[L < D ? L : 0], &abort_flag, p.err, 2,
-                                                       wait_ns);
-                            if (!__all_sync(0xffffffffu, w)) {
-                                ok = false;
-                                return false;
-                            }
-                            tc::fence_after_sync();
-                            if (tc::elect_one()) {
-                                const uint32_t tmem_d = tmem_base + (uint32_t)(L * S::BN);
-                                uint32_t accumulate = kb > 0;
-#pragma unroll
-                                for (int d = 0; d < D; d++) {
-                                    const int e = L - d;
-                                    if (e < 0 || e >= D) continue;
-                                    const uint64_t ad = tc::smem_desc_k_sw128(tc::smem_u32(smem + sl[d] * S::STAGE));
-                                    const uint64_t bd =
-                                        tc::smem_desc_k_sw128(tc::smem_u32(smem + sl[e] * S::STAGE + S::TILE_A));
-#pragma unroll
-                                    for (int kk = 0; kk < 4; kk++) {
-                                        tc::mma_i8(tmem_d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
-                                        accumulate = 1;
-                                    }
-                                }
-                                // stage L - D + 1 serves levels up to L
-                                if (L >= D - 1) tc::mma_commit(&empty[sl[L >= D - 1 ? L - (D - 1) : 0]]);
-                                if (kb == p.nkb - 1) tc::mma_commit(&acc_full[L]);
-                            }
-                            __syncwarp();
-                            issued = true;
-                        }
-                        base += D;
-                        if (base >= (uint32_t)S::ST) {
-                            base -= S::ST;
-                            bphase ^= 1u;
-                        }
-                    }
-                    units++;
-                    return true;
-                },
-                [](int, int) { return true; });
-            if (!ok && issued) {  // drain MMAs still in flight before tensor memory is released
-                if (tc::elect_one()) tc::mma_commit(drain);
-                const uint64_t t0 = tc::globaltimer();
-                while (!tc::mbar_try_wait(drain, 0) && tc::globaltimer() - t0 < 100000000ull) {
-                }
-            }
+            pp_issue<D, FUSED, 0>(p, &share, smem, full, empty, acc_full, acc_empty, drain, tmem_base, &abort_flag, wait_ns);
+        } else if (warp == 2) {
+            pp_issue<D, FUSED, 1>(p, &share, smem, full, empty, acc_full, acc_empty, drain + 1, tmem_base, &abort_flag, wait_ns);
         }
     } else {
         tc::reg_alloc<kPpRegHi>();
         // ---------------------------------------------------------------- epilogue
-        constexpr int CW = S::CW;
+        // FP64 instructions make next to no progress while MMAs stream (measured: 48
+        // columns' conversions and FMAs 720 cycles alone, 3900 beside N = 96 MMAs, which
+        // they do not slow), integer ones run beside them.  So the levels are combined
+        // as 64-bit integers, and the three FP64 operations per output that the ordered
+        // sum needs run between the read of the last accumulator and its release: the
+        // MMAs then wait for that accumulator, which opens the window they run in.
+        constexpr int CW = S::CW, LV = S::LV;
         const int q = warp & 3, half = (warp - 4) >> 2;
         const int row = q * 32 + lane;
         const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16) + half * CW;
-        double *sb = sbs + (warp - 4) * CW;  // this warp's column scales
-        const double rad = p.radix == 8 ? 256.0 : 128.0;
+        int *sb = sbs + (warp - 4) * CW;  // this warp's column exponents, shifted to the exponent field
+        constexpr int kShift = EPI == kPairSd ? 23 : 20, kOne = EPI == kPairSd ? 127 : 1023;
+        constexpr int kLo = EPI == kPairSd ? -126 : -1022, kHi = EPI == kPairSd ? 73 : 969;
+        constexpr int kColZero = -0x7f000000;  // plus any row term below: negative, clamped to a zero scale
         uint32_t units = 0;
-        double acc[CW];
+        long long acc[CW];
         typename std::conditional<EPI == kPairSd, float, double>::type t[FUSED ? CW : 1];
 #pragma unroll
         for (int c = 0; c < (FUSED ? CW : 1); c++) t[c] = 0;
         pp_units<FUSED>(
-            p,
+            p, &share,
+            [&](int kind) {
+                if (FUSED && kind == kTail) {  // go on from the previous CTA's sums (it ran its part first)
+                    bool ok = true;
+                    if (lane == 0) {
+                        const unsigned *f = p.handed + (blockIdx.x - 1) * 8 + (warp - 4);
+                        const uint64_t t0 = tc::globaltimer();
+                        unsigned v;
+                        for (;;) {
+                            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
+                            if (v != 0) break;
+                            if (abort_flag || tc::globaltimer() - t0 > wait_ns) {
+                                abort_flag = 1;
+                                atomicExch(p.err, 4);
+                                ok = false;
+                                break;
+                            }
+                        }
+                    }
+                    if (!__all_sync(0xffffffffu, ok)) return false;
+                    __syncwarp();
+                    const auto *from = reinterpret_cast<const decltype(&t[0])>(p.pbuf) +
+                                       (size_t)(blockIdx.x - 1) * (128 * S::BN) + (size_t)(half * CW) * 128 + row;
+#pragma unroll
+                    for (int c = 0; c < (FUSED ? CW : 1); c++) t[c] = __ldcg(from + c * 128);
+                }
+                return true;
+            },
             [&](int tm, int tn, int ia, int ib, int pr) {
                 const int gr = tm * 128 + row, gc0 = tn * S::BN + half * CW;
                 // the scales do not depend on the MMAs: loaded before the waits
-                int ea = p.ea && gr < p.m ? (int)p.ea[(size_t)ia * p.m + gr] : 0;
-                int ebmin = 0x7fffffff, ebmax = -0x7fffffff;
-                __syncwarp();
+                int ea = 0;
+                bool fast = false;
+                const short *ebr = nullptr;
+                if (FUSED) {
+                    ea = gr < p.m ? (int)p.ea[(size_t)ia * p.m + gr] : 0;
+                    ebr = p.eb + (size_t)ib * p.n + gc0;
+                    int ebmin = 0x7fffffff, ebmax = -0x7fffffff;
+                    bool nan = false;
+                    __syncwarp();
 #pragma unroll
-                for (int c = lane; c < CW; c += 32) {
-                    const int e = p.eb && gc0 + c < p.n ? (int)p.eb[(size_t)ib * p.n + gc0 + c] : 0;
-                    sb[c] = exp_scale(e);
-                    if (e != kExpZero && e != kExpNaN) {
-                        ebmin = min(ebmin, e);
-                        ebmax = max(ebmax, e);
+                    for (int c = lane; c < CW; c += 32) {
+                        const int e = gc0 + c < p.n ? (int)ebr[c] : 0;
+                        sb[c] = e == kExpZero ? kColZero : (int)((uint32_t)e << kShift);
+                        nan |= e == kExpNaN;
+                        if (e != kExpZero) {
+                            ebmin = min(ebmin, e);
+                            ebmax = max(ebmax, e);
+                        }
                     }
+                    ebmin = __reduce_min_sync(0xffffffffu, ebmin);
+                    ebmax = __reduce_max_sync(0xffffffffu, ebmax);
+                    nan = __any_sync(0xffffffffu, nan);
+                    // V 2^(bias + ea + eb) is an exact normal number for every column
+                    fast = !nan && ea != kExpNaN && ea != kExpZero && p.bias + ea >= kLo && p.bias + ea <= kHi &&
+                           (ebmin > ebmax || (p.bias + ea + ebmin >= kLo && p.bias + ea + ebmax <= kHi));
+                    __syncwarp();
                 }
-                ebmin = __reduce_min_sync(0xffffffffu, ebmin);
-                ebmax = __reduce_max_sync(0xffffffffu, ebmax);
-                const bool special = ea == kExpZero || ea == kExpNaN;
-                // V * 2^(bias + ea) and its product with 2^eb are exact normal numbers for every column
-                constexpr int kLo = EPI == kPairSd ? -126 : -1022, kHi = EPI == kPairSd ? 73 : 969;
-                const bool fast = special || ebmin > ebmax ||
-                                  (p.bias + ea >= kLo && p.bias + ea <= kHi && p.bias + ea + ebmin >= kLo &&
-                                   p.bias + ea + ebmax <= kHi && ebmin >= kLo && ebmax <= kHi + 53);
-                const double sa = special ? exp_scale(ea) : pow2(p.bias + ea);
 #pragma unroll
-                for (int L = 0; L < S::LV; L++) {
+                for (int L = 0; L < LV; L++) {
                     // the lanes agree before the warp-wide loads
                     if (!__all_sync(0xffffffffu,
                                     tc::mbar_wait(&acc_full[L], units & 1u, &abort_flag, p.err, 3, wait_ns)))
                         return false;
                     tc::fence_after_sync();
+                    const int sh = p.radix * (LV - 1 - L);
 #pragma unroll
                     for (int c0 = 0; c0 < CW; c0 += 16) {
                         uint32_t v[16];
                         tc::tmem_ld_32x32b_x16(lane_base + L * S::BN + c0, v);
                         tc::tmem_ld_wait();
 #pragma unroll
-                        for (int c = 0; c < 16; c++) acc[c0 + c] = L == 0 ? i2d(v[c]) : fma(acc[c0 + c], rad, i2d(v[c]));
+                        for (int c = 0; c < 16; c++) {
+                            const long long w = (long long)(int)v[c];
+                            if (L == 0)
+                                acc[c0 + c] = w << sh;
+                            else if (LV - 1 - L > 3)  // weights that leave 32 bits
+                                acc[c0 + c] += w << sh;
+                            else
+                                acc[c0 + c] += w * (long long)(1 << sh);
+                        }
                     }
                     tc::fence_before_sync();
-                    tc::mbar_arrive(&acc_empty[L]);
+                    if (!FUSED || L < LV - 1) tc::mbar_arrive(&acc_empty[L]);
                 }
                 units++;
-                __syncwarp();
                 if constexpr (EPI == kPairStore) {
                     if (gr < p.m) {
-                        double *o = p.pbuf + ((size_t)pr * p.n + gc0) * p.m + gr;
+                        long long *o = reinterpret_cast<long long *>(p.pbuf) + ((size_t)pr * p.n + gc0) * p.m + gr;
                         const int nc = min(CW, p.n - gc0);
-                        const short *ebr = p.eb ? p.eb + (size_t)ib * p.n + gc0 : nullptr;
 #pragma unroll
                         for (int c = 0; c < CW; c++)
-                            if (c < nc) {
-                                if (fast) {
-                                    o[(size_t)c * p.m] = (acc[c] * sa) * sb[c];
-                                } else {
-                                    const int e = ebr ? (int)ebr[c] : 0;
-                                    o[(size_t)c * p.m] = e == kExpZero || e == kExpNaN ? acc[c] * exp_scale(e)
-                                                                                       : scale2(acc[c], p.bias + ea + e);
-                                }
-                            }
-                    }
-                } else if constexpr (EPI == kPairFsum) {
-                    // the product is exact, so one fma rounds as the addition of the product
-                    if (fast) {
-#pragma unroll
-                        for (int c = 0; c < CW; c++) t[c] = fma(acc[c] * sa, sb[c], t[c]);
-                    } else {
-                        const short *ebr = p.eb + (size_t)ib * p.n;
-#pragma unroll
-                        for (int c = 0; c < CW; c++) {
-                            const int e = gc0 + c < p.n ? (int)ebr[gc0 + c] : 0;
-                            t[c] = __dadd_rn(t[c], e == kExpZero || e == kExpNaN ? acc[c] * exp_scale(e)
-                                                                                : scale2(acc[c], p.bias + ea + e));
-                        }
+                            if (c < nc) o[(size_t)c * p.m] = acc[c];
                     }
                 } else {
-                    const float saf = (float)sa;
                     if (fast) {
-#pragma unroll
-                        for (int c = 0; c < CW; c++)
-                            t[c] = fmaf(__double2float_rn(acc[c]) * saf, (float)sb[c], t[c]);
-                    } else {
-                        const short *ebr = p.eb + (size_t)ib * p.n;
+                        // the product is exact, so one fma rounds as the addition of the product
+                        const int rowhi = (p.bias + ea + kOne) * (1 << kShift);
 #pragma unroll
                         for (int c = 0; c < CW; c++) {
-                            const int e = gc0 + c < p.n ? (int)ebr[gc0 + c] : 0;
-                            const double c32 = (double)__double2float_rn(acc[c] * pow2(p.bias));
-                            t[c] = __fadd_rn(t[c], __double2float_rn(e == kExpZero || e == kExpNaN ? c32 * exp_scale(e)
-                                                                                                  : scale2(c32, ea + e)));
+                            const int sc = max(rowhi + sb[c], 0);
+                            if constexpr (EPI == kPairSd)
+                                t[c] = fmaf(__ll2float_rn(acc[c]), __int_as_float(sc), t[c]);
+                            else
+                                t[c] = fma(i2d(acc[c]), __hiloint2double(sc, 0), t[c]);
+                        }
+                    } else if (ea != kExpZero) {  // exponents at the ends of the range, NaN lines
+#pragma unroll 1
+                        for (int c = 0; c < CW; c++) {
+                            const int e = gc0 + c < p.n ? (int)ebr[c] : 0;
+                            double add;
+                            if constexpr (EPI == kPairSd)
+                                add = pair_term_sd((double)__ll2float_rn(pick(acc, c)) * pow2(p.bias), ea, e);
+                            else
+                                add = pair_value(pick(acc, c), p.bias, ea, e);
+#pragma unroll
+                            for (int j = 0; j < CW; j++)
+                                if (j == c) {
+                                    if constexpr (EPI == kPairSd)
+                                        t[j] = __fadd_rn(t[j], (float)add);
+                                    else
+                                        t[j] = __dadd_rn(t[j], add);
+                                }
                         }
                     }
+                    tc::mbar_arrive(&acc_empty[LV - 1]);
                 }
                 return true;
             },
-            [&](int tm, int tn) {
-                if (FUSED) {
+            [&](int tm, int tn, int kind) {
+                if (FUSED && kind == kHead) {
+                    auto *to = reinterpret_cast<decltype(&t[0])>(p.pbuf) + (size_t)blockIdx.x * (128 * S::BN) +
+                               (size_t)(half * CW) * 128 + row;
+#pragma unroll
+                    for (int c = 0; c < (FUSED ? CW : 1); c++) {
+                        __stcg(to + c * 128, t[c]);
+                        t[c] = 0;
+                    }
+                    __syncwarp();
+                    if (lane == 0) {
+                        __threadfence();
+                        asm volatile("st.release.gpu.global.u32 [%0], 1;" ::"l"(p.handed + blockIdx.x * 8 + (warp - 4))
+                                     : "memory");
+                    }
+                } else if (FUSED) {
                     const int gr = tm * 128 + row, gc0 = tn * S::BN + half * CW;
                     if (gr < p.m) {
 #pragma unroll
@@ -742,11 +956,12 @@ static int transpose_t(cuozblasHandle_t *h, int rows, int cols, const float *A, 
 bool pair_fuse_sum(int m, int n, int k_pad, int np, int D) {
     const int64_t tiles = (int64_t)((m + 127) / 128) * ((n + pair_tile_b(D) - 1) / pair_tile_b(D));
     const int sms = sm_count();
-    // microseconds: a pair's MMAs over 128 k (D^2 products of 4 MMAs at about 56 cycles) and its
-    // hand-over, against the pair buffer written and read back at about 3 TB/s
-    const double pair_us = (double)(k_pad / 128) * D * D * 4 * 56e-3 / 1.9 + 1.0;
-    const double fused = (double)((tiles + sms - 1) / sms) * np * pair_us;
-    const double split = (double)((tiles * np + sms - 1) / sms) * pair_us + 16.0 * np * (double)m * n / 3e6 + 4.0;
+    // Microseconds, as measured: a pair's 128 k take 1.35 (D = 3) and its hand-over 2 (1.5 more with the
+    // sum in the epilogue).  Fused, every CTA runs an equal share, but no tile on three CTAs (pp_share).
+    const double pair_us = (double)(k_pad / 128) * 0.15 * D * D + 2.0;
+    const int64_t share = (tiles * np + sms - 1) / sms;
+    const double fused = (double)(share > np ? share : np) * (pair_us + 1.5);
+    const double split = (double)share * pair_us + 8.0 * np * (double)m * n / 5e6 + 4.0;
     return fused <= split;
 }
 
@@ -783,12 +998,28 @@ int pair_products(cuozblasHandle_t *h, const PairDigits &pd, const PairOperand &
     OZB_TRY(make_map_planes(&tmB, B.dig, c.k_pad, c.n, (uint64_t)c.nB * pd.D, bn));
     const int64_t units = (int64_t)p.tiles_m * p.tiles_n * (c.epi == kPairStore ? p.np : 1);
     const int grid = (int)(units < sm_count() ? units : sm_count());
+    p.handed = nullptr;
+    if (c.epi != kPairStore) {
+        p.pbuf = c.pbuf;
+        p.handed = reinterpret_cast<unsigned *>(c.pbuf + (size_t)sm_count() * 128 * bn);
+        OZB_CHECK(cudaMemsetAsync(p.handed, 0, sizeof(unsigned) * 8 * sm_count(), st->stream));
+    }
+    // the fused CTAs wait for one another: a cooperative launch
     auto go = [&](auto kern, int smem, std::atomic<uint64_t> &done) -> cudaError_t {
-        const cudaError_t e = smem_optin((const void *)kern, smem, done);
+        cudaError_t e = smem_optin((const void *)kern, smem, done);
         if (e != cudaSuccess) return e;
         counted(h);
-        kern<<<grid, kPpThreads, smem, st->stream>>>(tmA, tmB, p, i8_test_wait_ns(), i8_test_hold_copies());
-        return cudaGetLastError();
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(kPpThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st->stream;
+        cfg.attrs = &at;
+        cfg.numAttrs = c.epi == kPairStore ? 0 : 1;
+        return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p, i8_test_wait_ns(), i8_test_hold_copies());
     };
     static std::atomic<uint64_t> done[6];
     if (pd.D == 3) {
@@ -816,7 +1047,7 @@ int pair_status(cuozblasHandle_t *h) {
     return CUOZBLAS_STATUS_SUCCESS;
 }
 
-// The ordered sum of a pair buffer pbuf[p][col][row] of exact products: FSum
+// The ordered sum of a pair buffer pbuf[p][col][row] of exact integer products V: FSum
 // in pair order, or NearSum (which overwrites the buffer); FLOATS: the
 // <float,double,double> sum, t += (float)scalbn((float)P, tauA + tauB).  One
 // thread per output, the loads of 4 pairs in flight; pairs that the product
@@ -826,7 +1057,7 @@ __global__ void __launch_bounds__(256) k_pair_sum(int m, int n, int nA, int nB, 
                                                   double *__restrict__ pbuf, const int *__restrict__ la,
                                                   const int *__restrict__ lb, int tile_b,
                                                   const short *__restrict__ ea, const short *__restrict__ eb,
-                                                  int sum_mode, double alpha, double beta, void *__restrict__ Cv,
+                                                  int bias, int sum_mode, double alpha, double beta, void *__restrict__ Cv,
                                                   int ldc) {
     const int rb = (m + 255) / 256, col = blockIdx.x / rb, row = (blockIdx.x - col * rb) * 256 + threadIdx.x;
     if (row >= m) return;
@@ -834,6 +1065,11 @@ __global__ void __launch_bounds__(256) k_pair_sum(int m, int n, int nA, int nB, 
     double *pe = pbuf + (size_t)col * m + row;
     const size_t at = (size_t)col * ldc + row;
     if (!FLOATS && sum_mode == 1) {
+        int p = 0;
+        for_each_pair(nA, nB, maxlevel, [&](int ia, int ib) {
+            double *v = pe + (size_t)p++ * count;
+            *v = pair_value(__double_as_longlong(*v), bias, ea[(size_t)ia * m + row], eb[(size_t)ib * n + col]);
+        });
         double *cp = reinterpret_cast<double *>(Cv) + at;
         *cp = fma(alpha, nearsum(np, pe, (int64_t)count), beta * *cp);
         return;
@@ -847,17 +1083,12 @@ __global__ void __launch_bounds__(256) k_pair_sum(int m, int n, int nA, int nB, 
         const int from = max(lo, ik - (LB - 1)), to = min(hi, LA - 1);  // the pairs in use
 #pragma unroll 4
         for (int ia = from; ia <= to; ia++) {
-            const double v = __ldcs(pe + (size_t)(p + ia - lo) * count);
-            if (FLOATS) {
-                const int a = ea[(size_t)ia * m + row], b = eb[(size_t)(ik - ia) * n + col];
-                const double c32 = (double)__double2float_rn(v);
-                const bool special = a == kExpZero || a == kExpNaN || b == kExpZero || b == kExpNaN;
-                tf = __fadd_rn(tf, __double2float_rn(special ? c32 * (a == kExpZero || a == kExpNaN ? exp_scale(a) : 1.0) *
-                                                                   (b == kExpZero || b == kExpNaN ? exp_scale(b) : 1.0)
-                                                             : scale2(c32, a + b)));
-            } else {
-                t += v;
-            }
+            const long long v = __double_as_longlong(__ldcs(pe + (size_t)(p + ia - lo) * count));
+            const int a = ea[(size_t)ia * m + row], b = __ldg(eb + (size_t)(ik - ia) * n + col);
+            if (FLOATS)
+                tf = __fadd_rn(tf, (float)pair_term_sd((double)__ll2float_rn(v) * pow2(bias), a, b));
+            else
+                t = __dadd_rn(t, pair_value(v, bias, a, b));
         }
         p += hi - lo + 1;
     }
@@ -987,19 +1218,24 @@ int gemm_pairs_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
             ar.release(mark0);
             return CUOZBLAS_STATUS_SUCCESS;
         }
+        ar.ok = true;
     }
     if (c.epi == kPairStore) {
         PairOperand a = op[0], b = op[1];
         if (near) a.tile_lev = b.tile_lev = nullptr;  // NearSum reads every term
-        if (kFloats) a.exps = b.exps = nullptr;       // the float sum scales after rounding
         OZB_TRY(pair_products(h, pd, a, b, c));
         ev_record(h, 3);
         counted(h);
         k_pair_sum<kFloats><<<(unsigned)((int64_t)((m + 255) / 256) * n), 256, 0, st->stream>>>(
             m, n, c.nA, c.nB, c.maxlevel, npu, c.pbuf, a.tile_lev, b.tile_lev, tile[1], op[0].exps, op[1].exps,
-            h->sumMode, alpha, beta, C, ldc);
+            c.bias, h->sumMode, alpha, beta, C, ldc);
         OZB_CHECK(cudaGetLastError());
     } else {
+        c.pbuf = ar.take<double>(pair_handover_doubles(pd.D));
+        if (!ar.ok) {
+            ar.release(mark0);
+            return CUOZBLAS_STATUS_SUCCESS;
+        }
         OZB_TRY(pair_products(h, pd, op[0], op[1], c));
         ev_record(h, 3);  // the ordered sum runs inside the product kernel
     }

@@ -34,7 +34,7 @@ constexpr short kExpZero = -32768, kExpNaN = 32767;
 
 // Where the pair products go.
 enum PairEpi {
-    kPairStore = 0,  // pbuf[pair][col][row] = 2^(bias + tauA + tauB) sum q q (without exps: 2^bias sum q q)
+    kPairStore = 0,  // pbuf[pair][col][row] = sum q q as a 64-bit integer (|.| < 2^53)
     kPairFsum = 1,   // C = fma(alpha, t, beta C), t the FP64 sum of the products in pair order
     kPairSd = 2,     // the <float,double,double> sum: each product rounded to float, scaled, added in float
 };
@@ -58,13 +58,16 @@ int pair_split(cuozblasHandle_t *h, int k, int k_pad, const T *X, int ldx, int r
 // The products of every pair (ia, ib), ia + ib <= maxlevel, ia < nA, ib < nB.
 // A bounded wait that runs out is reported by pair_status.
 struct PairCall {
-    int m, n, k_pad, nA, nB, maxlevel, bias;
+    int m, n, k_pad, nA, nB, maxlevel;
+    int bias = 0;  // a pair product is 2^(bias + tauA + tauB) sum q q (kPairStore: for the sum that reads pbuf)
     PairEpi epi;
     double alpha = 1.0, beta = 0.0;
     void *C = nullptr;
     int ldc = 0;
-    double *pbuf = nullptr;
+    double *pbuf = nullptr;  // kPairStore: np m n entries, else pair_handover_doubles
 };
+// Partial sums that one CTA of a fused launch hands to the next, and their flags.
+inline uint64_t pair_handover_doubles(int D) { return (uint64_t)sm_count() * (128 * pair_tile_b(D) + 4); }
 int pair_products(cuozblasHandle_t *h, const PairDigits &pd, const PairOperand &A, const PairOperand &B,
                   const PairCall &c);
 constexpr int kPairErrInt = 2;  // the kernel's error word among the handle's device ints (zeroed by the caller)
@@ -77,9 +80,9 @@ template <typename T>
 int gemm_pairs_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, double alpha, const T *A, int lda,
                     const T *B, int ldb, double beta, T *C, int ldc, int fastMode, int rho, bool *done);
 
-// True when the ordered sum should run in the product kernel's epilogue (one
-// CTA then runs all pairs of a tile), false when the pairs of a tile should be
-// spread over CTAs through a pair buffer.
+// True when the ordered sum should run in the product kernel's epilogue (at
+// most two CTAs then share a tile's pairs), false when they should be spread
+// over CTAs through a pair buffer: few tiles, short k.
 bool pair_fuse_sum(int m, int n, int k_pad, int np, int D);
 
 }  // namespace ozb

@@ -150,7 +150,9 @@ __global__ void __launch_bounds__(256) k_split_lines_q_digits(int k, int nl, con
 
 // General GEMM sum: element e = col * m + row of a block of nc columns from
 // c0; pbuf[p * count + e] exact FP64 products of pair dp[p].
-__global__ void k_sum_pairs_q(int m, int n, int64_t count, int c0, int np, const double *__restrict__ pbuf,
+// INT: the entries are 64-bit integers V below 2^53, the product V 2^vbias.
+template <bool INT>
+__global__ void k_sum_pairs_q(int m, int n, int64_t count, int c0, int np, const double *__restrict__ pbuf, int vbias,
                               const int2 *__restrict__ dp, const short *__restrict__ Ea,
                               const short *__restrict__ Eb, Q128 alpha, Q128 beta, Q128 *__restrict__ C, int ldc) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -160,7 +162,8 @@ __global__ void k_sum_pairs_q(int m, int n, int64_t count, int c0, int np, const
     for (int p = 0; p < np; p++) {
         const int2 pr = dp[p];
         const int sc = Ea[(size_t)pr.x * m + row] + Eb[(size_t)pr.y * n + col];
-        t = q_add(t, q_from_double_scaled(pbuf[(size_t)p * count + e], sc));
+        const double v = pbuf[(size_t)p * count + e];
+        t = q_add(t, INT ? q_from_double_scaled((double)__double_as_longlong(v), sc + vbias) : q_from_double_scaled(v, sc));
     }
     Q128 *cp = C + (size_t)col * ldc + row;
     q_st(cp, q_fma(alpha, t, q_mul(beta, q_ld(cp))));
@@ -327,7 +330,7 @@ int gemm_q_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, cons
             double *pbuf = pc.pbuf;
             const int64_t count = (int64_t)m * n;
             counted(h);
-            k_sum_pairs_q<<<(unsigned)((count + 255) / 256), 256, 0, st->stream>>>(m, n, count, 0, np, pbuf, dp, Ea,
+            k_sum_pairs_q<true><<<(unsigned)((count + 255) / 256), 256, 0, st->stream>>>(m, n, count, 0, np, pbuf, pc.bias, dp, Ea,
                                                                                   Eb, alpha, beta, C, ldc);
             OZB_CHECK(cudaGetLastError());
             ev_record(h, 3);
@@ -365,7 +368,7 @@ int gemm_q_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, cons
         OZB_TRY(gemm_pairs_store(h, m, nc, n, ldk, Sa, Sb + (size_t)c0 * ldk, dp, np, pbuf));
         const int64_t count = (int64_t)m * nc;
         counted(h);
-        k_sum_pairs_q<<<(unsigned)((count + 255) / 256), 256, 0, st->stream>>>(m, n, count, (int)c0, np, pbuf, dp, Ea,
+        k_sum_pairs_q<false><<<(unsigned)((count + 255) / 256), 256, 0, st->stream>>>(m, n, count, (int)c0, np, pbuf, 0, dp, Ea,
                                                                               Eb, alpha, beta, C, ldc);
         OZB_CHECK(cudaGetLastError());
     }

@@ -151,8 +151,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// True in one lane of a converged warp.  The compiler recognises the pattern
-// and issues the guarded tcgen05 instructions from uniform registers.
+// True in one lane of a converged warp.
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile(
@@ -178,6 +177,27 @@ __device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t
 __device__ __forceinline__ void mma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
+}
+
+// The same two for a converged warp in which one lane's `lead` is true: the
+// predicate is on the instruction, so there is no branch around it.
+__device__ __forceinline__ void mma_i8_if(bool lead, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                          uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"((uint32_t)lead)
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit_if(bool lead, uint64_t *bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(smem_u32(bar)),
+        "r"((uint32_t)lead)
+        : "memory");
 }
 
 // 32 lanes x 32 consecutive 32-bit columns: thread (lane l) gets row l of the
