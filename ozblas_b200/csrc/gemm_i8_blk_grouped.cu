@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(KB_THREADS, 1)
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int t_begin = p.cta_begin[blockIdx.x], t_end = p.cta_begin[blockIdx.x + 1];
 
     if (threadIdx.x == 0) {
@@ -189,19 +189,26 @@ __global__ void __launch_bounds__(KB_THREADS, 1)
         // Two threads issue, each the pairs of alternate levels of a block
         // (its own accumulators), so one thread's waits and commits between A
         // planes overlap the other's queued MMAs.  Both wait for every plane,
-        // and every release and accumulator barrier counts both.
-        if (lane == 0) {
+        // and every release and accumulator barrier counts both.  The whole warp
+        // walks the schedule and one elected lane's predicate issues: under a
+        // branch on the lane index an MMA took 80 cycles, 64 is the tensor rate.
+        // (256 uneven problems, full pairs: the call 14.1 -> 11.4 ms.)
+        {
             const int issuer = warp - 1;
             const uint32_t idesc = tc::idesc_i8(KB_BM, KB_BN);
             uint32_t na = 0, nb = 0, nbw = 0;  // A planes consumed, B planes retired, B planes waited for
             uint32_t step_no = 0;
+            const bool lead = tc::elect_one();
+            auto wait = [&](uint64_t *b, uint32_t parity) {
+                return __all_sync(0xffffffffu, tc::mbar_wait(b, parity, &abort_flag, p.err, 2, wait_ns)) != 0;
+            };
             bool ok = true, issued = false;
             for (int tile = t_begin; tile < t_end && ok; tile++) {
                 const BlkCtx c = blk_ctx(p, tile);
                 for (int st = 0; st < c.n_steps && ok; st++, step_no++) {
                     const BlkStep sp = c.steps[st];
                     // the epilogue has read the accumulators of the previous step
-                    if (step_no > 0 && !tc::mbar_wait(acc_empty, (step_no - 1) & 1u, &abort_flag, p.err, 2, wait_ns)) {
+                    if (step_no > 0 && !wait(acc_empty, (step_no - 1) & 1u)) {
                         ok = false;
                         break;
                     }
@@ -219,14 +226,13 @@ __global__ void __launch_bounds__(KB_THREADS, 1)
                             const int wlo = blk_wlo(sp.L0, ia), whi = blk_whi(sp.L1, ia, c.nB);
                             // wait for A_ia and the B planes down to ib = wlo
                             const uint32_t sa = na % KB_RA;
-                            if (!tc::mbar_wait(&fullA[sa], (na / KB_RA) & 1u, &abort_flag, p.err, 2, wait_ns)) {
+                            if (!wait(&fullA[sa], (na / KB_RA) & 1u)) {
                                 ok = false;
                                 break;
                             }
                             const uint32_t need = b0 + (uint32_t)(whi0 - wlo) + 1u;
                             while (nbw < need && ok) {
-                                if (!tc::mbar_wait(&fullB[nbw % KB_RB], (nbw / KB_RB) & 1u, &abort_flag, p.err, 2,
-                                                   wait_ns))
+                                if (!wait(&fullB[nbw % KB_RB], (nbw / KB_RB) & 1u))
                                     ok = false;
                                 else
                                     nbw++;
@@ -244,12 +250,12 @@ __global__ void __launch_bounds__(KB_THREADS, 1)
                                 if (nkk == KB_BK / 32) {
 #pragma unroll
                                     for (int kk = 0; kk < KB_BK / 32; kk++) {
-                                        tc::mma_i8(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
+                                        tc::mma_i8_if(lead, tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
                                         accumulate = 1;
                                     }
                                 } else {
                                     for (int kk = 0; kk < nkk; kk++) {
-                                        tc::mma_i8(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
+                                        tc::mma_i8_if(lead, tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
                                         accumulate = 1;
                                     }
                                 }
@@ -257,24 +263,24 @@ __global__ void __launch_bounds__(KB_THREADS, 1)
                                 issued = true;
                             }
                             // A_ia is done; B_whi retires when the next ia no longer reaches it
-                            tc::mma_commit(&emptyA[sa]);
+                            tc::mma_commit_if(lead, &emptyA[sa]);
                             na++;
                             const int nwhi = ia < ia_hi ? blk_whi(sp.L1, ia + 1, c.nB) : -1;
                             const int nwlo = ia < ia_hi ? blk_wlo(sp.L0, ia + 1) : 0x7fffffff;
                             // retire (FIFO: largest ib first) every B plane above the next window
                             for (int ib = whi; ib >= wlo && ib > nwhi; ib--) {
                                 (void)nwlo;
-                                tc::mma_commit(&emptyB[nb % KB_RB]);
+                                tc::mma_commit_if(lead, &emptyB[nb % KB_RB]);
                                 nb++;
                             }
                         }
                     }
                     if (!ok) break;
-                    tc::mma_commit(acc_full);  // this step's accumulators are complete
+                    tc::mma_commit_if(lead, acc_full);  // this step's accumulators are complete
                 }
             }
             if (!ok && issued) {  // drain MMAs still in flight before tensor memory is released
-                tc::mma_commit(drain + issuer);
+                tc::mma_commit_if(lead, drain + issuer);
                 const uint64_t t0 = tc::globaltimer();
                 while (!tc::mbar_try_wait(drain + issuer, 0) && tc::globaltimer() - t0 < 100000000ull) {
                 }
