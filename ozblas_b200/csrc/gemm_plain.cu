@@ -448,6 +448,22 @@ int gemm_plain_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
         }
         ev_record(h, 0);
     }
+    // GEMV 't' (lines contiguous): split and products in registers
+    if (skinny_n && !dot && is_trans(ta) && fastMode == 0 && h->splitEpsMode == 0 && !st->env.gemv_split) {
+        bool done = false;
+        int nAv = 0, nBv = 0;
+        OZB_TRY(gemv_t_fused(h, m, k, A, lda, B, alpha, beta, C, &done, &nAv, &nBv));
+        if (done) {
+            const int ml = (nAv - 1) + (nBv - 1);
+            h->nSplitA = (float)nAv;
+            h->nSplitB = (float)nBv;
+            h->nSplitC = (float)(ml + 1 < nAv ? ml + 1 : nAv);
+            h->mbk = m;
+            h->nbk = n;
+            return CUOZBLAS_STATUS_SUCCESS;
+        }
+        ev_record(h, 0);
+    }
     // GEMV 'n' (rows of A strided): fused split and products, A read nA + 2 times
     if (skinny_n && !dot && !is_trans(ta) && !state(h)->env.gemv_split) {
         const uint64_t mk0 = ar.mark();

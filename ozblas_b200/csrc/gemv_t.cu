@@ -1,0 +1,571 @@
+// gemv_t.cu — the plain GEMV with contiguous lines (y = A^T x) without slices
+// in memory, and the one-launch split of a short vector.
+//
+// The reference splits every line of A level by level, x likewise, forms the
+// exact products of all slice pairs of a line and sums them in pair order
+// (src/cpu/ozblas_gemm.cpp with n = 1, called by ozblas_gemv.cpp:22-26).  With
+// the slices materialised a line is read, its slices written and read again:
+// 8 (2 nA + 2) bytes an element.  Here a line is read twice:
+//   pass 1  its largest element and lowest set bit, which under the predicted
+//           chain tau_{s+1} = tau_s + rho - 54 (chain.cuh) fix every level;
+//   pass 2  each element is cut in registers and multiplied with x's slices
+//           (read through L1); the largest remainder of every level is kept
+//           until it proves the prediction.
+// A line whose prediction is not proven is done again with its exact chain
+// (one pass per level).  The pair products are exact, so their order is free;
+// the ordered sum over the pairs follows, per line.  What bounds it is the FP64
+// pipe: per element 3 L + L nB operations for L levels of the line against
+// nB slices of x (28 for 4 x 4), 18 T a second on the chip.
+// Lines with more than kGtLevels levels, Inf / NaN or exponents near the ends
+// of the range, and x with more than kGtLevels slices, leave the call to the
+// slice path (nothing is written).
+//
+// 6001 x 3001 (phi = 1, 5 x 4 levels), one B200: the materialised path 853 us a
+// call (split 309, products 466, x's split 19), this one 206 (statistics 35,
+// products 129, x's split 9.5).  The products run at a fifth of the FP64 pipe:
+// 16 warps per SM (the accumulators take the registers) and the loads of x's
+// slices between their steps.
+#include "chain.cuh"
+#include "ozb_device.cuh"
+#include "ozb_internal.h"
+#include "sum.cuh"
+
+namespace ozb {
+
+constexpr int kGtLevels = 6;
+constexpr int kGtThreads = 256;
+constexpr int kGtStages = 8;  // steps of a line's elements in flight per warp (a step: 64 elements)
+
+struct VecSplitInfo {
+    int ns;     // the reference's slice count
+    int nz;     // slices that can be nonzero
+    int tau0;   // tau of level 0
+    int glast;  // exponent of the last nonzero slice's grid
+    int bad;    // Inf / NaN or a sigma beyond the range: the slices are not meaningful here
+};
+
+// ---------------------------------------------------------------------------
+// The split of a vector of at most 16384 elements without a grid-wide barrier
+// per level (k_split_vector's cooperative launch, split.cu: 17-21 us at 8192):
+// every CTA holds the whole vector in registers and follows the chain by
+// itself, and writes its share of the slices (one CTA's stores alone take
+// 2 us a level).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint64_t mag_bits(double v) {  // |v| in order; 0 for NaN, which the reference's max skips
+    const uint64_t b = dbits(v) & 0x7fffffffffffffffULL;
+    return b > 0x7ff0000000000000ULL ? 0 : b;
+}
+
+// The block's largest |v| over C values per thread (NaN skipped): by high
+// words, the low words only where the rule for tau or a zero depends on them.
+template <int C>
+__device__ __forceinline__ double block_max_abs(const double (&v)[C], unsigned *red) {  // red: 2 x 32, used in turn
+    unsigned hm = 0;
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+        const unsigned h = abs_hiword(v[c]);
+        hm = max(hm, h > 0x7ff00000u ? 0u : h);
+    }
+    hm = __reduce_max_sync(0xffffffffu, hm);
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+    if (l == 0) red[w] = hm;
+    __syncthreads();
+    hm = __reduce_max_sync(0xffffffffu, l < nw ? red[l] : 0u);
+    unsigned lm = 1;
+    if ((hm & 0xfffffu) == 0) {  // uniform: at a power of two, or subnormal, or zero
+        lm = 0;
+#pragma unroll
+        for (int c = 0; c < C; c++)
+            if (abs_hiword(v[c]) == hm && mag_bits(v[c]) != 0) lm = max(lm, (unsigned)__double2loint(v[c]));
+        lm = __reduce_max_sync(0xffffffffu, lm);
+        __syncthreads();
+        if (l == 0) red[w] = lm;
+        __syncthreads();
+        lm = __reduce_max_sync(0xffffffffu, l < nw ? red[l] : 0u);
+    }
+    return __hiloint2double((int)hm, (int)lm);
+}
+
+template <int C>
+__global__ void __launch_bounds__(1024) k_split_vector_one(int n, const double *__restrict__ x, int rho, int maxS,
+                                                           double *__restrict__ out, int ldo,
+                                                           VecSplitInfo *__restrict__ info) {
+    __shared__ unsigned red[2][32];
+    const int tid = threadIdx.x, nt = blockDim.x;
+    double r[C];
+    bool bad = false;
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+        const int i = c * nt + tid;
+        r[c] = i < n ? x[i] : 0.0;
+        bad |= !isfinite(r[c]);
+    }
+    bad = __syncthreads_or(bad);
+    double mx = block_max_abs(r, red[0]);
+    int s = 0, tau0 = 0, glast = 0, nz = 0;
+    for (; s < maxS; s++) {
+        if (s >= 2 && mx == 0.0) break;
+        const int tau = tau_rule(mx);
+        const double sigma = 0.75 * pow2(rho + tau);
+        if (rho + tau > 1023) bad = true;
+        if (s == 0) tau0 = tau;
+        if (mx != 0.0) {
+            glast = rho + tau - 53;
+            nz = s + 1;
+        }
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            const int i = c * nt + tid;
+            const double sl = (r[c] + sigma) - sigma;
+            r[c] = r[c] - sl;
+            if (c % (int)gridDim.x == (int)blockIdx.x && i < ldo) out[(size_t)s * ldo + i] = i < n ? sl : 0.0;
+        }
+        mx = block_max_abs(r, red[(s + 1) & 1]);
+    }
+    if (tid == 0 && blockIdx.x == 0) *info = VecSplitInfo{s, nz, tau0, glast, bad ? 1 : 0};
+}
+
+constexpr int kSplitOneMax = 16384;
+
+static int split_vector_one(cuozblasHandle_t *h, int n, const double *x, int rho, int maxS, double *out, int ldo,
+                            VecSplitInfo *info) {
+    cudaStream_t s = state(h)->stream;
+    counted(h);
+    const int len = ldo > n ? ldo : n;
+    if (len <= 2048)
+        k_split_vector_one<2><<<2, 1024, 0, s>>>(n, x, rho, maxS, out, ldo, info);
+    else if (len <= 8192)
+        k_split_vector_one<8><<<8, 1024, 0, s>>>(n, x, rho, maxS, out, ldo, info);
+    else
+        k_split_vector_one<16><<<16, 1024, 0, s>>>(n, x, rho, maxS, out, ldo, info);
+    OZB_CHECK(cudaGetLastError());
+    return CUOZBLAS_STATUS_SUCCESS;
+}
+
+// ---------------------------------------------------------------------------
+// The lines.  WPR warps per line (8 / WPR lines per CTA).
+// ---------------------------------------------------------------------------
+struct GemvTStatus {  // zeroed before the launch
+    int declined;     // some line (or x) needs the slice path: y is not written
+    int zmax;         // the largest first all-zero level of a line
+};
+
+struct GtPlan {
+    double sig[kGtLevels];
+    int L, z, bad;
+};
+
+// A (part of a) line's statistics from the first pass: the largest |v| (+inf
+// where it holds Inf or NaN) and the lowest set-bit exponent (4000: all zero).
+struct GtStat {
+    double mx;
+    int lb, pad;
+};
+
+// The levels of a line from tau_0 and its lowest set bit, under the predicted chain.
+__device__ __forceinline__ GtPlan gt_predict(int tau0, int lb, int rho, int maxS, int glast) {
+    GtPlan p;
+    const int d = 54 - rho, G0 = rho + tau0 - 53;
+    const int num = lb >= 4000 ? 0 : G0 - lb;
+    p.z = num <= 0 ? 0 : (num + d - 1) / d;
+    p.L = p.z + 1 < maxS ? p.z + 1 : maxS;
+    // every sigma and grid normal, every slice product on a representable grid
+    p.bad = p.L > kGtLevels || rho + tau0 > 1000 || G0 - p.z * d < -1000 || G0 - (p.L - 1) * d + glast < -1060;
+#pragma unroll
+    for (int s = 0; s < kGtLevels; s++) p.sig[s] = 0.75 * pow2(rho + tau0 - s * d);
+    return p;
+}
+
+// Pass 1: one warp per (line, part of it).
+__global__ void __launch_bounds__(256) k_gemv_t_stats(int nl, int k, const double *__restrict__ A, int lda, int parts,
+                                                      GtStat *__restrict__ out) {
+    const int w = (int)(((int64_t)blockIdx.x * 256 + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    const int row = w / parts, part = w % parts;
+    if (row >= nl) return;
+    const double *a = A + (size_t)row * lda;
+    LazyStats rs;
+    constexpr int kIn = 8;
+    const int step = 32 * parts;
+    int i = part * 32 + lane;
+    for (; i - lane + (kIn - 1) * step + 31 < k; i += kIn * step) {
+        double v[kIn];
+#pragma unroll
+        for (int u = 0; u < kIn; u++) v[u] = __ldg(a + i + u * step);
+#pragma unroll
+        for (int u = 0; u < kIn; u++) lazy_elem(rs, v[u]);
+        lazy_sync(rs);
+    }
+    for (; i - lane < k; i += step) lazy_elem(rs, i < k ? __ldg(a + i) : 0.0);
+    const uint64_t b = dbits(rs.mx);
+    const uint32_t hi = __reduce_max_sync(0xffffffffu, (uint32_t)(b >> 32));
+    const uint32_t lo = __reduce_max_sync(0xffffffffu, (uint32_t)(b >> 32) == hi ? (uint32_t)b : 0u);
+    const unsigned hmx = __reduce_max_sync(0xffffffffu, rs.hmax);
+    const int lb = __reduce_min_sync(0xffffffffu, rs.lb);
+    if (lane == 0)
+        out[w] = GtStat{hmx >= 0x7ff00000u ? __longlong_as_double(0x7ff0000000000000LL) : __hiloint2double((int)hi, (int)lo),
+                        lb, 0};
+}
+
+// E elements at once: their slices (levels 0..L-1) against x's; hm[s] the
+// largest high word of the remainder after level s.  The levels are a
+// dependent chain of 3 operations each, so the elements are interleaved.
+template <int L, int NB, int E, bool HM>
+__device__ __forceinline__ void gt_elements(double (&r)[E], const double (&xb)[E][NB], const double (&sig)[kGtLevels],
+                                            double (&P)[kGtLevels][NB], unsigned (&hm)[kGtLevels]) {
+#pragma unroll
+    for (int s = 0; s < L; s++) {
+        double sl[E];
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            sl[e] = (r[e] + sig[s]) - sig[s];
+            r[e] = r[e] - sl[e];
+            if (HM) hm[s] = max(hm[s], abs_hiword(r[e]));
+        }
+#pragma unroll
+        for (int e = 0; e < E; e++)
+#pragma unroll
+            for (int b = 0; b < NB; b++) P[s][b] = fma(sl[e], xb[e][b], P[s][b]);
+    }
+}
+template <int NB, int E, bool HM>
+__device__ __forceinline__ void gt_elements(int L, double (&r)[E], const double (&xb)[E][NB],
+                                            const double (&sig)[kGtLevels], double (&P)[kGtLevels][NB],
+                                            unsigned (&hm)[kGtLevels]) {
+    switch (L) {  // uniform over a line
+        case 0: break;
+        case 1: gt_elements<1, NB, E, HM>(r, xb, sig, P, hm); break;
+        case 2: gt_elements<2, NB, E, HM>(r, xb, sig, P, hm); break;
+        case 3: gt_elements<3, NB, E, HM>(r, xb, sig, P, hm); break;
+        case 4: gt_elements<4, NB, E, HM>(r, xb, sig, P, hm); break;
+        case 5: gt_elements<5, NB, E, HM>(r, xb, sig, P, hm); break;
+        default: gt_elements<6, NB, E, HM>(r, xb, sig, P, hm); break;
+    }
+}
+
+template <int WPR>
+__device__ __forceinline__ void gt_bar(int group) {  // the warps of one line
+    if (WPR == 1)
+        __syncwarp();
+    else
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(32 * WPR) : "memory");
+}
+
+// The ordered sum of a line's pairs from its warps' partial products.
+template <int WPR, int NB>
+__device__ __forceinline__ void gt_line_sum(double (&P)[kGtLevels][NB], int L, int nB, int sum_mode, double *ps,
+                                            int warp, int lane, int group, double *out) {
+    double *mine = ps + warp * (kGtLevels * kGtLevels);
+#pragma unroll
+    for (int s = 0; s < kGtLevels; s++)
+        if (s < L) {
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                double v = P[s][b];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0) mine[s * kGtLevels + b] = v;
+            }
+        }
+    gt_bar<WPR>(group);
+    if ((warp & (WPR - 1)) == 0) {
+        // lane = index of a pair in summation order
+        double *terms = ps + (size_t)(8 * kGtLevels * kGtLevels) + warp * 64;
+        int np = 0;
+        for_each_pair(L, nB, L + nB - 2, [&](int ia, int ib) {
+            if ((np & 31) == lane) {
+                double v = 0.0;
+                for (int w = 0; w < WPR; w++) v += mine[w * (kGtLevels * kGtLevels) + ia * kGtLevels + ib];
+                terms[np] = v;
+            }
+            np++;
+        });
+        __syncwarp();
+        if (lane == 0) {
+            double t = 0.0;
+            if (sum_mode == 1)
+                t = nearsum(np, terms, 1);
+            else
+                for (int i = 0; i < np; i++) t += terms[i];
+            *out = t;
+        }
+    }
+}
+
+struct GtShared {
+    double am[kGtStages][8][64];  // per warp: its elements, each read back by the lane that copied it
+    double ps[8 * kGtLevels * kGtLevels + 8 * 64];
+    uint64_t smx[8];
+    unsigned shm[8][kGtLevels];
+};
+
+template <int WPR, int NB>
+__device__ __forceinline__ void gt_lines(int nl, int k, const double *__restrict__ A, int lda,
+                                         const double *__restrict__ xs, int ldx, const VecSplitInfo &xi, int rho,
+                                         int maxS, int sum_mode, int parts, const GtStat *__restrict__ stats,
+                                         double *__restrict__ yt, GemvTStatus *st, GtShared &sh) {
+    auto &ps = sh.ps;
+    auto &smx = sh.smx;
+    auto &shm = sh.shm;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int group = warp / WPR, sub = warp % WPR, w0 = group * WPR;
+    const int row = blockIdx.x * (8 / WPR) + group;
+    const bool live = row < nl;
+    const double *a = A + (size_t)(live ? row : nl - 1) * lda;
+    const int nB = xi.nz;
+
+    // step `it` of this warp: elements (it WPR + sub) 64 + 2 lane, + 1.  x's slices
+    // come from L1, where the warps that run side by side share them.
+    const int nsteps = ((k + 63) / 64 - sub + WPR - 1) / WPR;
+    const int last_full = nsteps - (((nsteps - 1) * WPR + sub) * 64 + 64 > k ? 1 : 0);  // steps below it lie within the line
+    double *ring = &sh.am[0][warp][2 * lane];
+    constexpr int kRing = 8 * 64;
+    const double *aj = a + sub * 64 + 2 * lane;  // of the next step to issue
+    int slot = 0;
+    auto issue = [&](int it) {
+        if (it < last_full) {
+            cp_async8(ring + slot * kRing, aj);
+            cp_async8(ring + slot * kRing + 1, aj + 1);
+        } else if (it < nsteps) {
+            const int j = (it * WPR + sub) * 64 + 2 * lane;
+            cp_async8_zfill(ring + slot * kRing, j < k ? aj : a, j < k ? 8u : 0u);
+            cp_async8_zfill(ring + slot * kRing + 1, j + 1 < k ? aj + 1 : a, j + 1 < k ? 8u : 0u);
+        }
+        cp_async_commit();
+        aj += 64 * WPR;
+        slot = slot == kGtStages - 1 ? 0 : slot + 1;
+    };
+#pragma unroll
+    for (int g = 0; g < kGtStages - 1; g++) issue(g);
+
+    // the line's statistics
+    double mx = 0.0;
+    int lb = 4000;
+    for (int w = 0; w < parts; w++) {
+        const GtStat g = stats[(size_t)(live ? row : nl - 1) * parts + w];
+        mx = fmax(mx, g.mx);
+        lb = min(lb, g.lb);
+    }
+    const bool nonfinite = !(mx <= 1.7976931348623157e308);
+    const int tau0 = nonfinite ? 0 : tau_rule(mx);
+    GtPlan pl = gt_predict(tau0, lb, rho, maxS, xi.glast);
+    bool bad = nonfinite || pl.bad || tau0 + xi.tau0 + ceil_log2_int((uint32_t)k) > 1000;
+    if (bad) pl.L = 0;
+    const int step = 32 * WPR;
+
+    // ---- pass 2 ----
+    double P[kGtLevels][NB];
+    unsigned hm[kGtLevels];
+#pragma unroll
+    for (int s = 0; s < kGtLevels; s++) {
+        hm[s] = 0;
+#pragma unroll
+        for (int b = 0; b < NB; b++) P[s][b] = 0.0;
+    }
+    // tau_rule of a value of at most 2^t is t when its high word is above that
+    // of 2^(t-1): level s is proven by a remainder above thr(s)
+    auto thr = [&](int s) { return (unsigned)(dbits(pow2(tau0 - (s + 1) * (54 - rho) - 1)) >> 32); };
+    bool track = true;  // per warp, until its own elements prove every level
+    const double *xj = xs + sub * 64 + 2 * lane;  // slices are padded with zeros to whole steps
+    int rd = 0;
+    for (int it = 0; it < nsteps; it++, xj += 64 * WPR) {
+        double xb[2][NB];
+#pragma unroll
+        for (int b = 0; b < NB; b++) {
+            const double2 v = b < nB ? __ldg(reinterpret_cast<const double2 *>(xj + (size_t)b * ldx))
+                                     : make_double2(0.0, 0.0);
+            xb[0][b] = v.x;
+            xb[1][b] = v.y;
+        }
+        cp_async_wait<kGtStages - 2>();
+        const double2 av = *reinterpret_cast<const double2 *>(ring + rd * kRing);
+        rd = rd == kGtStages - 1 ? 0 : rd + 1;
+        double r[2] = {av.x, av.y};
+        issue(it + kGtStages - 1);
+        if (track) {
+            gt_elements<NB, 2, true>(pl.L, r, xb, pl.sig, P, hm);
+            if ((it & 7) == 0) {
+                bool open = false;
+#pragma unroll
+                for (int s = 0; s + 1 < kGtLevels; s++)
+                    if (s + 1 < pl.L) open |= !__any_sync(0xffffffffu, hm[s] > thr(s));
+                track = open;
+            }
+        } else {
+            gt_elements<NB, 2, false>(pl.L, r, xb, pl.sig, P, hm);
+        }
+    }
+    cp_async_wait<0>();
+
+    // ---- proof: the first level that leaves nothing, and that every level before it leaves a remainder whose tau
+    // is the predicted one
+#pragma unroll
+    for (int s = 0; s < kGtLevels; s++) {
+        const unsigned h = __reduce_max_sync(0xffffffffu, hm[s]);
+        if (lane == 0) shm[warp][s] = h;
+    }
+    gt_bar<WPR>(group);
+    bool proven = true, ended = false;
+#pragma unroll
+    for (int s = 0; s + 1 < kGtLevels; s++)
+        if (s + 1 < pl.L && !ended) {
+            unsigned h = 0;
+            for (int w = 0; w < WPR; w++) h = max(h, shm[w0 + w][s]);
+            if (h == 0) {  // exact zeros from here on: grids are normal, so no remainder hides below the high word
+                pl.z = s;
+                ended = true;
+            } else {
+                proven = proven && h > thr(s);
+            }
+        }
+    if (!bad && !proven) {  // the exact chain, one pass per level, and the products again (x's slices from L2)
+        int z = maxS - 1, L = maxS;
+        for (int s = 1;; s++) {
+            uint64_t m = 0;
+            for (int j = sub * 32 + lane; j < k; j += step) {
+                double r = __ldg(a + j);
+#pragma unroll
+                for (int q = 0; q < kGtLevels; q++)
+                    if (q < s) r = r - ((r + pl.sig[q]) - pl.sig[q]);
+                const uint64_t b = mag_bits(r);
+                m = b > m ? b : m;
+            }
+            const uint32_t hi = __reduce_max_sync(0xffffffffu, (uint32_t)(m >> 32));
+            const uint32_t lo = __reduce_max_sync(0xffffffffu, (uint32_t)(m >> 32) == hi ? (uint32_t)m : 0u);
+            gt_bar<WPR>(group);
+            if (lane == 0) smx[warp] = ((uint64_t)hi << 32) | lo;
+            gt_bar<WPR>(group);
+            uint64_t mm = 0;
+            for (int w = 0; w < WPR; w++) mm = smx[w0 + w] > mm ? smx[w0 + w] : mm;
+            if (mm == 0) {
+                z = s - 1 < maxS - 1 ? s - 1 : maxS - 1;
+                L = s;
+                break;
+            }
+            if (s == maxS) break;
+            const int tau = tau_rule(__longlong_as_double((long long)mm));
+            if (s == kGtLevels || rho + tau - 53 < -1000 || rho + tau - 53 + xi.glast < -1060) {
+                bad = true;
+                break;
+            }
+#pragma unroll
+            for (int q = 0; q < kGtLevels; q++)
+                if (q == s) pl.sig[q] = 0.75 * pow2(rho + tau);
+        }
+        pl.z = z;
+        pl.L = bad ? 0 : L;
+#pragma unroll
+        for (int s = 0; s < kGtLevels; s++)
+#pragma unroll
+            for (int b = 0; b < NB; b++) P[s][b] = 0.0;
+        for (int j = sub * 32 + lane; j < k; j += step) {
+            double xb[1][NB], r[1] = {__ldg(a + j)};
+#pragma unroll
+            for (int b = 0; b < NB; b++) xb[0][b] = b < nB ? xs[(size_t)b * ldx + j] : 0.0;
+            gt_elements<NB, 1, false>(pl.L, r, xb, pl.sig, P, hm);
+        }
+    }
+    double t = 0.0;
+    gt_line_sum<WPR, NB>(P, pl.L, nB, sum_mode, ps, warp, lane, group, &t);
+    if (live && sub == 0 && lane == 0) {
+        if (bad)
+            atomicOr(&st->declined, 1);
+        else
+            __stcg(yt + row, t);
+        const int z = pl.z < maxS - 1 ? pl.z : maxS - 1;
+        if (z > __ldcg(&st->zmax)) atomicMax(&st->zmax, z);
+    }
+}
+
+template <int WPR>
+__global__ void __launch_bounds__(kGtThreads, 2)
+    k_gemv_t(int nl, int k, const double *__restrict__ A, int lda, const double *__restrict__ xs, int ldx,
+             const VecSplitInfo *__restrict__ info, int rho, int maxS, int sum_mode, int parts,
+             const GtStat *__restrict__ stats, double *__restrict__ yt, GemvTStatus *st) {
+    const VecSplitInfo xi = *info;
+    __shared__ __align__(16) GtShared sh;
+    if (xi.bad || xi.nz > kGtLevels) {  // uniform over the grid
+        if (blockIdx.x == 0 && threadIdx.x == 0) st->declined = 1;
+        return;
+    }
+    if (xi.nz <= 4)
+        gt_lines<WPR, 4>(nl, k, A, lda, xs, ldx, xi, rho, maxS, sum_mode, parts, stats, yt, st, sh);
+    else
+        gt_lines<WPR, 6>(nl, k, A, lda, xs, ldx, xi, rho, maxS, sum_mode, parts, stats, yt, st, sh);
+}
+
+// y, once it is known that every line has its sum.
+__global__ void k_gemv_t_write(int nl, const double *__restrict__ yt, const GemvTStatus *__restrict__ st, double alpha,
+                               double beta, double *__restrict__ y) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r < nl && !st->declined) y[r] = fma(alpha, yt[r], beta * y[r]);
+}
+
+// y = alpha A^T x + beta y over nl lines of length k (line l at A + l lda),
+// splitEpsMode 0 and the full pair set.  *done false (y untouched) when the
+// slice path must run.
+int gemv_t_fused(cuozblasHandle_t *h, int nl, int k, const double *A, int lda, const double *x, double alpha,
+                 double beta, double *y, bool *done, int *nA, int *nB) {
+    State *st = state(h);
+    *done = false;
+    if (k < 1 || nl < 1 || k > kSplitOneMax) return CUOZBLAS_STATUS_SUCCESS;
+    const int maxS = h->nSplitMax > 0 ? h->nSplitMax : kMaxSplitDefault;
+    const int rho = rho_rule(k, 0);
+    const int ldx = (k + 63) / 64 * 64;  // whole steps, zero padded
+    Arena ar(h);
+    const uint64_t mk = ar.mark();
+    double *xs = ar.take<double>((uint64_t)maxS * ldx);
+    double *yt = ar.take<double>(nl);
+    // parts of a line in pass 1: enough warps to keep the memory busy
+    int parts = 1;
+    while (parts < 8 && (int64_t)nl * parts < 48 * sm_count() && k > 512 * parts) parts *= 2;
+    GtStat *stats = ar.take<GtStat>((uint64_t)nl * parts);
+    struct Block {
+        GemvTStatus st;
+        VecSplitInfo info;
+    } *blk = ar.take<Block>(1);
+    if (!ar.ok) {
+        ar.release(mk);
+        return CUOZBLAS_STATUS_SUCCESS;
+    }
+    span_begin(h);
+    OZB_CHECK(cudaMemsetAsync(blk, 0, sizeof(Block), st->stream));
+    OZB_TRY(split_vector_one(h, k, x, rho, maxS, xs, ldx, &blk->info));
+    counted(h);
+    k_gemv_t_stats<<<(unsigned)(((int64_t)nl * parts * 32 + 255) / 256), 256, 0, st->stream>>>(nl, k, A, lda, parts, stats);
+    OZB_CHECK(cudaGetLastError());
+    // Warps per line: the fewest rounds of the 16 resident warps per SM over (line part + its reductions).
+    int wpr = 1;
+    int64_t best = INT64_MAX;
+    for (int w = 1; w <= 8; w *= 2) {
+        const int64_t rounds = ((int64_t)nl * w + 16 * sm_count() - 1) / (16 * sm_count());
+        const int64_t cost = rounds * ((k + w - 1) / w + 400);
+        if (cost < best) {
+            best = cost;
+            wpr = w;
+        }
+    }
+    const int rows = 8 / wpr, grid = (nl + rows - 1) / rows;
+    counted(h);
+    auto go = [&](auto kern) {
+        kern<<<grid, kGtThreads, 0, st->stream>>>(nl, k, A, lda, xs, ldx, &blk->info, rho, maxS, h->sumMode, parts, stats,
+                                                  yt, &blk->st);
+    };
+    wpr == 1 ? go(k_gemv_t<1>) : wpr == 2 ? go(k_gemv_t<2>) : wpr == 4 ? go(k_gemv_t<4>) : go(k_gemv_t<8>);
+    OZB_CHECK(cudaGetLastError());
+    counted(h);
+    k_gemv_t_write<<<(nl + 255) / 256, 256, 0, st->stream>>>(nl, yt, &blk->st, alpha, beta, y);
+    OZB_CHECK(cudaGetLastError());
+    span_end(h);
+    Block *hb = reinterpret_cast<Block *>(st->h_ints);
+    OZB_CHECK(cudaMemcpyAsync(hb, blk, sizeof(Block), cudaMemcpyDeviceToHost, st->stream));
+    OZB_CHECK(cudaStreamSynchronize(st->stream));
+    ar.release(mk);
+    if (hb->st.declined) return CUOZBLAS_STATUS_SUCCESS;
+    const int c = (hb->st.zmax < 1 ? 1 : hb->st.zmax) + 1;
+    *nA = c < maxS ? c : maxS;
+    *nB = hb->info.ns;
+    *done = true;
+    return CUOZBLAS_STATUS_SUCCESS;
+}
+
+}  // namespace ozb

@@ -267,11 +267,13 @@ int pair_products_skinny(cuozblasHandle_t *h, bool dot, int m, int k, int nA, in
 int gemm_q_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, const void *alpha, const void *A, int lda,
                 const void *B, int ldb, const void *beta, void *C, int ldc, int fastMode);
 
-// ---- skinny forms (gemm_plain.cu, gemv_fused.cu) ----
+// ---- skinny forms (gemm_plain.cu, gemv_fused.cu, gemv_t.cu) ----
 int sum_rows_launch(cuozblasHandle_t *h, int m, int nA, int nB, int maxlevel, double *P, int64_t ldp, double alpha,
                     double beta, double *y, double *scratch);
 int gemv_fused_n(cuozblasHandle_t *h, int m, int n, const double *A, int lda, const double *xs, int ldx, int nB,
                  int rho, int maxS, int fastMode, double alpha, double beta, double *y, int *nA_out);
+int gemv_t_fused(cuozblasHandle_t *h, int nl, int k, const double *A, int lda, const double *x, double alpha,
+                 double beta, double *y, bool *done, int *nA, int *nB);
 int gemv_rn_n(cuozblasHandle_t *h, int m, int n, const double *A, int lda, const double *x, double alpha, double beta,
               double *y, bool *done, int *nA, int *nB);
 
