@@ -362,6 +362,7 @@ struct PpShape {
 
 struct PpParams {
     int m, n, ldc, nkb, tiles_m, tiles_n, strip;
+    int col0, cn;        // the launch's columns: cn from col0 (a tile boundary); tiles_n and lb count from col0
     int nA, nB, maxlevel, np, bias, radix;
     const int *la, *lb;  // levels in use per tile, or null
     const short *ea, *eb;
@@ -556,8 +557,9 @@ __device__ __forceinline__ double i2d(long long v) {
            __hiloint2double(0x43300000, lo);
 }
 // The exact pair product V 2^e of a pair-buffer entry, 0 or NaN where either
-// line's exponent says so, rounded once if it is subnormal.
-__device__ __forceinline__ double pair_value(long long v, int bias, int ea, int eb) {
+// line's exponent says so, rounded once if it is subnormal.  Not inlined: the
+// callers' common case is one test away, and inlined this ran predicated.
+__device__ __noinline__ double pair_value(long long v, int bias, int ea, int eb) {
     const bool spa = ea == kExpZero || ea == kExpNaN, spb = eb == kExpZero || eb == kExpNaN;
     const double d = i2d(v);
     if (spa || spb) return d * (spa ? exp_scale(ea) : 1.0) * (spb ? exp_scale(eb) : 1.0);
@@ -567,7 +569,7 @@ __device__ __forceinline__ double pair_value(long long v, int bias, int ea, int 
 
 // The <float,double,double> sum's term of c32, the product rounded to float:
 // (float)scalbn(c32, tauA + tauB).
-__device__ __forceinline__ double pair_term_sd(double c32, int ea, int eb) {
+__device__ __noinline__ double pair_term_sd(double c32, int ea, int eb) {
     const bool spa = ea == kExpZero || ea == kExpNaN, spb = eb == kExpZero || eb == kExpNaN;
     if (spa || spb) return c32 * (spa ? exp_scale(ea) : 1.0) * (spb ? exp_scale(eb) : 1.0);
     return (double)__double2float_rn(scale2(c32, ea + eb));
@@ -727,7 +729,8 @@ __global__ void __launch_bounds__(kPpThreads, 1)
                                 uint8_t *sa = smem + slot * S::STAGE;
                                 tc::mbar_arrive_expect_tx(&full[slot], S::STAGE);
                                 tc::tma_load_3d(sa, &tmA, &full[slot], kb * 128, tm * 128, ia * D + d);
-                                tc::tma_load_3d(sa + S::TILE_A, &tmB, &full[slot], kb * 128, tn * S::BN, ib * D + d);
+                                tc::tma_load_3d(sa + S::TILE_A, &tmB, &full[slot], kb * 128, p.col0 + tn * S::BN,
+                                                ib * D + d);
                                 issued |= 1u << slot;
                                 issued_phase = (issued_phase & ~(1u << slot)) | (phase << slot);
                                 if (++slot == S::ST) {
@@ -796,7 +799,7 @@ __global__ void __launch_bounds__(kPpThreads, 1)
                 return true;
             },
             [&](int tm, int tn, int ia, int ib, int pr) {
-                const int gr = tm * 128 + row, gc0 = tn * S::BN + half * CW;
+                const int gr = tm * 128 + row, gc0 = p.col0 + tn * S::BN + half * CW;
                 // the scales do not depend on the MMAs: loaded before the waits
                 int ea = 0;
                 bool fast = false;
@@ -855,8 +858,9 @@ __global__ void __launch_bounds__(kPpThreads, 1)
                 units++;
                 if constexpr (EPI == kPairStore) {
                     if (gr < p.m) {
-                        long long *o = reinterpret_cast<long long *>(p.pbuf) + ((size_t)pr * p.n + gc0) * p.m + gr;
-                        const int nc = min(CW, p.n - gc0);
+                        long long *o = reinterpret_cast<long long *>(p.pbuf) + ((size_t)pr * p.cn + (gc0 - p.col0)) * p.m +
+                                       gr;
+                        const int nc = min(CW, p.col0 + p.cn - gc0);
 #pragma unroll
                         for (int c = 0; c < CW; c++)
                             if (c < nc) o[(size_t)c * p.m] = acc[c];
@@ -912,7 +916,7 @@ __global__ void __launch_bounds__(kPpThreads, 1)
                                      : "memory");
                     }
                 } else if (FUSED) {
-                    const int gr = tm * 128 + row, gc0 = tn * S::BN + half * CW;
+                    const int gr = tm * 128 + row, gc0 = p.col0 + tn * S::BN + half * CW;
                     if (gr < p.m) {
 #pragma unroll
                         for (int c = 0; c < CW; c++) {
@@ -953,16 +957,42 @@ static int transpose_t(cuozblasHandle_t *h, int rows, int cols, const float *A, 
     return transpose_f32(h, rows, cols, A, lda, out, ldo);
 }
 
-bool pair_fuse_sum(int m, int n, int k_pad, int np, int D) {
+// The two ways to the ordered sum, in microseconds as measured: a pair's 128 k
+// take 1.35 (D = 3), its hand-over 2 (1.5 more with the sum in the epilogue).
+static double pair_us(int k_pad, int D) { return (double)(k_pad / 128) * 0.15 * D * D + 2.0; }
+
+// In the epilogue: every CTA runs an equal share, but no tile meets three CTAs
+// (pp_share), so a CTA runs at least a tile's pairs.
+static double pair_fused_us(int m, int n, int k_pad, int np, int D) {
     const int64_t tiles = (int64_t)((m + 127) / 128) * ((n + pair_tile_b(D) - 1) / pair_tile_b(D));
-    const int sms = sm_count();
-    // Microseconds, as measured: a pair's 128 k take 1.35 (D = 3) and its hand-over 2 (1.5 more with the
-    // sum in the epilogue).  Fused, every CTA runs an equal share, but no tile on three CTAs (pp_share).
-    const double pair_us = (double)(k_pad / 128) * 0.15 * D * D + 2.0;
-    const int64_t share = (tiles * np + sms - 1) / sms;
-    const double fused = (double)(share > np ? share : np) * (pair_us + 1.5);
-    const double split = (double)share * pair_us + 8.0 * np * (double)m * n / 5e6 + 4.0;
-    return fused <= split;
+    const int64_t share = (tiles * np + sm_count() - 1) / sm_count();
+    return (double)(share > np ? share : np) * (pair_us(k_pad, D) + 1.5);
+}
+
+// Through a pair buffer: the pairs of a tile spread over the CTAs, then the
+// sum.  A buffer beyond L2 is written back while it is read; in column blocks of
+// at most 64 MB it stays on chip, at the price of a last wave and two launches
+// per block.
+struct PairStorePlan {
+    int blocks;
+    double us;
+};
+static PairStorePlan pair_store_plan(int m, int n, int k_pad, int np, int D) {
+    const int bn = pair_tile_b(D), tn = (n + bn - 1) / bn, tm = (m + 127) / 128;
+    PairStorePlan best{1, 1e30};
+    for (int blocks = 1; blocks <= 8 && blocks <= tn; blocks++) {
+        const int cols = (tn + blocks - 1) / blocks;  // tile columns per block
+        const int count = (tn + cols - 1) / cols;
+        const double mb = 8e-6 * np * (double)m * (cols * bn < n ? cols * bn : n);
+        double us = 0.0;
+        for (int b = 0; b < count; b++) {
+            const int64_t units = (int64_t)tm * (b + 1 < count ? cols : tn - cols * (count - 1)) * np;
+            us += (double)((units + sm_count() - 1) / sm_count()) * pair_us(k_pad, D) + 7.0;
+        }
+        us += count * mb / (mb <= 64.0 ? 5.0 : 3.5);  // MB / (TB/s) = us
+        if (us < best.us) best = PairStorePlan{count, us};
+    }
+    return best;
 }
 
 int pair_products(cuozblasHandle_t *h, const PairDigits &pd, const PairOperand &A, const PairOperand &B,
@@ -975,7 +1005,9 @@ int pair_products(cuozblasHandle_t *h, const PairDigits &pd, const PairOperand &
     p.nkb = c.k_pad / 128;
     const int bn = pair_tile_b(pd.D);
     p.tiles_m = (c.m + 127) / 128;
-    p.tiles_n = (c.n + bn - 1) / bn;
+    p.col0 = c.col0;
+    p.cn = c.cn > 0 ? c.cn : c.n;
+    p.tiles_n = (p.cn + bn - 1) / bn;
     p.strip = p.tiles_m < 12 ? p.tiles_m : 12;
     p.nA = c.nA;
     p.nB = c.nB;
@@ -985,7 +1017,7 @@ int pair_products(cuozblasHandle_t *h, const PairDigits &pd, const PairOperand &
     p.bias = c.bias;
     p.radix = pd.radix;
     p.la = A.tile_lev;
-    p.lb = B.tile_lev;
+    p.lb = B.tile_lev ? B.tile_lev + c.col0 / bn : nullptr;
     p.ea = A.exps;
     p.eb = B.exps;
     p.alpha = c.alpha;
@@ -1047,51 +1079,26 @@ int pair_status(cuozblasHandle_t *h) {
     return CUOZBLAS_STATUS_SUCCESS;
 }
 
-// The ordered sum of a pair buffer pbuf[p][col][row] of exact integer products V: FSum
-// in pair order, or NearSum (which overwrites the buffer); FLOATS: the
-// <float,double,double> sum, t += (float)scalbn((float)P, tauA + tauB).  One
-// thread per output, the loads of 4 pairs in flight; pairs that the product
-// kernel skipped (levels not in use in the tile) are skipped here too.
+// The ordered sum of a pair buffer pbuf[p][col][row] of exact integer products V
+// (columns col0 .. col0 + cn): FSum in pair order, or NearSum (which overwrites
+// the buffer); FLOATS: the <float,double,double> sum, t += (float)scalbn((float)P,
+// tauA + tauB).  One thread per output row and kPsCols columns, the loads of
+// kPsIn pairs in flight.  A block lists, per column, each pair's A level and
+// its part of the exponent, so that a term takes two shared loads and about
+// fifteen instructions (with the list found per term and both forms of it
+// inlined a term took 74, and the code did not fit the instruction cache).
+// Entries of pairs that the product kernel skipped hold anything: the lines'
+// marks at those levels make them zeros.
+constexpr int kPsRows = 256, kPsCols = 2, kPsIn = 16;
+constexpr int kPsLevels = 12, kPsPairs = 144;  // held in shared memory; k_pair_sum_any beyond
+
 template <bool FLOATS>
-__global__ void __launch_bounds__(256) k_pair_sum(int m, int n, int nA, int nB, int maxlevel, int np,
-                                                  double *__restrict__ pbuf, const int *__restrict__ la,
-                                                  const int *__restrict__ lb, int tile_b,
-                                                  const short *__restrict__ ea, const short *__restrict__ eb,
-                                                  int bias, int sum_mode, double alpha, double beta, void *__restrict__ Cv,
-                                                  int ldc) {
-    const int rb = (m + 255) / 256, col = blockIdx.x / rb, row = (blockIdx.x - col * rb) * 256 + threadIdx.x;
-    if (row >= m) return;
-    const size_t count = (size_t)m * n;
-    double *pe = pbuf + (size_t)col * m + row;
-    const size_t at = (size_t)col * ldc + row;
-    if (!FLOATS && sum_mode == 1) {
-        int p = 0;
-        for_each_pair(nA, nB, maxlevel, [&](int ia, int ib) {
-            double *v = pe + (size_t)p++ * count;
-            *v = pair_value(__double_as_longlong(*v), bias, ea[(size_t)ia * m + row], eb[(size_t)ib * n + col]);
-        });
-        double *cp = reinterpret_cast<double *>(Cv) + at;
-        *cp = fma(alpha, nearsum(np, pe, (int64_t)count), beta * *cp);
-        return;
-    }
-    const int LA = la ? min(la[row / kPairTileA], nA) : nA, LB = lb ? min(lb[col / tile_b], nB) : nB;
-    double t = 0.0;
-    float tf = 0.f;
-    int p = 0;
-    for (int ik = 0; ik <= maxlevel; ik++) {
-        const int lo = max(0, ik - (nB - 1)), hi = min(ik, nA - 1);
-        const int from = max(lo, ik - (LB - 1)), to = min(hi, LA - 1);  // the pairs in use
-#pragma unroll 4
-        for (int ia = from; ia <= to; ia++) {
-            const long long v = __double_as_longlong(__ldcs(pe + (size_t)(p + ia - lo) * count));
-            const int a = ea[(size_t)ia * m + row], b = __ldg(eb + (size_t)(ik - ia) * n + col);
-            if (FLOATS)
-                tf = __fadd_rn(tf, (float)pair_term_sd((double)__ll2float_rn(v) * pow2(bias), a, b));
-            else
-                t = __dadd_rn(t, pair_value(v, bias, a, b));
-        }
-        p += hi - lo + 1;
-    }
+__device__ __noinline__ double pair_term(long long v, int bias, int a, int b) {
+    return FLOATS ? pair_term_sd((double)__ll2float_rn(v) * pow2(bias), a, b) : pair_value(v, bias, a, b);
+}
+
+template <bool FLOATS>
+__device__ __forceinline__ void pair_out(void *Cv, size_t at, double alpha, double beta, double t, float tf) {
     if (FLOATS) {
         float *cp = reinterpret_cast<float *>(Cv) + at;
         *cp = __double2float_rn(fma((double)(float)alpha, (double)tf, (double)__fmul_rn((float)beta, *cp)));
@@ -1099,6 +1106,91 @@ __global__ void __launch_bounds__(256) k_pair_sum(int m, int n, int nA, int nB, 
         double *cp = reinterpret_cast<double *>(Cv) + at;
         *cp = fma(alpha, t, beta * *cp);
     }
+}
+
+template <bool FLOATS>
+__global__ void __launch_bounds__(kPsRows, 4)
+    k_pair_sum(int m, int n, int col0, int cn, int nA, int nB, int np, const double *__restrict__ pbuf,
+               const short *__restrict__ ea, const short *__restrict__ eb, int bias, double alpha, double beta,
+               void *__restrict__ Cv, int ldc) {
+    __shared__ short sA[kPsLevels][kPsRows];
+    __shared__ int2 sP[kPsCols][kPsPairs];  // A level, B level's tau
+    const int rb = (m + kPsRows - 1) / kPsRows, tr = threadIdx.x;
+    const int row = (int)(blockIdx.x % rb) * kPsRows + tr, c0 = col0 + (int)(blockIdx.x / rb) * kPsCols;
+    const int nc = min(kPsCols, col0 + cn - c0);
+    if (row < m)
+        for (int s = 0; s < nA; s++) sA[s][tr] = ea[(size_t)s * m + row];
+    for (int i = tr; i < np * nc; i += kPsRows) {
+        const int q = i / nc, c = i - q * nc;
+        int ia, ib;
+        pair_at(q, nA, nB, ia, ib);
+        sP[c][q] = make_int2(ia, eb[(size_t)ib * n + c0 + c]);
+    }
+    __syncthreads();
+    if (row >= m) return;
+    const size_t count = (size_t)m * cn;
+    for (int c = 0; c < nc; c++) {
+        const double *pe = pbuf + (size_t)(c0 + c - col0) * m + row;
+        double t = 0.0;
+        float tf = 0.f;
+        for (int q0 = 0; q0 < np; q0 += kPsIn) {
+            long long v[kPsIn];
+#pragma unroll
+            for (int j = 0; j < kPsIn; j++) v[j] = __double_as_longlong(pe[(size_t)min(q0 + j, np - 1) * count]);
+#pragma unroll
+            for (int j = 0; j < kPsIn; j++) asm volatile("" : "+l"(v[j]));  // all loaded here, not each at its use
+#pragma unroll
+            for (int j = 0; j < kPsIn; j++) {
+                if (q0 + j < np) {  // uniform
+                    const int2 pr = sP[c][q0 + j];
+                    const int a = sA[pr.x][tr], e = bias + a + pr.y;
+                    // V 2^e is exact when e is well inside the range: one fma rounds as the addition.  The
+                    // line marks lie far outside, so one test sends them to the general form.
+                    if (FLOATS) {
+                        if (e >= -126 && e <= 73)  // float(V) has at most 24 bits
+                            tf = fmaf(__ll2float_rn(v[j]), __int_as_float((e + 127) << 23), tf);
+                        else
+                            tf = __fadd_rn(tf, (float)pair_term<true>(v[j], bias, a, pr.y));
+                    } else {
+                        if (e >= -1022 && e <= 969)
+                            t = fma(i2d(v[j]), __hiloint2double((e + 1023) << 20, 0), t);
+                        else
+                            t = __dadd_rn(t, pair_term<false>(v[j], bias, a, pr.y));
+                    }
+                }
+            }
+        }
+        pair_out<FLOATS>(Cv, (size_t)(c0 + c) * ldc + row, alpha, beta, t, tf);
+    }
+}
+
+// The same without the shared lists (any counts), and NearSum.
+template <bool FLOATS>
+__global__ void __launch_bounds__(256)
+    k_pair_sum_any(int m, int n, int col0, int cn, int nA, int nB, int maxlevel, int np, double *__restrict__ pbuf,
+                   const short *__restrict__ ea, const short *__restrict__ eb, int bias, int sum_mode, double alpha,
+                   double beta, void *__restrict__ Cv, int ldc) {
+    const int rb = (m + 255) / 256;
+    const int row = (int)(blockIdx.x % rb) * 256 + threadIdx.x, col = col0 + (int)(blockIdx.x / rb);
+    if (row >= m) return;
+    const size_t count = (size_t)m * cn;
+    double *pe = pbuf + (size_t)(col - col0) * m + row;
+    double t = 0.0;
+    float tf = 0.f;
+    int p = 0;
+    for_each_pair(nA, nB, maxlevel, [&](int ia, int ib) {
+        double *v = pe + (size_t)p++ * count;
+        const double term =
+            pair_term<FLOATS>(__double_as_longlong(*v), bias, ea[(size_t)ia * m + row], eb[(size_t)ib * n + col]);
+        if (FLOATS)
+            tf = __fadd_rn(tf, (float)term);
+        else if (sum_mode == 1)
+            *v = term;
+        else
+            t = __dadd_rn(t, term);
+    });
+    if (!FLOATS && sum_mode == 1) t = nearsum(np, pe, (int64_t)count);
+    pair_out<FLOATS>(Cv, (size_t)col * ldc + row, alpha, beta, t, tf);
 }
 
 // C = alpha op(A) op(B) + beta C with m, n > 1 in the plain form (T = double)
@@ -1210,26 +1302,45 @@ int gemm_pairs_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
     Arena ar(h);
     const bool near = !kFloats && h->sumMode == 1;
     c.epi = kFloats ? kPairSd : kPairFsum;
-    if (near || !pair_fuse_sum(m, n, k_pad, npu, pd.D)) {
-        c.pbuf = ar.take<double>((uint64_t)npu * m * n);
-        if (ar.ok)
+    const PairStorePlan sp = pair_store_plan(m, n, k_pad, npu, pd.D);
+    if (near || sp.us < pair_fused_us(m, n, k_pad, npu, pd.D)) {
+        // in column blocks: as many as the plan asks for, or as the arena does
+        const uint64_t avail = h->workSizeBytes - ((ar.mark() + 255) / 256 * 256);
+        int64_t cols = (n + sp.blocks - 1) / sp.blocks;
+        const int64_t most = (int64_t)(avail / (sizeof(double) * (uint64_t)npu * (uint64_t)m));
+        if (cols > most) cols = most;
+        if (cols < n) cols = (cols + (sp.blocks > 1 && cols < most ? tile[1] - 1 : 0)) / tile[1] * tile[1];
+        if (cols > 0) {
+            c.cn = (int)cols;
+            c.pbuf = ar.take<double>((uint64_t)npu * m * cols);
             c.epi = kPairStore;
-        else if (near) {  // the slice path blocks the columns
+        } else if (near) {  // the slice path blocks the columns further
             ar.release(mark0);
             return CUOZBLAS_STATUS_SUCCESS;
         }
-        ar.ok = true;
+        if (!ar.ok) {
+            ar.release(mark0);
+            return CUOZBLAS_STATUS_SUCCESS;
+        }
     }
     if (c.epi == kPairStore) {
-        PairOperand a = op[0], b = op[1];
-        if (near) a.tile_lev = b.tile_lev = nullptr;  // NearSum reads every term
-        OZB_TRY(pair_products(h, pd, a, b, c));
-        ev_record(h, 3);
-        counted(h);
-        k_pair_sum<kFloats><<<(unsigned)((int64_t)((m + 255) / 256) * n), 256, 0, st->stream>>>(
-            m, n, c.nA, c.nB, c.maxlevel, npu, c.pbuf, a.tile_lev, b.tile_lev, tile[1], op[0].exps, op[1].exps,
-            c.bias, h->sumMode, alpha, beta, C, ldc);
-        OZB_CHECK(cudaGetLastError());
+        const int cols = c.cn;
+        for (int c0 = 0; c0 < n; c0 += cols) {
+            c.col0 = c0;
+            c.cn = n - c0 < cols ? n - c0 : cols;
+            OZB_TRY(pair_products(h, pd, op[0], op[1], c));
+            if (c0 + cols >= n) ev_record(h, 3);
+            counted(h);
+            if (!near && c.nA <= kPsLevels && npu <= kPsPairs)
+                k_pair_sum<kFloats><<<(unsigned)((int64_t)((m + kPsRows - 1) / kPsRows) * ((c.cn + kPsCols - 1) / kPsCols)),
+                                      kPsRows, 0, st->stream>>>(m, n, c0, c.cn, c.nA, c.nB, npu, c.pbuf, op[0].exps,
+                                                                op[1].exps, c.bias, alpha, beta, C, ldc);
+            else
+                k_pair_sum_any<kFloats><<<(unsigned)((int64_t)((m + 255) / 256) * c.cn), 256, 0, st->stream>>>(
+                    m, n, c0, c.cn, c.nA, c.nB, c.maxlevel, npu, c.pbuf, op[0].exps, op[1].exps, c.bias, h->sumMode,
+                    alpha, beta, C, ldc);
+            OZB_CHECK(cudaGetLastError());
+        }
     } else {
         c.pbuf = ar.take<double>(pair_handover_doubles(pd.D));
         if (!ar.ok) {

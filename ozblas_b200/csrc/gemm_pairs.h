@@ -30,7 +30,7 @@ struct PairOperand {
     int *tile_lev = nullptr;  // levels in use per tile of the product kernel (null: all)
     int nl = 0, levels = 0;   // lines, levels the planes hold
 };
-constexpr short kExpZero = -32768, kExpNaN = 32767;
+constexpr short kExpZero = -32768, kExpNaN = -32767;  // both far below any exponent, also in a sum
 
 // Where the pair products go.
 enum PairEpi {
@@ -64,7 +64,8 @@ struct PairCall {
     double alpha = 1.0, beta = 0.0;
     void *C = nullptr;
     int ldc = 0;
-    double *pbuf = nullptr;  // kPairStore: np m n entries, else pair_handover_doubles
+    double *pbuf = nullptr;  // kPairStore: np m cn entries, else pair_handover_doubles
+    int col0 = 0, cn = 0;    // kPairStore: the columns of this launch, from a tile boundary (cn = 0: all)
 };
 // Partial sums that one CTA of a fused launch hands to the next, and their flags.
 inline uint64_t pair_handover_doubles(int D) { return (uint64_t)sm_count() * (128 * pair_tile_b(D) + 4); }
@@ -79,10 +80,5 @@ int pair_status(cuozblasHandle_t *h);
 template <typename T>
 int gemm_pairs_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, double alpha, const T *A, int lda,
                     const T *B, int ldb, double beta, T *C, int ldc, int fastMode, int rho, bool *done);
-
-// True when the ordered sum should run in the product kernel's epilogue (at
-// most two CTAs then share a tile's pairs), false when they should be spread
-// over CTAs through a pair buffer: few tiles, short k.
-bool pair_fuse_sum(int m, int n, int k_pad, int np, int D);
 
 }  // namespace ozb

@@ -365,9 +365,12 @@ __global__ void __launch_bounds__(256) k_pair_gemv(int m, int k, int na, int nb,
 // Sum a per-row pair buffer P[(ia*nB+ib)*ldp + row] in order; y = fma(alpha, t, beta*y).
 // NearSum gathers the terms in summation order into `scratch` (np x ldp).
 __global__ void k_sum_rows(int m, int nA, int nB, int maxlevel, double *__restrict__ P, int64_t ldp, int sum_mode,
-                           double alpha, double beta, double *__restrict__ y, double *__restrict__ scratch) {
+                           double alpha, double beta, double *__restrict__ y, double *__restrict__ scratch,
+                           const int *__restrict__ gate, int open) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= m) return;
+    // gated (gemv_fused.cu): only when no flag of the passes before is set
+    if (gate && (gate[1] | gate[2] | gate[open])) return;
     double t = 0.0;
     if (sum_mode == 1) {
         int np = 0;
@@ -387,7 +390,17 @@ int sum_rows_launch(cuozblasHandle_t *h, int m, int nA, int nB, int maxlevel, do
                     double beta, double *y, double *scratch) {
     counted(h);
     k_sum_rows<<<(m + 127) / 128, 128, 0, state(h)->stream>>>(m, nA, nB, maxlevel, P, ldp, h->sumMode, alpha, beta, y,
-                                                               scratch);
+                                                               scratch, nullptr, 0);
+    OZB_CHECK(cudaGetLastError());
+    return CUOZBLAS_STATUS_SUCCESS;
+}
+
+// The same, doing nothing when flags[1], flags[2] or flags[open] is set.
+int sum_rows_if_launch(cuozblasHandle_t *h, int m, int nA, int nB, int maxlevel, double *P, int64_t ldp, double alpha,
+                       double beta, double *y, double *scratch, const int *flags, int open) {
+    counted(h);
+    k_sum_rows<<<(m + 127) / 128, 128, 0, state(h)->stream>>>(m, nA, nB, maxlevel, P, ldp, h->sumMode, alpha, beta, y,
+                                                               scratch, flags, open);
     OZB_CHECK(cudaGetLastError());
     return CUOZBLAS_STATUS_SUCCESS;
 }
@@ -584,7 +597,7 @@ int gemm_plain_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
         } else {
             counted(h);
             k_sum_rows<<<(m + 127) / 128, 128, 0, st->stream>>>(m, nA, nB, maxlevel, P, ldp, h->sumMode, alpha, beta,
-                                                              C, scr);
+                                                              C, scr, nullptr, 0);
         }
         OZB_CHECK(cudaGetLastError());
         ev_record(h, 4);

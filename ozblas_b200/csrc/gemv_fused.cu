@@ -22,6 +22,7 @@
 // k_sum_rows, as for the materialised path.
 #include <stdlib.h>
 
+#include "chain.cuh"
 #include "ozb_device.cuh"
 #include "ozb_internal.h"
 #include "tc05.cuh"
@@ -31,6 +32,7 @@ namespace ozb {
 constexpr int kGvCols = 64;    // columns per warp per pass
 constexpr int kGvWarps = 8;    // warps per block (same 32 rows, different column chunks)
 constexpr int kGvMaxLevels = 8;
+constexpr int kRowBad = 1 << 20;  // above every kLsbBias - lsb
 
 // Pass p: M[p * m + row] = max |r_p| over the row (r_0 = a), with
 // sigma_l = 0.75 2^(rho + tau(M[l * m + row])) for l < p.  M zeroed before.
@@ -152,15 +154,17 @@ constexpr int kGtTile = 32 * kGtCols;  // doubles per tile
 constexpr uint32_t kGtTileBytes = kGtTile * sizeof(double);
 constexpr int kGtSmem = kGtStages * kGtTileBytes + 1024;  // + room to align the ring to 1 KB
 constexpr uint64_t kGtWaitNs = 2000000000ull;  // 2 s without progress
-constexpr int kGtIters = 3;                     // products passes enqueued before the one host read
+constexpr int kGtIters = 3;                     // exact products passes at most
 
-// PRED = false: Ma[row] = max |a| over the row (Ma zeroed before).
+// PRED = false: Ma[row] = max |a| over the row, and state[row] (here the keys) = kLsbBias - the
+// lowest set-bit exponent of its elements (0: all zero; kRowBad: Inf or NaN);
+// both zeroed before.
 // PRED = true: for the rows with state != 0, P[(l * NB + b) * m + row] += sum_j
 // slice_l(a) xs[b][j] on the chain T, and Ma[(l + 1) * m + row] = max |r_{l+1}|.
 // A timed-out wait sets err[0] and ends the block after its loads in flight.
 template <int NB, bool PRED>
 __global__ void __launch_bounds__(256) k_gemv_tma(const __grid_constant__ CUtensorMap tmA, int m, int n, int rho, int cpb,
-                                                  const int *__restrict__ T, const int *__restrict__ state,
+                                                  const int *__restrict__ T, int *__restrict__ state,
                                                   const double *__restrict__ xs, int ldx, double *__restrict__ P,
                                                   double *__restrict__ Ma, int *__restrict__ err) {
     extern __shared__ __align__(1024) unsigned char gt_smem[];
@@ -206,6 +210,7 @@ __global__ void __launch_bounds__(256) k_gemv_tma(const __grid_constant__ CUtens
         for (int b = 0; b < NB; b++) acc[l][b] = 0.0;
     }
     int consumed = 0;  // tiles this thread waited for
+    LazyStats rs;      // PRED = false: this lane's row
     for (int t = 0; t < nt; t++) {
         const int q = t % kGtStages;
         const uint32_t ph = (uint32_t)(t / kGtStages) & 1u;
@@ -214,14 +219,16 @@ __global__ void __launch_bounds__(256) k_gemv_tma(const __grid_constant__ CUtens
         consumed = t + 1;
         const double *tl = tiles + q * kGtTile + warp * 8 * 32;
         const int jb = c0 + t * kGtCols + warp * 8;
-        if (active) {
+        if (!PRED) {  // every lane: the statistics vote over the warp (rows past m read zeros)
+#pragma unroll
+            for (int c = 0; c < 8; c++)
+                if (jb + c < cend) lazy_elem1(rs, tl[c * 32 + lane]);
+        } else if (active) {
 #pragma unroll
             for (int c = 0; c < 8; c++) {
                 if (jb + c < cend) {
                     double r = tl[c * 32 + lane];
-                    if (!PRED) {
-                        mxl[0] = ref_max(mxl[0], fabs(r));
-                    } else {
+                    {
                         double xv[NB];
                         bool xfin = true;  // a zero slice times Inf or NaN still makes NaN
 #pragma unroll
@@ -266,6 +273,15 @@ __global__ void __launch_bounds__(256) k_gemv_tma(const __grid_constant__ CUtens
     }
     __syncthreads();
     if (abort_flag) return;
+    if (!PRED) {
+        // NaN: fmax keeps the finite maximum, as the reference's max does; the
+        // row's chain is then checked by the exact pass (k_gemv_chain)
+        mxl[0] = rs.mx;
+        if (active) {
+            const int key = lazy_bad(rs) ? kRowBad : lazy_key(rs);
+            if (key) atomicMax(&state[row], key);
+        }
+    }
     if (PRED) {
         for (int w = 0; w < kGvWarps; w++) {  // the 8 warps hold the same 32 rows
             if (warp == w) {
@@ -295,18 +311,281 @@ __global__ void __launch_bounds__(256) k_gemv_tma(const __grid_constant__ CUtens
     }
 }
 
+// ---------------------------------------------------------------------------
+// The products pass that almost every row needs once: on the predicted chain
+// the row's lowest set bit gives its first all-zero level z, so a block cuts exactly the levels its 32 rows need, without a test per
+// element and level, two columns interleaved (the cut is a dependent chain of
+// three operations a level), with x's slices in the tile's ring stage.  Per
+// level below z only the largest high word of the remainder is kept, and only
+// until it proves the row's prediction: W[(l + 1) * m + row] = that word.  That
+// word also gives the true tau where the prediction fails (k_gemv_check), and
+// the row takes part in a second pass; `predicted` false: chains may be
+// corrected ones, and every level is cut from its own remainder.
+// 8192 x 8192, 4 slices of x, 5 levels, one B200: the pass 530 -> 269 us.
+// ---------------------------------------------------------------------------
+// HM: the remainders' largest high words too, one level after the other.
+// Otherwise two levels from one base (chain.cuh: RN_g(b) = (b + sigma) - sigma
+// is exact while |b| <= sigma / 3, which holds one level down for rho >= 29),
+// half the depth for the same operations.
+template <int L, int NB, bool HM>
+__device__ __forceinline__ void gv_columns(double (&r)[2], const double (&xv)[2][NB], const double (&sig)[kGvMaxLevels],
+                                           double (&acc)[kGvMaxLevels][NB], unsigned (&hm)[kGvMaxLevels]) {
+    constexpr int G = HM ? 1 : 2;
+#pragma unroll
+    for (int l = 0; l < L; l += G) {
+        double s0[2], s1[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            s0[e] = (r[e] + sig[l]) - sig[l];
+            if (G == 2 && l + 1 < L) {
+                const double rn = (r[e] + sig[l + 1]) - sig[l + 1];
+                s1[e] = rn - s0[e];
+                r[e] = r[e] - rn;
+            } else {
+                r[e] = r[e] - s0[e];
+            }
+            if (HM) hm[l] = max(hm[l], abs_hiword(r[e]));
+        }
+#pragma unroll
+        for (int e = 0; e < 2; e++)
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                acc[l][b] = fma(s0[e], xv[e][b], acc[l][b]);  // exact
+                if (G == 2 && l + 1 < L) acc[l + 1][b] = fma(s1[e], xv[e][b], acc[l + 1][b]);
+            }
+    }
+}
+
+template <int NB>
+constexpr int gv_fast_smem() {
+    return kGtStages * (kGtTile + NB * kGtCols) * (int)sizeof(double) + 1024;
+}
+
+template <int NB>
+__global__ void __launch_bounds__(256, NB <= 4 ? 2 : 1)
+    k_gemv_fast(const __grid_constant__ CUtensorMap tmA, int m, int n, int rho, int cpb, int nB, bool predicted,
+                const int *__restrict__ state, const int *__restrict__ T, const int *__restrict__ Z,
+                const double *__restrict__ xs, int ldx, double *__restrict__ P, unsigned *__restrict__ W,
+                int *__restrict__ err) {
+    extern __shared__ __align__(1024) unsigned char gt_smem[];
+    double *tiles = reinterpret_cast<double *>(gt_smem + ((1024 - (tc::smem_u32(gt_smem) & 1023)) & 1023));
+    double *xtiles = tiles + kGtStages * kGtTile;  // [stage][slice][column]
+    __shared__ __align__(8) uint64_t full[kGtStages], empty[kGtStages];
+    __shared__ int abort_flag, never;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int row0 = blockIdx.x * 32, row = row0 + lane;
+    const bool active = row < m && state[row] != 0;
+    if (!__syncthreads_or(active)) return;  // block-uniform: every row is proven
+    const int c0 = blockIdx.y * cpb;
+    const int cend = c0 + cpb < n ? c0 + cpb : n;
+    const int nt = (cend - c0 + kGtCols - 1) / kGtCols;
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < kGtStages; q++) {
+            tc::mbar_init(&full[q], 1);
+            tc::mbar_init(&empty[q], kGvWarps);
+        }
+        abort_flag = 0;
+        never = 0;
+        tc::fence_mbar_init();
+    }
+    // slices of x beyond nB multiply as zeros
+    for (int i = threadIdx.x; i < kGtStages * NB * kGtCols; i += blockDim.x)
+        if ((i / kGtCols) % NB >= nB) xtiles[i] = 0.0;
+    __syncthreads();
+    auto load = [&](int t) {
+        const int q = t % kGtStages, col = c0 + t * kGtCols;
+        // the slices' rows hold ldx >= n values, ldx even: the copied columns end there
+        const uint32_t xb = (uint32_t)(ldx - col < kGtCols ? ldx - col : kGtCols) * 8u;
+        tc::mbar_arrive_expect_tx(&full[q], kGtTileBytes + xb * (uint32_t)nB);
+        tc::tma_load_2d(tiles + q * kGtTile, &tmA, &full[q], row0, col);
+        for (int b = 0; b < nB; b++)
+            tc::bulk_load(xtiles + (q * NB + b) * kGtCols, xs + (size_t)b * ldx + col, xb, &full[q]);
+    };
+    int issued = 0;
+    if (threadIdx.x == 0) {
+        tc::prefetch_tmap(&tmA);
+        for (; issued < nt && issued < kGtStages; issued++) load(issued);
+    }
+    // this row's chain and level count (rows past m or proven: none)
+    const int z = active ? Z[row] : 0;
+    double sig[kGvMaxLevels], acc[kGvMaxLevels][NB];
+    unsigned hm[kGvMaxLevels], thr[kGvMaxLevels];
+#pragma unroll
+    for (int l = 0; l < kGvMaxLevels; l++) {
+        const int tau = active ? T[(size_t)l * m + row] : 0;
+        sig[l] = 0.75 * pow2(rho + tau);
+        // level l - 1 is proven by a remainder whose high word exceeds that of 2^(tau_l - 1)
+        if (l > 0) thr[l - 1] = l <= z ? (unsigned)(dbits(pow2(tau - 1)) >> 32) : 0u;
+        hm[l] = 0;
+#pragma unroll
+        for (int b = 0; b < NB; b++) acc[l][b] = 0.0;
+    }
+    thr[kGvMaxLevels - 1] = 0u;
+    int L = __reduce_max_sync(0xffffffffu, z + 1);
+    if (L > kGvMaxLevels) L = kGvMaxLevels;  // such a row is not proven: the exact pass decides
+    bool track = true;
+    int consumed = 0;
+    for (int t = 0; t < nt; t++) {
+        const int q = t % kGtStages;
+        const uint32_t ph = (uint32_t)(t / kGtStages) & 1u;
+        if (!__all_sync(0xffffffffu, tc::mbar_wait(&full[q], ph, &abort_flag, err, 1, kGtWaitNs))) break;
+        consumed = t + 1;
+        const double *tl = tiles + q * kGtTile + warp * 8 * 32;
+        const double *xl = xtiles + q * NB * kGtCols + warp * 8;
+        const int jb = c0 + t * kGtCols + warp * 8;
+        const int nc = cend - jb < 8 ? cend - jb : 8;  // columns of this warp in the range
+#pragma unroll 1
+        for (int c = 0; c < nc; c += 2) {
+            const bool two = c + 1 < nc;
+            double r[2] = {tl[c * 32 + lane], two ? tl[(c + 1) * 32 + lane] : 0.0}, xv[2][NB];
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                const double2 v = *reinterpret_cast<const double2 *>(xl + b * kGtCols + c);
+                xv[0][b] = v.x;
+                xv[1][b] = two ? v.y : 0.0;
+            }
+            if (track) {
+                switch (L) {
+                case 1: gv_columns<1, NB, true>(r, xv, sig, acc, hm); break;
+                case 2: gv_columns<2, NB, true>(r, xv, sig, acc, hm); break;
+                case 3: gv_columns<3, NB, true>(r, xv, sig, acc, hm); break;
+                case 4: gv_columns<4, NB, true>(r, xv, sig, acc, hm); break;
+                case 5: gv_columns<5, NB, true>(r, xv, sig, acc, hm); break;
+                case 6: gv_columns<6, NB, true>(r, xv, sig, acc, hm); break;
+                default: gv_columns<8, NB, true>(r, xv, sig, acc, hm); break;
+                }
+            } else {
+                switch (L) {
+                case 1: gv_columns<1, NB, false>(r, xv, sig, acc, hm); break;
+                case 2: gv_columns<2, NB, false>(r, xv, sig, acc, hm); break;
+                case 3: gv_columns<3, NB, false>(r, xv, sig, acc, hm); break;
+                case 4: gv_columns<4, NB, false>(r, xv, sig, acc, hm); break;
+                case 5: gv_columns<5, NB, false>(r, xv, sig, acc, hm); break;
+                case 6: gv_columns<6, NB, false>(r, xv, sig, acc, hm); break;
+                default: gv_columns<8, NB, false>(r, xv, sig, acc, hm); break;
+                }
+            }
+        }
+        if (track) {  // stop when this warp's own elements prove every level of its rows
+            bool open = false;
+#pragma unroll
+            for (int l = 0; l < kGvMaxLevels - 1; l++) open |= l < z && hm[l] <= thr[l];
+            track = __any_sync(0xffffffffu, open) || rho < 29 || !predicted;
+        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&empty[q]);
+        int rok = 1;
+        if (threadIdx.x == 0 && issued < nt) {
+            rok = tc::mbar_wait(&empty[q], ph, &abort_flag, err, 2, kGtWaitNs);
+            if (rok) load(issued++);
+        }
+        if (!__shfl_sync(0xffffffffu, rok, 0)) break;  // warp 0 leaves together
+    }
+    if (threadIdx.x == 0) {  // after a timeout: let the loads in flight land before the block ends
+        for (int t = consumed; t < issued; t++)
+            if (!tc::mbar_wait(&full[t % kGtStages], (uint32_t)(t / kGtStages) & 1u, &never, err, 3, kGtWaitNs)) break;
+    }
+    __syncthreads();
+    if (abort_flag) return;
+    // the 8 warps hold the same 32 rows: their partial products through the ring's memory
+    double *ps = tiles;  // [warp][level][slice][row]; 8 x 8 x NB x 32 doubles would not fit at once: level by level
+#pragma unroll
+    for (int l = 0; l < kGvMaxLevels; l++) {
+        if (l >= L) break;  // uniform over the block: every warp has the same rows
+        __syncthreads();
+#pragma unroll
+        for (int b = 0; b < NB; b++) ps[(warp * NB + b) * 32 + lane] = acc[l][b];
+        __syncthreads();
+        for (int i = threadIdx.x; i < nB * 32; i += blockDim.x) {
+            double v = 0.0;
+#pragma unroll
+            for (int w = 0; w < kGvWarps; w++) v += ps[w * NB * 32 + i];
+            const int rr = row0 + (i & 31);
+            if (rr < m && state[rr] != 0) atomicAdd(&P[((size_t)l * nB + (i >> 5)) * m + rr], v);
+        }
+    }
+    if (active)
+        for (int l = 0; l < kGvMaxLevels - 1; l++)
+            if (l < z) {
+                unsigned h = 0;
+#pragma unroll
+                for (int j = 0; j < kGvMaxLevels; j++)
+                    if (j == l) h = hm[j];
+                if (h) atomicMax(&W[(size_t)(l + 1) * m + row], h);
+            }
+}
+
+// After a pass: a row is proven when every level below its z left a remainder
+// with the tau that the chain has for it (or nothing: then z was too large).
+// A row whose chain breaks at level l gets the true tau_l, a prediction beyond
+// it, the z that follows and another pass.  Rows without a z within the levels
+// held, or whose tau depends on a low word, are left to the exact pass (Z =
+// kGvMaxLevels).  out[0] = the largest
+// z of the proven rows, out[open] counts the others.
+__global__ void k_gemv_check(int m, int rho, unsigned *__restrict__ W, int *__restrict__ T, int *__restrict__ Z,
+                             const int *__restrict__ key, int *__restrict__ state, double *__restrict__ P, int np,
+                             int *__restrict__ out, int open) {
+    const int row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row >= m || state[row] == 0) return;
+    int z = Z[row], bad = -1;
+    unsigned h = 0;
+    for (int l = 1; l <= z && z < kGvMaxLevels; l++) {
+        h = W[(size_t)l * m + row];
+        if (h == 0) {  // grids are normal, so nothing hides below the high word
+            z = l - 1;
+            break;
+        }
+        if (h <= (unsigned)(dbits(pow2(T[(size_t)l * m + row] - 1)) >> 32)) {
+            bad = l;
+            break;
+        }
+    }
+    if (z < kGvMaxLevels && bad < 0) {
+        state[row] = 0;
+        atomicMax(&out[0], z);
+        return;
+    }
+    atomicAdd(&out[open], 1);
+    int nz = kGvMaxLevels;
+    // 2^e <= v < 2^(e + 1).  At a power of two's high word v is that power when the
+    // remainders, multiples of the lowest set bit, cannot differ below it (the
+    // usual case: a last level with one bit left); otherwise tau is open.
+    const int e = (int)(h >> 20) - 1023, low = kLsbBias - key[row];
+    const bool power = (h & 0xfffffu) == 0;
+    if (bad > 0 && (!power || low >= e - 20)) {
+        const int d = 54 - rho;
+        int tau = power ? e : e + 1;
+        const int G = rho + tau - 53, num = G - low;
+        nz = bad + (num <= 0 ? 0 : (num + d - 1) / d);
+        if (nz > kGvMaxLevels || G - (nz - bad) * d < -1000) nz = kGvMaxLevels;
+        if (nz < kGvMaxLevels)
+            for (int l = bad; l < kGvMaxLevels; l++, tau -= d) T[(size_t)l * m + row] = tau;
+    }
+    Z[row] = nz;
+    for (int l = 1; l < kGvMaxLevels; l++) W[(size_t)l * m + row] = 0;
+    for (int i = 0; i < np; i++) P[(size_t)i * m + row] = 0.0;
+}
+
 // it < 0: the predicted chains T from the row maxima Ma[0..m), every row
-// unproven.  it >= 0: the proof after products pass `it` (see above).  out[0]
+// unproven (state 1), and Z[row] the first all-zero level that the lowest set
+// bit in keys[row] gives (kGvMaxLevels where the prediction does not apply).  it >= 0: the proof after products pass `it` (see above).  out[0]
 // = max over proven rows of z - 1 (z = the first level with a zero remainder
 // maximum), out[1] = 1 when a row has no zero level within the capacity,
 // out[2] is the wait-error flag of the passes, out[4 + it] = rows whose
 // chain broke in pass `it`.
 __global__ void k_gemv_chain(int m, int rho, int it, double *__restrict__ Ma, int *__restrict__ T,
-                             int *__restrict__ state, double *__restrict__ P, int np, int *__restrict__ out) {
+                             int *__restrict__ state, int *__restrict__ Z, const int *__restrict__ keys,
+                             double *__restrict__ P, int np, int *__restrict__ out) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= m) return;
     if (it < 0) {
         int tau = tau_rule(Ma[row]);
+        const int key = keys[row], d = 54 - rho, G0 = rho + tau - 53;
+        const int num = key == 0 ? 0 : G0 - (kLsbBias - key);
+        int z = num <= 0 ? 0 : (num + d - 1) / d;
+        // sigma, every grid and every threshold normal
+        if (key >= kRowBad || rho + tau > 1000 || G0 - z * d < -1000 || z > kGvMaxLevels) z = kGvMaxLevels;
+        Z[row] = z;
         for (int l = 0; l < kGvMaxLevels; l++, tau += rho - 54) T[(size_t)l * m + row] = tau;
         state[row] = 1;
         return;
@@ -339,7 +618,7 @@ __global__ void k_gemv_chain(int m, int rho, int it, double *__restrict__ Ma, in
 
 template <int NB, bool PRED>
 static int launch_gt(dim3 grid, cudaStream_t s, const CUtensorMap &tm, int m, int n, int rho, int cpb, const int *T,
-                     const int *state, const double *xs, int ldx, double *P, double *Ma, int *err) {
+                     int *state, const double *xs, int ldx, double *P, double *Ma, int *err) {
     static std::atomic<uint64_t> attr{0};  // devices already opted in, per instantiation
     if (smem_optin((const void *)k_gemv_tma<NB, PRED>, kGtSmem, attr) != cudaSuccess)
         return CUOZBLAS_STATUS_CUDA_ERROR;
@@ -348,7 +627,7 @@ static int launch_gt(dim3 grid, cudaStream_t s, const CUtensorMap &tm, int m, in
 }
 
 static int launch_gt_pred(int nB, dim3 grid, cudaStream_t s, const CUtensorMap &tm, int m, int n, int rho, int cpb,
-                          const int *T, const int *state, const double *xs, int ldx, double *P, double *Ma, int *err) {
+                          const int *T, int *state, const double *xs, int ldx, double *P, double *Ma, int *err) {
     switch (nB) {
     case 1: return launch_gt<1, true>(grid, s, tm, m, n, rho, cpb, T, state, xs, ldx, P, Ma, err);
     case 2: return launch_gt<2, true>(grid, s, tm, m, n, rho, cpb, T, state, xs, ldx, P, Ma, err);
@@ -359,6 +638,17 @@ static int launch_gt_pred(int nB, dim3 grid, cudaStream_t s, const CUtensorMap &
     case 7: return launch_gt<7, true>(grid, s, tm, m, n, rho, cpb, T, state, xs, ldx, P, Ma, err);
     default: return launch_gt<8, true>(grid, s, tm, m, n, rho, cpb, T, state, xs, ldx, P, Ma, err);
     }
+}
+
+template <int NB>
+static int launch_gt_fast(dim3 grid, cudaStream_t s, const CUtensorMap &tm, int m, int n, int rho, int cpb, int nB,
+                          bool predicted, const int *state, const int *T, const int *Z, const double *xs, int ldx, double *P, unsigned *W, int *err) {
+    static std::atomic<uint64_t> attr{0};
+    if (smem_optin((const void *)k_gemv_fast<NB>, gv_fast_smem<NB>(), attr) != cudaSuccess)
+        return CUOZBLAS_STATUS_CUDA_ERROR;
+    k_gemv_fast<NB><<<grid, 256, gv_fast_smem<NB>(), s>>>(tm, m, n, rho, cpb, nB, predicted, state, T, Z, xs, ldx, P, W,
+                                                             err);
+    return cudaGetLastError() == cudaSuccess ? CUOZBLAS_STATUS_SUCCESS : CUOZBLAS_STATUS_CUDA_ERROR;
 }
 
 // y = fma(alpha, t, beta y) for the 'n' GEMV with the plain form's split
@@ -378,8 +668,6 @@ int gemv_fused_n(cuozblasHandle_t *h, int m, int n, const double *A, int lda, co
         ar.release(mk);
         return CUOZBLAS_STATUS_NOT_SUPPORTED;
     }
-    OZB_CHECK(cudaMemsetAsync(M, 0, sizeof(double) * (kGvMaxLevels + 1) * m, st->stream));
-    OZB_CHECK(cudaMemsetAsync(gmax, 0, sizeof(double) * (kGvMaxLevels + 2), st->stream));
     const dim3 grid((m + 31) / 32, (n + kGvWarps * kGvCols - 1) / (kGvWarps * kGvCols));
     auto finish_sum = [&](int nA) -> int {
         int maxlevel = (nA - 1) + (nB - 1);
@@ -395,44 +683,88 @@ int gemv_fused_n(cuozblasHandle_t *h, int m, int n, const double *A, int lda, co
     CUtensorMap tm;
     if (!state(h)->env.gemv_levels && make_map_f64(&tm, A, m, n, lda, 32, kGtCols) == CUOZBLAS_STATUS_SUCCESS) {
         const uint64_t mk2 = ar.mark();
+        // one zeroed block: Ma, the rows' keys, W and the flags
+        const uint64_t zfrom = ar.mark();
         double *Ma = ar.take<double>((uint64_t)(kGvMaxLevels + 1) * m);
+        int *keys = ar.take<int>((uint64_t)m);
+        unsigned *W = ar.take<unsigned>((uint64_t)kGvMaxLevels * m);
+        int *flags = ar.take<int>(6 + kGtIters);  // zmax, capacity, err, pad, rows left per pass (2 fast, the exact ones)
+        const uint64_t zto = ar.mark();
         int *T = ar.take<int>((uint64_t)kGvMaxLevels * m);
+        int *Z = ar.take<int>((uint64_t)m);
         int *rstate = ar.take<int>((uint64_t)m);
-        int *flags = ar.take<int>(4 + kGtIters);  // zmax, capacity, err, pad, failures per pass
         if (ar.ok) {
             const int rb = (m + 31) / 32, ctiles = (n + kGtCols - 1) / kGtCols;
-            int gy = (sm_count() * 8 + rb - 1) / rb;  // about eight blocks per SM in all
+            // about eight blocks per SM in all, up to twelve where that fills the last wave
+            // of two blocks per SM better (8192 rows: 256 x 8 blocks leave 1 % of it idle, x 5 14 %)
+            const int sms = sm_count();
+            int gy = (sms * 8 + rb - 1) / rb;
+            if (gy < ctiles) {
+                const int64_t slots = 2 * (int64_t)sms;
+                auto waste = [&](int g) {
+                    const int64_t bl = (int64_t)rb * g;
+                    return (double)((bl + slots - 1) / slots * slots - bl) / (double)bl;
+                };
+                const int top = (sms * 14 + rb - 1) / rb;
+                for (int g = gy + 1; g <= top && g <= ctiles; g++)
+                    if (waste(g) < waste(gy) - 0.02) gy = g;
+            }
             gy = gy < 1 ? 1 : (gy > ctiles ? ctiles : gy);
             const int cpb = (ctiles + gy - 1) / gy * kGtCols;
             const dim3 g2(rb, (n + cpb - 1) / cpb);
             int *err = flags + 2;
-            OZB_CHECK(cudaMemsetAsync(Ma, 0, sizeof(double) * (kGvMaxLevels + 1) * m, st->stream));
+            const uint64_t z0 = (zfrom + kArenaAlign - 1) / kArenaAlign * kArenaAlign;
+            OZB_CHECK(cudaMemsetAsync(h->devWork + z0, 0, zto - z0, st->stream));
             OZB_CHECK(cudaMemsetAsync(P, 0, sizeof(double) * kGvMaxLevels * nB * m, st->stream));
-            OZB_CHECK(cudaMemsetAsync(flags, 0, sizeof(int) * (4 + kGtIters), st->stream));
             counted(h);
-            OZB_TRY((launch_gt<1, false>(g2, st->stream, tm, m, n, rho, cpb, nullptr, nullptr, nullptr, 0, nullptr, Ma,
+            OZB_TRY((launch_gt<1, false>(g2, st->stream, tm, m, n, rho, cpb, nullptr, keys, nullptr, 0, nullptr, Ma,
                                          err)));
             counted(h);
-            k_gemv_chain<<<(m + 255) / 256, 256, 0, st->stream>>>(m, rho, -1, Ma, T, rstate, P, kGvMaxLevels * nB,
+            k_gemv_chain<<<(m + 255) / 256, 256, 0, st->stream>>>(m, rho, -1, Ma, T, rstate, Z, keys, P, kGvMaxLevels * nB,
                                                                   flags);
             OZB_CHECK(cudaGetLastError());
-            for (int it = 0; it < kGtIters; it++) {
+            for (int it = 0; it < 2; it++) {
                 counted(h);
-                OZB_TRY(launch_gt_pred(nB, g2, st->stream, tm, m, n, rho, cpb, T, rstate, xs, ldx, P, Ma, err));
+                OZB_TRY(nB <= 4 ? launch_gt_fast<4>(g2, st->stream, tm, m, n, rho, cpb, nB, it == 0, rstate, T, Z, xs, ldx,
+                                                    P, W, err)
+                                : launch_gt_fast<8>(g2, st->stream, tm, m, n, rho, cpb, nB, it == 0, rstate, T, Z, xs, ldx,
+                                                    P, W, err));
                 counted(h);
-                k_gemv_chain<<<(m + 255) / 256, 256, 0, st->stream>>>(m, rho, it, Ma, T, rstate, P,
-                                                                      kGvMaxLevels * nB, flags);
+                k_gemv_check<<<(m + 255) / 256, 256, 0, st->stream>>>(m, rho, W, T, Z, keys, rstate, P, kGvMaxLevels * nB,
+                                                                      flags, 4 + it);
                 OZB_CHECK(cudaGetLastError());
             }
-            OZB_CHECK(cudaMemcpyAsync(st->h_ints, flags, sizeof(int) * (4 + kGtIters), cudaMemcpyDeviceToHost,
-                                      st->stream));
-            OZB_CHECK(cudaStreamSynchronize(st->stream));
-            if (st->h_ints[2] != 0) return CUOZBLAS_STATUS_DEVICE_TIMEOUT;
-            if (st->h_ints[1] == 0 && st->h_ints[4 + kGtIters - 1] == 0) {  // every chain proven
-                const int zmax = st->h_ints[0];
+            // The sum where the second pass proves the rest, and one host read; exact passes only when
+            // it does not.  The sum runs over every level held (those past nA add zeros), so it needs
+            // no count.
+            const int lv = maxS < kGvMaxLevels ? maxS : kGvMaxLevels;
+            const bool early = fastMode == 0;
+            for (int it = 0; it <= kGtIters; it++) {
+                const int open = 5 + it;  // rows left by the second fast pass, by the exact passes
+                if (it > 0) {
+                    counted(h);
+                    OZB_TRY(launch_gt_pred(nB, g2, st->stream, tm, m, n, rho, cpb, T, rstate, xs, ldx, P, Ma, err));
+                    counted(h);
+                    k_gemv_chain<<<(m + 255) / 256, 256, 0, st->stream>>>(m, rho, it + 1, Ma, T, rstate, Z, keys, P,
+                                                                          kGvMaxLevels * nB, flags);
+                    OZB_CHECK(cudaGetLastError());
+                }
+                if (early) OZB_TRY(sum_rows_if_launch(h, m, lv, nB, lv + nB - 2, P, m, alpha, beta, y, scratch, flags, open));
+                OZB_CHECK(cudaMemcpyAsync(st->h_ints, flags, sizeof(int) * (6 + kGtIters), cudaMemcpyDeviceToHost,
+                                          st->stream));
+                OZB_CHECK(cudaStreamSynchronize(st->stream));
+                if (st->h_ints[2] != 0) return CUOZBLAS_STATUS_DEVICE_TIMEOUT;
+                if (st->h_ints[1] != 0) break;  // a row has no zero level within the capacity
+                if (st->h_ints[open] != 0) continue;
+                const int zmax = st->h_ints[0];  // every chain proven
                 const int c = (zmax < 1 ? 1 : zmax) + 1;  // the lines rule's count
                 const int nA = c < maxS ? c : maxS;
-                if (nA <= kGvMaxLevels) return finish_sum(nA);
+                if (nA > kGvMaxLevels) break;
+                if (early) {
+                    *nA_out = nA;
+                    return CUOZBLAS_STATUS_SUCCESS;
+                }
+                return finish_sum(nA);
             }
         }
         ar.release(mk2);
@@ -442,6 +774,8 @@ int gemv_fused_n(cuozblasHandle_t *h, int m, int n, const double *A, int lda, co
     // remainder zero returns at once); then the count rule of split_lines_count
     // (level 0 always; the level that leaves every remainder zero counts; at
     // most maxS) from the passes' maxima
+    OZB_CHECK(cudaMemsetAsync(M, 0, sizeof(double) * (kGvMaxLevels + 1) * m, st->stream));
+    OZB_CHECK(cudaMemsetAsync(gmax, 0, sizeof(double) * (kGvMaxLevels + 2), st->stream));
     const int last = maxS < kGvMaxLevels ? maxS : kGvMaxLevels;
     for (int p = 0; p <= last; p++) {
         counted(h);

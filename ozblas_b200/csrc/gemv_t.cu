@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(1024) k_split_vector_one(int n, const double *
     if (tid == 0 && blockIdx.x == 0) *info = VecSplitInfo{s, nz, tau0, glast, bad ? 1 : 0};
 }
 
-constexpr int kSplitOneMax = 16384;
+constexpr int kSplitOneMax = kSplitVectorSmallMax;
 
 static int split_vector_one(cuozblasHandle_t *h, int n, const double *x, int rho, int maxS, double *out, int ldo,
                             VecSplitInfo *info) {
@@ -139,6 +139,17 @@ static int split_vector_one(cuozblasHandle_t *h, int n, const double *x, int rho
     else
         k_split_vector_one<16><<<16, 1024, 0, s>>>(n, x, rho, maxS, out, ldo, info);
     OZB_CHECK(cudaGetLastError());
+    return CUOZBLAS_STATUS_SUCCESS;
+}
+
+// The same for a caller that needs the count on the host.
+int split_vector_small(cuozblasHandle_t *h, int n, const double *x, int rho, int maxS, double *out, int ldo, int *ns) {
+    State *st = state(h);
+    VecSplitInfo *info = reinterpret_cast<VecSplitInfo *>(st->d_ints + 16);
+    OZB_TRY(split_vector_one(h, n, x, rho, maxS, out, ldo, info));
+    OZB_CHECK(cudaMemcpyAsync(st->h_ints, info, sizeof(int), cudaMemcpyDeviceToHost, st->stream));
+    OZB_CHECK(cudaStreamSynchronize(st->stream));
+    *ns = st->h_ints[0];
     return CUOZBLAS_STATUS_SUCCESS;
 }
 
@@ -206,39 +217,50 @@ __global__ void __launch_bounds__(256) k_gemv_t_stats(int nl, int k, const doubl
                         lb, 0};
 }
 
-// E elements at once: their slices (levels 0..L-1) against x's; hm[s] the
-// largest high word of the remainder after level s.  The levels are a
-// dependent chain of 3 operations each, so the elements are interleaved.
-template <int L, int NB, int E, bool HM>
+// E elements at once: their slices (levels 0..L-1) against x's, interleaved.
+// STEP: level by level, with hm[s] the largest high word of the remainder
+// after level s.  Otherwise two levels from one base, half the depth for the
+// same operations (chain.cuh; holds on the predicted chain for rho >= 29).
+template <int L, int NB, int E, bool STEP>
 __device__ __forceinline__ void gt_elements(double (&r)[E], const double (&xb)[E][NB], const double (&sig)[kGtLevels],
                                             double (&P)[kGtLevels][NB], unsigned (&hm)[kGtLevels]) {
+    constexpr int G = STEP ? 1 : 2;
 #pragma unroll
-    for (int s = 0; s < L; s++) {
-        double sl[E];
+    for (int s = 0; s < L; s += G) {
+        double s0[E], s1[E];
 #pragma unroll
         for (int e = 0; e < E; e++) {
-            sl[e] = (r[e] + sig[s]) - sig[s];
-            r[e] = r[e] - sl[e];
-            if (HM) hm[s] = max(hm[s], abs_hiword(r[e]));
+            s0[e] = (r[e] + sig[s]) - sig[s];
+            if (G == 2 && s + 1 < L) {
+                const double rn = (r[e] + sig[s + 1]) - sig[s + 1];
+                s1[e] = rn - s0[e];
+                r[e] = r[e] - rn;
+            } else {
+                r[e] = r[e] - s0[e];
+            }
+            if (STEP) hm[s] = max(hm[s], abs_hiword(r[e]));
         }
 #pragma unroll
         for (int e = 0; e < E; e++)
 #pragma unroll
-            for (int b = 0; b < NB; b++) P[s][b] = fma(sl[e], xb[e][b], P[s][b]);
+            for (int b = 0; b < NB; b++) {
+                P[s][b] = fma(s0[e], xb[e][b], P[s][b]);
+                if (G == 2 && s + 1 < L) P[s + 1][b] = fma(s1[e], xb[e][b], P[s + 1][b]);
+            }
     }
 }
-template <int NB, int E, bool HM>
+template <int NB, int E, bool STEP>
 __device__ __forceinline__ void gt_elements(int L, double (&r)[E], const double (&xb)[E][NB],
                                             const double (&sig)[kGtLevels], double (&P)[kGtLevels][NB],
                                             unsigned (&hm)[kGtLevels]) {
     switch (L) {  // uniform over a line
         case 0: break;
-        case 1: gt_elements<1, NB, E, HM>(r, xb, sig, P, hm); break;
-        case 2: gt_elements<2, NB, E, HM>(r, xb, sig, P, hm); break;
-        case 3: gt_elements<3, NB, E, HM>(r, xb, sig, P, hm); break;
-        case 4: gt_elements<4, NB, E, HM>(r, xb, sig, P, hm); break;
-        case 5: gt_elements<5, NB, E, HM>(r, xb, sig, P, hm); break;
-        default: gt_elements<6, NB, E, HM>(r, xb, sig, P, hm); break;
+        case 1: gt_elements<1, NB, E, STEP>(r, xb, sig, P, hm); break;
+        case 2: gt_elements<2, NB, E, STEP>(r, xb, sig, P, hm); break;
+        case 3: gt_elements<3, NB, E, STEP>(r, xb, sig, P, hm); break;
+        case 4: gt_elements<4, NB, E, STEP>(r, xb, sig, P, hm); break;
+        case 5: gt_elements<5, NB, E, STEP>(r, xb, sig, P, hm); break;
+        default: gt_elements<6, NB, E, STEP>(r, xb, sig, P, hm); break;
     }
 }
 
@@ -388,7 +410,7 @@ __device__ __forceinline__ void gt_lines(int nl, int k, const double *__restrict
 #pragma unroll
                 for (int s = 0; s + 1 < kGtLevels; s++)
                     if (s + 1 < pl.L) open |= !__any_sync(0xffffffffu, hm[s] > thr(s));
-                track = open;
+                track = open || rho < 29;
             }
         } else {
             gt_elements<NB, 2, false>(pl.L, r, xb, pl.sig, P, hm);
@@ -461,7 +483,7 @@ __device__ __forceinline__ void gt_lines(int nl, int k, const double *__restrict
             double xb[1][NB], r[1] = {__ldg(a + j)};
 #pragma unroll
             for (int b = 0; b < NB; b++) xb[0][b] = b < nB ? xs[(size_t)b * ldx + j] : 0.0;
-            gt_elements<NB, 1, false>(pl.L, r, xb, pl.sig, P, hm);
+            gt_elements<NB, 1, true>(pl.L, r, xb, pl.sig, P, hm);
         }
     }
     double t = 0.0;

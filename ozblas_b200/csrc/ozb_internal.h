@@ -227,6 +227,10 @@ int transpose_f32(cuozblasHandle_t *h, int rows, int cols, const float *A, int l
 // Transpose rows x cols (column-major, ld) into cols x rows (ldo).
 int transpose(cuozblasHandle_t *h, int rows, int cols, const double *A, int lda, double *out, int ldo);
 // Vector split with one global tau chain (n-vector).  Writes ns slices of ldo.
+// Vectors of at most kSplitVectorSmallMax (ldo included) go to split_vector_small
+// (gemv_t.cu: one launch without grid barriers; 8192 elements 19 -> 10 us).
+constexpr int kSplitVectorSmallMax = 16384;
+int split_vector_small(cuozblasHandle_t *h, int n, const double *x, int rho, int maxS, double *out, int ldo, int *ns);
 int split_vector(cuozblasHandle_t *h, int n, const double *x, int rho, int maxS, double *out, int ldo, int *ns);
 // CSR row split; slices laid out ns x nnz.  shift divides sigma.
 int split_csr_count(cuozblasHandle_t *h, int m, const double *val, const int *rowptr, int epsmode, int shift,
@@ -270,6 +274,8 @@ int gemm_q_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, cons
 // ---- skinny forms (gemm_plain.cu, gemv_fused.cu, gemv_t.cu) ----
 int sum_rows_launch(cuozblasHandle_t *h, int m, int nA, int nB, int maxlevel, double *P, int64_t ldp, double alpha,
                     double beta, double *y, double *scratch);
+int sum_rows_if_launch(cuozblasHandle_t *h, int m, int nA, int nB, int maxlevel, double *P, int64_t ldp, double alpha,
+                       double beta, double *y, double *scratch, const int *flags, int open);
 int gemv_fused_n(cuozblasHandle_t *h, int m, int n, const double *A, int lda, const double *xs, int ldx, int nB,
                  int rho, int maxS, int fastMode, double alpha, double beta, double *y, int *nA_out);
 int gemv_t_fused(cuozblasHandle_t *h, int nl, int k, const double *A, int lda, const double *x, double alpha,

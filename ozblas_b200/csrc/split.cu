@@ -384,6 +384,8 @@ static int split_vector_t(cuozblasHandle_t *h, int n, const double *x, int rho, 
 }
 
 int split_vector(cuozblasHandle_t *h, int n, const double *x, int rho, int maxS, double *out, int ldo, int *ns) {
+    if (n <= kSplitVectorSmallMax && ldo <= kSplitVectorSmallMax)
+        return split_vector_small(h, n, x, rho, maxS, out, ldo, ns);
     return split_vector_t<double>(h, n, x, rho, maxS, out, ldo, nullptr, ns);
 }
 
