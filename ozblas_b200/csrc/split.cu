@@ -11,6 +11,8 @@
 // for a line, the count is min(maxS, max(1, max_lines z) + 1).
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "ozb_device.cuh"
 #include "ozb_internal.h"
 
@@ -395,50 +397,122 @@ int split_vector_f32(cuozblasHandle_t *h, int n, const double *x, int rho, int m
 }
 
 // ---------------------------------------------------------------------------
-// CSR row split (src/cpu/ozblas_split.cpp:779-815, driver :875-928): one warp
-// per row; rho from the row's nnz; sigma divided by shift.  Remainders live
-// in `rem` (nnz doubles).  COUNT atomicMax(z); WRITE writes ns slices of nnz.
+// CSR row split (src/cpu/ozblas_split.cpp:779-815, driver :875-928): rho from
+// the row's nnz; sigma divided by shift.  The count pass leaves the largest
+// z in *zmax, the write pass writes `levels` slices of nnz.
+//
+// W lanes hold a row and kCsrHeld entries each in registers, W so that this
+// covers twice the mean row length (a longer row keeps its remainders in
+// `rem`, nnz doubles): the level's sigma is computed by every lane of a row,
+// so wider rows only repeat it.  The counts are folded per block: one atomic
+// per row on the one counter was the bound (10^6 rows of 7 with it and a warp
+// per row: 675 us, of which the 56 MB of values account for 9; 8 lanes per
+// row 94, 4 lanes 55; the writing pass 385 -> 63).
 // ---------------------------------------------------------------------------
-template <bool WRITE>
+constexpr int kCsrHeld = 4;  // entries of a row per lane in registers
+
+template <bool WRITE, int W>
 __global__ void __launch_bounds__(256) k_split_csr(int m, const double *__restrict__ val,
                                                    const int *__restrict__ rowptr, int epsmode, int shift,
                                                    int levels, double *__restrict__ rem, double *__restrict__ out,
                                                    int64_t ldo, int *__restrict__ zmax) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= m) return;
-    const int lo = rowptr[warp], hi = rowptr[warp + 1];
-    double mx = 0.0;
-    for (int i = lo + lane; i < hi; i += 32) {
-        const double v = val[i];
-        rem[i] = v;
-        mx = ref_max(mx, fabs(v));
-    }
-    for (int o = 16; o > 0; o >>= 1) mx = ref_max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    int z = levels;
-    if (hi > lo) {
+    __shared__ int zsh[8];
+    const int lane = threadIdx.x & 31, sub = lane % W;
+    const unsigned rows_lanes = W == 32 ? 0xffffffffu : ((1u << W) - 1u) << (lane - sub);  // this row's lanes
+    const int64_t nrows = (int64_t)gridDim.x * (256 / W);
+    int zbest = 0;
+    for (int64_t row = (int64_t)blockIdx.x * (256 / W) + threadIdx.x / W; row < m; row += nrows) {
+        const int lo = rowptr[row], hi = rowptr[row + 1];
+        if (hi <= lo) continue;  // z = 0
+        const bool held = hi - lo <= kCsrHeld * W;  // uniform over the row's lanes
+        double r[kCsrHeld], mx = 0.0;
+        if (held) {
+#pragma unroll
+            for (int e = 0; e < kCsrHeld; e++) {
+                const int i = lo + e * W + sub;
+                r[e] = i < hi ? val[i] : 0.0;
+                mx = ref_max(mx, fabs(r[e]));
+            }
+        } else {
+            for (int i = lo + sub; i < hi; i += W) {
+                const double v = val[i];
+                rem[i] = v;
+                mx = ref_max(mx, fabs(v));
+            }
+        }
+        for (int o = W / 2; o > 0; o >>= 1) mx = ref_max(mx, __shfl_xor_sync(rows_lanes, mx, o));
+        int z = levels;
         const int rho = rho_rule(hi - lo, epsmode);
         for (int s = 0; s < levels; s++) {
             const double sigma = shift_sigma(0.75 * pow2(rho + tau_rule(mx)), shift);
             double nm = 0.0;
-            for (int i = lo + lane; i < hi; i += 32) {
-                double r = rem[i];
-                const double sl = (r + sigma) - sigma;
-                r = r - sl;
-                rem[i] = r;
-                nm = ref_max(nm, fabs(r));
-                if (WRITE) out[(size_t)s * ldo + i] = sl;
+            if (held) {
+#pragma unroll
+                for (int e = 0; e < kCsrHeld; e++) {
+                    const int i = lo + e * W + sub;
+                    if (i < hi) {
+                        const double sl = (r[e] + sigma) - sigma;
+                        r[e] = r[e] - sl;
+                        nm = ref_max(nm, fabs(r[e]));
+                        if (WRITE) out[(size_t)s * ldo + i] = sl;
+                    }
+                }
+            } else {
+                for (int i = lo + sub; i < hi; i += W) {
+                    double v = rem[i];
+                    const double sl = (v + sigma) - sigma;
+                    v = v - sl;
+                    rem[i] = v;
+                    nm = ref_max(nm, fabs(v));
+                    if (WRITE) out[(size_t)s * ldo + i] = sl;
+                }
             }
-            for (int o = 16; o > 0; o >>= 1) nm = ref_max(nm, __shfl_xor_sync(0xffffffffu, nm, o));
+            for (int o = W / 2; o > 0; o >>= 1) nm = ref_max(nm, __shfl_xor_sync(rows_lanes, nm, o));
             mx = nm;
             if (!WRITE && mx == 0.0) {
                 z = s;
                 break;
             }
         }
-    } else {
-        z = 0;
+        zbest = z > zbest ? z : zbest;
     }
-    if (!WRITE && lane == 0) atomicMax(zmax, z);
+    if (!WRITE) {
+        const int zw = __reduce_max_sync(0xffffffffu, zbest);
+        if (lane == 0) zsh[threadIdx.x >> 5] = zw;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int zb = 0;
+            for (int w = 0; w < 8; w++) zb = zsh[w] > zb ? zsh[w] : zb;
+            if (zb > 0) atomicMax(zmax, zb);
+        }
+    }
+}
+
+template <bool WRITE>
+static int split_csr_launch(cuozblasHandle_t *h, int m, int nnz, const double *val, const int *rowptr, int epsmode,
+                            int shift, int levels, double *rem, double *out, int64_t ldo, int *zmax) {
+    if (m <= 0) return CUOZBLAS_STATUS_SUCCESS;
+    cudaStream_t s = state(h)->stream;
+    const int64_t mean = ((int64_t)nnz + m - 1) / m;
+    auto go = [&](auto width) {
+        constexpr int W = decltype(width)::value;
+        const int64_t need = ((int64_t)m + 256 / W - 1) / (256 / W), cap = (int64_t)sm_count() * 8;
+        k_split_csr<WRITE, W><<<(int)(need < cap ? need : cap), 256, 0, s>>>(m, val, rowptr, epsmode, shift, levels,
+                                                                             rem, out, ldo, zmax);
+    };
+    counted(h);
+    if (mean <= 4)
+        go(std::integral_constant<int, 2>{});
+    else if (mean <= 8)
+        go(std::integral_constant<int, 4>{});
+    else if (mean <= 16)
+        go(std::integral_constant<int, 8>{});
+    else if (mean <= 32)
+        go(std::integral_constant<int, 16>{});
+    else
+        go(std::integral_constant<int, 32>{});
+    OZB_CHECK(cudaGetLastError());
+    return CUOZBLAS_STATUS_SUCCESS;
 }
 
 int split_csr_count(cuozblasHandle_t *h, int m, const double *val, const int *rowptr, int epsmode, int shift,
@@ -457,13 +531,7 @@ int split_csr_count(cuozblasHandle_t *h, int m, const double *val, const int *ro
     double *rem = ar.take<double>(nnz > 0 ? nnz : 1);
     if (!ar.ok) return CUOZBLAS_STATUS_WORKSPACE;
     OZB_CHECK(cudaMemsetAsync(st->d_ints, 0, sizeof(int), st->stream));
-    const int blocks = (int)(((int64_t)m * 32 + 255) / 256);
-    if (m > 0) {
-        counted(h);
-        k_split_csr<false><<<blocks, 256, 0, st->stream>>>(m, val, rowptr, epsmode, shift, maxS - 1, rem, nullptr, 0,
-                                                           st->d_ints);
-    }
-    OZB_CHECK(cudaGetLastError());
+    OZB_TRY(split_csr_launch<false>(h, m, nnz, val, rowptr, epsmode, shift, maxS - 1, rem, nullptr, 0, st->d_ints));
     OZB_CHECK(cudaMemcpyAsync(st->h_ints, st->d_ints, sizeof(int), cudaMemcpyDeviceToHost, st->stream));
     OZB_CHECK(cudaStreamSynchronize(st->stream));
     const int zmax = st->h_ints[0];
@@ -475,18 +543,11 @@ int split_csr_count(cuozblasHandle_t *h, int m, const double *val, const int *ro
 
 int split_csr_write(cuozblasHandle_t *h, int m, int nnz, const double *val, const int *rowptr, int epsmode,
                     int shift, int ns, double *out, int64_t ld) {
-    State *st = state(h);
     Arena ar(h);
     const uint64_t mk = ar.mark();
     double *rem = ar.take<double>(nnz > 0 ? nnz : 1);
     if (!ar.ok) return CUOZBLAS_STATUS_WORKSPACE;
-    const int blocks = (int)(((int64_t)m * 32 + 255) / 256);
-    if (m > 0) {
-        counted(h);
-        k_split_csr<true><<<blocks, 256, 0, st->stream>>>(m, val, rowptr, epsmode, shift, ns, rem, out, ld,
-                                                          nullptr);
-    }
-    OZB_CHECK(cudaGetLastError());
+    OZB_TRY(split_csr_launch<true>(h, m, nnz, val, rowptr, epsmode, shift, ns, rem, out, ld, nullptr));
     ar.release(mk);
     return CUOZBLAS_STATUS_SUCCESS;
 }
