@@ -237,19 +237,37 @@ __global__ void __launch_bounds__(256) k_cg_xr_rr(int n, double *__restrict__ x,
     xacc_init(acc);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t iw = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31);
-    const int64_t steps = iw < n ? ((int64_t)n - iw + stride - 1) / stride : 0;
+    // U elements per lane per step, their four loads each in flight together
+    constexpr int U = 2;
+    const int64_t steps = iw < n ? ((int64_t)n - iw + U * stride - 1) / (U * stride) : 0;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (int64_t s = 0; s < steps; s++, i += stride) {
-        double ri = 0.0;
-        if (i < n) {
-            x[i] = fma(al, p[i], x[i]);
-            ri = fma(-al, q[i], r[i]);
-            r[i] = ri;
-            scan_elem(ri, mx, lsb, bad);
+    for (int64_t s = 0; s < steps; s++, i += U * stride) {
+        double pv[U], xv[U], qv[U], rv[U];
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            const int64_t e = i + k * stride;
+            const bool in = e < n;
+            pv[k] = in ? p[e] : 0.0;
+            xv[k] = in ? x[e] : 0.0;
+            qv[k] = in ? q[e] : 0.0;
+            rv[k] = in ? r[e] : 0.0;
         }
-        xacc_fit(acc, __reduce_max_sync(0xffffffffu, abs_hiword(__dmul_rn(ri, ri))));
-        xacc_product(acc, ri, ri);
-        if ((s & 63) == 63) xacc_normalize(acc);
+        unsigned hi = 0u;
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            const int64_t e = i + k * stride;
+            if (e < n) {
+                x[e] = fma(al, pv[k], xv[k]);
+                rv[k] = fma(-al, qv[k], rv[k]);
+                r[e] = rv[k];
+                scan_elem(rv[k], mx, lsb, bad);
+            }
+            hi = max(hi, abs_hiword(__dmul_rn(rv[k], rv[k])));
+        }
+        xacc_fit(acc, __reduce_max_sync(0xffffffffu, hi));
+#pragma unroll
+        for (int k = 0; k < U; k++) xacc_product(acc, rv[k], rv[k]);
+        if ((s & 31) == 31) xacc_normalize(acc);  // every 64 products per lane
     }
     scan_commit(rs, 0, mx, lsb, bad, red);
     if (!xreduce_finish(acc, xr, &res_sh, &cert_sh)) return;

@@ -140,10 +140,32 @@ __device__ __forceinline__ void xacc_raise(XAcc &x) {
     xacc_sigmas(x);
 }
 
+// True while nothing but zeros has been deposited.
+__device__ __forceinline__ bool xacc_empty(const XAcc &x) {
+    bool zero = true;
+#pragma unroll
+    for (int j = 0; j < kXK; j++) zero = zero && x.a[j] == 0.0;
+    return zero;
+}
+
+// With empty bins: the top bin xacc_raise would reach for the high word `hi`
+// in one step (B with 2^(B W) <= |p| < 2^((B + 1) W)), not one raise after the
+// other up from kXBmin.
+__device__ __forceinline__ void xacc_start(XAcc &x, unsigned hi) {
+    const int top = ((int)(hi >> 20) - 1023 + 64 * kXW) / kXW - 64;  // floor(E / W): the argument is positive
+    x.B = top > kXBmax ? kXBmax : (top < kXBmin ? kXBmin : top);
+    xacc_sigmas(x);
+}
+
 // Before depositing products whose largest magnitude (over the warp) has the
 // high word `hi_max` (sign cleared): raise B until they lie below 2^((B+1)W).
 __device__ __forceinline__ void xacc_fit(XAcc &x, unsigned hi_max) {
-    while (x.B < kXBmax && hi_max >= (unsigned)((x.B + 1) * kXW + 1023) << 20) xacc_raise(x);
+    if (x.B < kXBmax && hi_max >= (unsigned)((x.B + 1) * kXW + 1023) << 20) {  // uniform
+        if (__all_sync(0xffffffffu, xacc_empty(x)))
+            xacc_start(x, hi_max);
+        else
+            while (x.B < kXBmax && hi_max >= (unsigned)((x.B + 1) * kXW + 1023) << 20) xacc_raise(x);
+    }
 }
 
 // Carry every bin's part above the next bin's grid into it (exact), then keep
@@ -169,7 +191,12 @@ __device__ __forceinline__ void xacc_normalize(XAcc &x) {
 // Per-lane forms, for lanes that accumulate different reductions (the rows of
 // a matrix): every lane keeps its own B, and the decisions diverge.
 __device__ __forceinline__ void xacc_fit1(XAcc &x, unsigned hi) {
-    while (x.B < kXBmax && hi >= (unsigned)((x.B + 1) * kXW + 1023) << 20) xacc_raise(x);
+    if (x.B < kXBmax && hi >= (unsigned)((x.B + 1) * kXW + 1023) << 20) {
+        if (xacc_empty(x))
+            xacc_start(x, hi);
+        else
+            while (x.B < kXBmax && hi >= (unsigned)((x.B + 1) * kXW + 1023) << 20) xacc_raise(x);
+    }
 }
 
 __device__ __forceinline__ void xacc_normalize1(XAcc &x) {
@@ -241,23 +268,32 @@ __device__ inline bool xparts_round1(int np, Get part, double &out) {
 }
 
 
-// Warp sum of the lanes' bins (same B), then block sum into `out` (thread 0;
-// `wsh` holds one XPart per warp).  Exact: every lane is normalised first, a
-// warp's bins stay below 2^(W+4) g and a block of at most 8 warps below
-// 2^(W+7) g.
+// Move a set's bins `d` bins down, what leaves the window into the bound.
+__device__ __forceinline__ void xbins_lower(double (&a)[kXK], double &drop, int d) {
+    for (int u = 0; u < d && u < kXK; u++) {
+        drop = __dadd_ru(drop, fabs(a[kXK - 1]));
+#pragma unroll
+        for (int j = kXK - 1; j >= 1; j--) a[j] = a[j - 1];
+        a[0] = 0.0;
+    }
+}
+
+// Warp sum of the lanes' bins (same B), then block sum into `out` (`wsh`
+// holds one XPart per warp; at most 8 warps, one lane of warp 0 each).  Exact:
+// every lane is normalised first, a warp's bins stay below 2^(W+4) g and a
+// block of at most 8 warps below 2^(W+7) g.
 __device__ __forceinline__ void xacc_block_reduce(XAcc &x, XPart *wsh, XPart &out) {
     xacc_normalize(x);
-#pragma unroll
-    for (int j = 0; j < kXK; j++)
-        for (int o = 16; o > 0; o >>= 1) x.a[j] = __dadd_rn(x.a[j], __shfl_xor_sync(0xffffffffu, x.a[j], o));
     for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int j = 0; j < kXK; j++) x.a[j] = __dadd_rn(x.a[j], __shfl_xor_sync(0xffffffffu, x.a[j], o));
         x.drop = __dadd_ru(x.drop, __shfl_xor_sync(0xffffffffu, x.drop, o));
         x.es = __dadd_rn(x.es, __shfl_xor_sync(0xffffffffu, x.es, o));
         x.ea = __dadd_ru(x.ea, __shfl_xor_sync(0xffffffffu, x.ea, o));
     }
     const int fl = (int)__reduce_or_sync(0xffffffffu, (unsigned)x.flags);
-    const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if ((threadIdx.x & 31) == 0) {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    if (lane == 0) {
         wsh[w].B = (double)x.B;
 #pragma unroll
         for (int j = 0; j < kXK; j++) wsh[w].a[j] = x.a[j];
@@ -267,57 +303,88 @@ __device__ __forceinline__ void xacc_block_reduce(XAcc &x, XPart *wsh, XPart &ou
         wsh[w].flags = (double)fl;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int Bb = kXBmin;
-        for (int i = 0; i < nw; i++) Bb = max(Bb, (int)wsh[i].B);
-        XPart r;
-        r.B = (double)Bb;
-        for (int j = 0; j < kXK; j++) r.a[j] = 0.0;
-        r.drop = r.es = r.ea = 0.0;
-        int f = 0;
-        for (int i = 0; i < nw; i++) {  // <= 8 warps of bins below 2^(W+4) g: exact
-            const int d = Bb - (int)wsh[i].B;
-            for (int j = 0; j < kXK; j++) {
-                if (j + d < kXK)
-                    r.a[j + d] = __dadd_rn(r.a[j + d], wsh[i].a[j]);
-                else
-                    r.drop = __dadd_ru(r.drop, fabs(wsh[i].a[j]));
-            }
-            r.drop = __dadd_ru(r.drop, wsh[i].drop);
-            r.es = __dadd_rn(r.es, wsh[i].es);
-            r.ea = __dadd_ru(r.ea, wsh[i].ea);
-            f |= (int)wsh[i].flags;
+    if (w == 0) {
+        const bool in = lane < nw;
+        const XPart &q = wsh[in ? lane : 0];
+        const int B = in ? (int)q.B : kXBmin;
+        double a[kXK], drop = in ? q.drop : 0.0, es = in ? q.es : 0.0, ea = in ? q.ea : 0.0;
+#pragma unroll
+        for (int j = 0; j < kXK; j++) a[j] = in ? q.a[j] : 0.0;
+        const unsigned f = __reduce_or_sync(0xffffffffu, in ? (unsigned)(int)q.flags : 0u);
+        const int Bb = __reduce_max_sync(0xffffffffu, B);
+        xbins_lower(a, drop, Bb - B);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {  // <= 8 warps of bins below 2^(W+4) g: exact
+#pragma unroll
+            for (int j = 0; j < kXK; j++) a[j] = __dadd_rn(a[j], __shfl_xor_sync(0xffffffffu, a[j], o));
+            drop = __dadd_ru(drop, __shfl_xor_sync(0xffffffffu, drop, o));
+            es = __dadd_rn(es, __shfl_xor_sync(0xffffffffu, es, o));
+            ea = __dadd_ru(ea, __shfl_xor_sync(0xffffffffu, ea, o));
         }
-        r.flags = (double)f;
-        out = r;
+        if (lane == 0) {
+            out.B = (double)Bb;
+#pragma unroll
+            for (int j = 0; j < kXK; j++) out.a[j] = a[j];
+            out.drop = drop;
+            out.es = es;
+            out.ea = ea;
+            out.flags = (double)f;
+        }
     }
 }
+
+// NearSum where CrSum cannot certify: rare, kept out of the callers' code.
+__device__ __noinline__ inline double xnearsum_cold(int n, double *v) { return nearsum(n, v, 1); }
 
 // Exact sum of `np` block parts into a correctly rounded double (one block
 // of 256 threads; the caller synchronises before and reads *result after).
 // Parts are shifted onto the largest top bin with two spare bins above it;
 // *certified = 0 when the drop bound leaves the rounding open or a flag is
 // set.  `sh` is shared scratch of at least 256 * (kXK2 + 3) doubles.
+//
+// This tail is a chain of latencies that every exact reduction pays whatever
+// its length, so no step of it is left to one thread: a part's values are
+// loaded together, one lane per slot adds the warps, and the two roundings
+// (minus and plus the bound) run side by side in two lanes.
 constexpr int kXK2 = kXK + 2;
 __device__ inline void xparts_round(const XPart *parts, int np, double *sh, double *result, int *certified) {
     __shared__ int s_B, s_flags;
-    const int t = threadIdx.x;
+    const int t = threadIdx.x, nw = blockDim.x >> 5;
     if (t == 0) {
         s_B = kXBmin;
         s_flags = 0;
     }
     __syncthreads();
+    auto load = [&](int i, double (&a)[kXK], double &drop, double &es, double &ea) {
+        const bool in = i < np;
+        const XPart *q = parts + (in ? i : 0);
+#pragma unroll
+        for (int j = 0; j < kXK; j++) a[j] = __ldcg(&q->a[j]);
+        drop = __ldcg(&q->drop);
+        es = __ldcg(&q->es);
+        ea = __ldcg(&q->ea);
+        if (!in) {
+#pragma unroll
+            for (int j = 0; j < kXK; j++) a[j] = 0.0;
+            drop = es = ea = 0.0;
+        }
+    };
+    double a[kXK], pd, pes, pea;  // the part being added: the first one loads beside the bins' tops
+    load(t, a, pd, pes, pea);
+    int pB = kXBmin;
     {  // the largest top bin and the flags, every thread over its parts
         int Bg = kXBmin, f = 0;
         for (int i = t; i < np; i += blockDim.x) {
-            Bg = max(Bg, (int)__ldcg(&parts[i].B));
+            const int b = (int)__ldcg(&parts[i].B);
             f |= (int)__ldcg(&parts[i].flags);
+            if (i == t) pB = b;
+            Bg = max(Bg, b);
         }
         Bg = __reduce_max_sync(0xffffffffu, Bg);
         f = (int)__reduce_or_sync(0xffffffffu, (unsigned)f);
         if ((t & 31) == 0) {
             atomicMax(&s_B, Bg);
-            atomicOr(&s_flags, f);
+            if (f) atomicOr(&s_flags, f);
         }
     }
     __syncthreads();
@@ -329,18 +396,16 @@ __device__ inline void xparts_round(const XPart *parts, int np, double *sh, doub
         sig[j] = 1.5 * pow2((Bt - j) * kXW + 52);
     }
     for (int i = t; i < np; i += blockDim.x) {
-        const int d = s_B - (int)__ldcg(&parts[i].B);
-        for (int j = 0; j < kXK; j++) {
-            const double v = __ldcg(&parts[i].a[j]);
-            const int k = j + d + 2;
-            if (k < kXK2)
-                c[k] = __dadd_rn(c[k], v);
-            else
-                drop = __dadd_ru(drop, fabs(v));
+        if (i != t) {
+            load(i, a, pd, pes, pea);
+            pB = (int)__ldcg(&parts[i].B);
         }
-        drop = __dadd_ru(drop, __ldcg(&parts[i].drop));
-        es = __dadd_rn(es, __ldcg(&parts[i].es));
-        ea = __dadd_ru(ea, __ldcg(&parts[i].ea));
+        xbins_lower(a, pd, s_B - pB);  // leaving the part's window is leaving the layout's
+#pragma unroll
+        for (int j = 0; j < kXK; j++) c[j + 2] = __dadd_rn(c[j + 2], a[j]);
+        drop = __dadd_ru(drop, pd);
+        es = __dadd_rn(es, pes);
+        ea = __dadd_ru(ea, pea);
         // a part's bins are below 2^(W+7) g (8 warps of normalised lanes) and c's
         // below 2^(W-1) g after this carry: the next part adds exactly
 #pragma unroll
@@ -361,7 +426,6 @@ __device__ inline void xparts_round(const XPart *parts, int np, double *sh, doub
         drop = __dadd_ru(drop, __shfl_xor_sync(0xffffffffu, drop, o));
         ea = __dadd_ru(ea, __shfl_xor_sync(0xffffffffu, ea, o));
     }
-    const int nw = blockDim.x >> 5;
     if ((t & 31) == 0) {
         const int w = t >> 5;
 #pragma unroll
@@ -371,35 +435,39 @@ __device__ inline void xparts_round(const XPart *parts, int np, double *sh, doub
         sh[(kXK2 + 2) * nw + w] = ea;
     }
     __syncthreads();
-    if (t == 0) {
-        for (int j = 0; j < kXK2 + 3; j++) {
-            double v = sh[j * nw];
-            for (int w = 1; w < nw; w++)
-                v = j == kXK2 + 1 || j == kXK2 + 2 ? __dadd_ru(v, sh[j * nw + w]) : __dadd_rn(v, sh[j * nw + w]);
-            sh[j * nw] = v;
+    if (t >= 32) return;
+    double slot = 0.0;  // lane j: slot j over the warps (the bounds rounded up)
+    if (t < kXK2 + 3) {
+        for (int w = 0; w < nw; w++) {
+            const double v = sh[t * nw + w];
+            slot = t > kXK2 ? __dadd_ru(slot, v) : __dadd_rn(slot, v);
         }
     }
-    if (t == 0) {
-        double terms[kXK2 + 2];
-        for (int j = 0; j <= kXK2; j++) terms[j] = sh[j * nw];
-        const double D = __dadd_ru(sh[(kXK2 + 1) * nw], xes_bound(sh[(kXK2 + 2) * nw]));
-        int ok = s_flags == 0;
-        double r = 0.0;
-        if (ok) {
-            if (D == 0.0) {
-                r = nearsum(kXK2 + 1, terms, 1);
-            } else {
-                double lo[kXK2 + 2], hi[kXK2 + 2];
-                for (int j = 0; j <= kXK2; j++) lo[j] = hi[j] = terms[j];
-                lo[kXK2 + 1] = -D;
-                hi[kXK2 + 1] = D;
-                const double rl = nearsum(kXK2 + 2, lo, 1), rh = nearsum(kXK2 + 2, hi, 1);
-                ok = (dbits(rl) == dbits(rh));
-                r = rl;
-            }
+    const double D = __dadd_ru(__shfl_sync(0xffffffffu, slot, kXK2 + 1),
+                               xes_bound(__shfl_sync(0xffffffffu, slot, kXK2 + 2)));
+    // lane 0 rounds the held sum minus the bound, lane 1 plus the bound
+    double terms[kXK2 + 2];
+#pragma unroll
+    for (int j = 0; j <= kXK2; j++) terms[j] = __shfl_sync(0xffffffffu, slot, j);
+    terms[kXK2 + 1] = t == 0 ? -D : D;
+    const int flagged = s_flags;
+    double r = 0.0;
+    if (t < 2 && !flagged) {
+        CrSum cs;
+#pragma unroll
+        for (int j = 0; j < kXK2 + 2; j++) cs.add(terms[j]);
+        if (!cs.finish(r)) {
+            double *tm = sh + (kXK2 + 3) * nw + t * (kXK2 + 2);
+#pragma unroll
+            for (int j = 0; j < kXK2 + 2; j++) tm[j] = terms[j];
+            r = xnearsum_cold(D == 0.0 ? kXK2 + 1 : kXK2 + 2, tm);
         }
+    }
+    __syncwarp();
+    const double rh = __shfl_sync(0xffffffffu, r, 1);
+    if (t == 0) {
         *result = r;
-        *certified = ok;
+        *certified = !flagged && dbits(r) == dbits(rh);
     }
 }
 

@@ -29,3 +29,26 @@ def test_row_split_widths(n, lo, hi, oracle, handle, ozb, cuda):
     ozb.dcsrmv(handle, "n", n, n, len(val), 0.5, dev(val), dev(colind), dev(rowptr), dev(x), -2.0, dy)
     assert bits_equal(dy.cpu().numpy(), ref), first_diff(dy.cpu().numpy(), ref)
     assert (handle.nSplitA, handle.nSplitB) == (info.nSplitA, info.nSplitB)
+
+
+@pytest.mark.parametrize("n,kind", [(1, ""), (33, ""), (1024, ""), (1025, "rising"), (40001, "rising"),
+                                    (40001, "blocks"), (5000, "cancel"), (3000, "zeros"), (70000, "high"),
+                                    (70000, "low")])
+def test_exact_reduction_bins(n, kind, oracle, handle, ozb, cuda):
+    x, y = oracle.phi_vector(n, 1.0, 1), oracle.phi_vector(n, 1.0, 2)
+    if kind == "rising":
+        x *= 2.0 ** np.linspace(-30, 30, n).astype(int)
+    if kind == "blocks":
+        x *= np.where((np.arange(n) // 1024) % 3 == 0, 2.0 ** 50, 2.0 ** -20)
+    if kind == "cancel":
+        x[n // 2:], y[n // 2:] = x[:n - n // 2], -y[:n - n // 2]
+    if kind == "zeros":
+        x[::2] = 0.0
+    if kind in ("high", "low"):
+        x *= 2.0 ** (400 if kind == "high" else -400)
+    handle.sumMode = 1
+    dx, dy = cuda.from_numpy(x).cuda(), cuda.from_numpy(y).cuda()
+    d = ozb.ddot(handle, n, dx, dy)
+    r, info = oracle.ddot(make_flags(sumMode=1), x, y)
+    assert np.float64(d).view(np.int64) == np.float64(r).view(np.int64), (d, r)
+    assert (handle.nSplitA, handle.nSplitB) == (info.nSplitA, info.nSplitB)
