@@ -351,15 +351,19 @@ int cg_graph(cuozblasHandle_t *h, int n, const double *val, const int *colind, c
             return CUOZBLAS_STATUS_CUDA_ERROR;              \
         }                                                   \
     } while (0)
-    // rows the row kernel defers: a property of A, listed once
-    int nslow = 0;
+    // rows the row kernel defers, and whether all others meet the conditions of
+    // the correctly rounded rows: properties of A, found once
+    int nslow = 0, nunfit = 0;
+    int *unfit = &cs->rn_declined;  // (cs is zeroed before the iterations)
     CG_CHECK(cudaMemsetAsync(slow + nn, 0, sizeof(int), s));
-    if ((status = csr_slow_rows_launch(s, n, val, rowptr, shift, h->splitEpsMode, maxS, na_hint, slow,
-                                       reinterpret_cast<int *>(slow + nn)))) {
+    CG_CHECK(cudaMemsetAsync(unfit, 0, sizeof(int), s));
+    if ((status = csr_slow_rows_launch(s, n, n, val, rowptr, shift, h->splitEpsMode, maxS, na_hint, slow,
+                                       reinterpret_cast<int *>(slow + nn), unfit))) {
         cleanup();
         return status;
     }
     CG_CHECK(cudaMemcpyAsync(&nslow, slow + nn, sizeof(int), cudaMemcpyDeviceToHost, s));
+    CG_CHECK(cudaMemcpyAsync(&nunfit, unfit, sizeof(int), cudaMemcpyDeviceToHost, s));
     CG_CHECK(cudaStreamSynchronize(s));
     double *terms = nullptr;
     if (nslow > 0) {
@@ -417,7 +421,8 @@ int cg_graph(cuozblasHandle_t *h, int n, const double *val, const int *colind, c
     for (int k = 0; k < K && !cap; k++) {
         if (!no_proof) cap = csr_proof_launch(s, n, p, rho, maxS, cs, &d->gate);
         if (!cap)
-            cap = rn_rows ? csr_rn_launch(s, spmv, cs, slow, nslow, &dpq->vs, 1, terms, &d->gate,
+            cap = no_proof && nunfit == 0 ? csr_rn_ready_launch(s, spmv, cs, &dpq->vs, 1, &d->gate, &dpq->vs)
+                  : rn_rows ? csr_rn_launch(s, spmv, cs, slow, nslow, &dpq->vs, 1, terms, &d->gate,
                                           no_proof ? &dpq->vs : nullptr)
                           : csr_rows_launch(s, spmv, cs, slow, nslow, &dpq->vs, 1, terms, &d->gate);
         if (fused_dots) {

@@ -254,12 +254,21 @@ __device__ __forceinline__ bool row_chain(const double (&a)[kCsrRowMax], int len
     return !(mx != 0.0 && na < maxS);
 }
 
+__host__ __device__ __forceinline__ int ceil_log2_small(int v) {
+    int c = 0;
+    while ((1 << c) < v) c++;
+    return c;
+}
+
 // The rows the row kernel defers (more than kCsrRowMax entries, or more than
-// NA levels), listed once for a matrix that is multiplied many times.
+// NA levels), listed once for a matrix that is multiplied many times.  With
+// `unfit`: also whether some other row fails k_csrmv_rn's conditions on A and
+// the row length (lg_shift: the log2 of the shift).
 template <int NA>
 __global__ void __launch_bounds__(128) k_csr_slow_rows(int m, const double *__restrict__ val,
                                                        const int *__restrict__ rowptr, int shift, int epsmode,
-                                                       int maxS, int *__restrict__ list, int *__restrict__ count) {
+                                                       int maxS, int *__restrict__ list, int *__restrict__ count,
+                                                       int *__restrict__ unfit, int rho_x, int lg_shift) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= m) return;
     const int lo = rowptr[row], len = rowptr[row + 1] - lo;
@@ -271,19 +280,25 @@ __global__ void __launch_bounds__(128) k_csr_slow_rows(int m, const double *__re
         double sigA[NA];
         int na, z;
         defer = !row_chain<NA>(a, len, shift, epsmode, maxS, sigA, na, z);
+        if (!defer && unfit && len > 0 &&
+            (z >= maxS || ceil_log2_small(len) + 106 - rho_rule(len, epsmode) - rho_x + lg_shift > 53))
+            *unfit = 1;
     }
     if (defer) list[atomicAdd(count, 1)] = row;
 }
 
-int csr_slow_rows_launch(cudaStream_t s, int m, const double *val, const int *rowptr, int shift, int epsmode,
-                         int maxS, int na_hint, int *list, int *count) {
+int csr_slow_rows_launch(cudaStream_t s, int m, int n, const double *val, const int *rowptr, int shift, int epsmode,
+                         int maxS, int na_hint, int *list, int *count, int *unfit) {
     if (m <= 0) return CUOZBLAS_STATUS_SUCCESS;
+    const int rho_x = rho_rule(n > 0 ? n : 1, epsmode);
+    const int lg_shift = shift > 0 ? 31 - __builtin_clz((unsigned)shift) : 0;
+    const int grid = (m + 127) / 128;
     if (na_hint > 0 && na_hint <= 2)
-        k_csr_slow_rows<2><<<(m + 127) / 128, 128, 0, s>>>(m, val, rowptr, shift, epsmode, maxS, list, count);
+        k_csr_slow_rows<2><<<grid, 128, 0, s>>>(m, val, rowptr, shift, epsmode, maxS, list, count, unfit, rho_x, lg_shift);
     else if (na_hint > 4)
-        k_csr_slow_rows<6><<<(m + 127) / 128, 128, 0, s>>>(m, val, rowptr, shift, epsmode, maxS, list, count);
+        k_csr_slow_rows<6><<<grid, 128, 0, s>>>(m, val, rowptr, shift, epsmode, maxS, list, count, unfit, rho_x, lg_shift);
     else
-        k_csr_slow_rows<4><<<(m + 127) / 128, 128, 0, s>>>(m, val, rowptr, shift, epsmode, maxS, list, count);
+        k_csr_slow_rows<4><<<grid, 128, 0, s>>>(m, val, rowptr, shift, epsmode, maxS, list, count, unfit, rho_x, lg_shift);
     return cudaGetLastError() == cudaSuccess ? CUOZBLAS_STATUS_SUCCESS : CUOZBLAS_STATUS_CUDA_ERROR;
 }
 
@@ -890,12 +905,6 @@ __device__ __forceinline__ bool rn_row_dot(const double (&v)[kCsrRowMax], const 
     return true;
 }
 
-__host__ __device__ __forceinline__ int ceil_log2_small(int v) {
-    int c = 0;
-    while ((1 << c) < v) c++;
-    return c;
-}
-
 template <int NA>
 __global__ void __launch_bounds__(kCsrThreads, 4)
     k_csrmv_rn(int m, int n, const double *__restrict__ val, const int *__restrict__ colind,
@@ -1050,6 +1059,103 @@ __global__ void __launch_bounds__(kCsrThreads, 4)
     if (ystats) scan_commit(ystats, ystats_index, smx, slsb, sbad, red);
 }
 
+// The same product when every row of A is known to meet the conditions (a
+// solver checks its matrix once, k_csr_slow_rows with `unfit`): no row is
+// split again, so the entries need not wait in one thread's hands.  A tile is
+// 256 rows, at most 2048 entries: the block takes the entries flat and
+// coalesced (values, columns, then the gathers of x, eight of each in flight
+// per thread), leaves each one's TwoProd in shared memory, and then one thread
+// adds each row.  What is left of the bound is half memory (84 MB for 10^6
+// rows of 7: 13 us), half the rows' TwoSum cascades.  10^6 rows: 36 us; the
+// kernel above, which also splits each row, 53.
+constexpr int kReadyRows = 256;
+
+// A row CrSum cannot certify, with rn_row_dot's terms and padding.
+__device__ __noinline__ double csr_nearsum_cold(const double2 *q, int len) {
+    double t[2 * kCsrRowMax];
+    for (int e = 0; e < kCsrRowMax; e++) {
+        t[2 * e] = e < len ? q[e].x : 0.0;
+        t[2 * e + 1] = e < len ? q[e].y : 0.0;
+    }
+    return nearsum(2 * kCsrRowMax, t, 1);
+}
+
+__global__ void __launch_bounds__(kReadyRows, 4)
+    k_csrmv_rn_ready(int m, const double *__restrict__ val, const int *__restrict__ colind,
+                     const int *__restrict__ rowptr, const double *__restrict__ x, int rho_x, int maxS, double alpha,
+                     double beta, double *__restrict__ y, CsrScratch *__restrict__ sc, VecStats *__restrict__ ystats,
+                     int ystats_index, const VecStats *__restrict__ xstats, const int *__restrict__ gate) {
+    if (gate && *gate == 0) return;  // uniform: a captured solver step that is switched off
+    __shared__ double2 te[kReadyRows * kCsrRowMax];
+    __shared__ double red[kReadyRows / 32];
+    __shared__ int xok, bad;
+    const int t = threadIdx.x;
+    if (t == 0) {  // x's split must be complete
+        VecStats vs;
+        vs.mx[0] = __ldcg(&xstats->mx[0]);
+        vs.lsb[0] = __ldcg(&xstats->lsb[0]);
+        vs.bad[0] = __ldcg(&xstats->bad[0]);
+        xok = split_complete(vs, 0, rho_x, maxS) ? 1 : 0;
+        bad = 0;
+    }
+    __syncthreads();
+    if (!xok) {  // uniform: the caller computes the slices instead
+        if (blockIdx.x == 0 && t == 0) sc->rn_declined = 1;
+        return;
+    }
+    double smx = 0.0;
+    int slsb = 0, sbad = 0;
+    bool wide = false;  // a product outside the range TwoProd keeps exact
+    const int ntiles = (m + kReadyRows - 1) / kReadyRows;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int r0 = tile * kReadyRows, row = r0 + t;
+        const int rend = m - r0 < kReadyRows ? m : r0 + kReadyRows;
+        const int base = rowptr[r0], end = rowptr[rend];
+        const bool active = row < m;
+        const int lo = active ? rowptr[row] - base : 0, len = active ? rowptr[row + 1] - base - lo : 0;
+        const double yold = active ? y[row] : 0.0;
+        double v[kCsrRowMax], xv[kCsrRowMax];
+        int c[kCsrRowMax];
+#pragma unroll
+        for (int k = 0; k < kCsrRowMax; k++) {
+            const int i = base + k * kReadyRows + t;
+            c[k] = i < end ? colind[i] : -1;
+            v[k] = i < end ? val[i] : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < kCsrRowMax; k++) xv[k] = c[k] >= 0 ? x[c[k]] : 0.0;
+#pragma unroll
+        for (int k = 0; k < kCsrRowMax; k++) {
+            const double p = __dmul_rn(v[k], xv[k]);
+            const double er = __fma_rn(v[k], xv[k], -p);
+            const double ap = fabs(p);
+            if ((ap < 0x1p-969 && v[k] != 0.0 && xv[k] != 0.0) || !(ap < 0x1p1023)) wide = true;
+            te[k * kReadyRows + t] = make_double2(p, er);
+        }
+        __syncthreads();
+        if (active) {
+            CrSum cs;
+#pragma unroll
+            for (int e = 0; e < kCsrRowMax; e++)
+                if (e < len) {
+                    const double2 q = te[lo + e];
+                    cs.add(q.x);
+                    cs.add(q.y);
+                }
+            double tsum;
+            if (!cs.finish(tsum)) tsum = csr_nearsum_cold(te + lo, len);
+            const double ynew = fma(alpha, tsum, beta * yold);
+            y[row] = ynew;
+            if (ystats) scan_elem(ynew, smx, slsb, sbad);
+        }
+        __syncthreads();
+    }
+    if (wide) bad = 1;
+    __syncthreads();
+    if (t == 0 && bad) sc->rn_declined = 1;  // the whole product: the host path takes this iteration
+    if (ystats) scan_commit(ystats, ystats_index, smx, slsb, sbad, red);
+}
+
 bool csr_rn_applies(const CsrmvArgs &a) {
     return a.sum_mode == 1 && a.epsmode == 0 && a.shift > 0 && (a.shift & (a.shift - 1)) == 0;
 }
@@ -1073,6 +1179,18 @@ static void launch_rn(const CsrmvArgs &a, cudaStream_t s, CsrScratch *sc, int *s
     k_csrmv_rn<NA><<<grid, kCsrThreads, 0, s>>>(a.m, a.n, a.val, a.colind, a.rowptr, a.x, a.shift, lg_shift, rho_x,
                                                  a.epsmode, a.maxS, a.alpha, a.beta, a.y, sc, slow, append, ystats,
                                                  ystats_index, xstats, gate);
+}
+
+// Every row of A meets k_csrmv_rn's conditions (k_csr_slow_rows found no
+// listed and no unfit row); `xstats` are x's statistics.
+int csr_rn_ready_launch(cudaStream_t s, const CsrmvArgs &a, CsrScratch *sc, VecStats *ystats, int ystats_index,
+                        const int *gate, const VecStats *xstats) {
+    if (a.m <= 0) return CUOZBLAS_STATUS_SUCCESS;
+    const int tiles = (a.m + kReadyRows - 1) / kReadyRows, cap = sm_count() * 4;
+    k_csrmv_rn_ready<<<tiles < cap ? tiles : cap, kReadyRows, 0, s>>>(
+        a.m, a.val, a.colind, a.rowptr, a.x, rho_rule(a.n > 0 ? a.n : 1, a.epsmode), a.maxS, a.alpha, a.beta, a.y, sc,
+        ystats, ystats_index, xstats, gate);
+    return cudaGetLastError() == cudaSuccess ? CUOZBLAS_STATUS_SUCCESS : CUOZBLAS_STATUS_CUDA_ERROR;
 }
 
 int csr_rn_launch(cudaStream_t s, const CsrmvArgs &a, CsrScratch *sc, int *slow, int fixed_slow, VecStats *ystats,

@@ -74,8 +74,10 @@ struct CsrmvArgs {
     int shift, epsmode, maxS, sum_mode, na_hint;
 };
 int vec_stats_launch(cudaStream_t s, int nsm, int n, const double *x, VecStats *vs, int index);
-int csr_slow_rows_launch(cudaStream_t s, int m, const double *val, const int *rowptr, int shift, int epsmode,
-                         int maxS, int na_hint, int *list, int *count);
+int csr_slow_rows_launch(cudaStream_t s, int m, int n, const double *val, const int *rowptr, int shift, int epsmode,
+                         int maxS, int na_hint, int *list, int *count, int *unfit);
+int csr_rn_ready_launch(cudaStream_t s, const CsrmvArgs &a, CsrScratch *sc, VecStats *ystats, int ystats_index,
+                        const int *gate, const VecStats *xstats);
 int csr_proof_launch(cudaStream_t s, int n, const double *x, int rho, int maxS, CsrScratch *sc, const int *gate);
 int csr_rows_launch(cudaStream_t s, const CsrmvArgs &a, CsrScratch *sc, int *slow, int fixed_slow,
                     VecStats *ystats, int ystats_index, double *terms, const int *gate);

@@ -10,6 +10,47 @@ from tests.conftest import bits_equal, first_diff
 pytestmark = pytest.mark.gpu
 
 
+def _sym(n, deg, seed):
+    """A symmetric, diagonally dominant matrix with at most `deg` entries in a row, as (rowptr, colind, val)."""
+    rng = np.random.default_rng(seed)
+    rows = [{i: 0.0} for i in range(n)]
+    for _ in range(4 * n):
+        i, j = (int(v) for v in rng.integers(0, n, 2))
+        if i != j and len(rows[i]) < deg and len(rows[j]) < deg:
+            rows[i][j] = rows[j][i] = float(rng.random() - 0.5)
+    for i in range(n):
+        rows[i][i] = 1.0 + sum(abs(v) for v in rows[i].values()) + float(rng.random())
+    rowptr = np.cumsum([0] + [len(r) for r in rows]).astype(np.int32)
+    colind = np.concatenate([sorted(r) for r in rows]).astype(np.int32)
+    val = np.concatenate([[r[c] for c in sorted(r)] for r in rows])
+    return rowptr, colind, val
+
+
+@pytest.mark.parametrize("n,deg,kind", [(1, 1, ""), (255, 7, ""), (256, 8, ""), (257, 8, ""), (1500, 5, ""),
+                                        (700, 12, ""), (600, 6, "deep"), (600, 6, "integers"), (300, 6, "huge")])
+def test_cg_rows(n, deg, kind, oracle, handle, ozb, cuda):
+    rowptr, colind, val = _sym(n, deg, n + deg)
+    b = oracle.normal(n, 4)
+    if kind == "deep":  # one row needs more levels than the others
+        val[rowptr[n // 2]] *= 2.0 ** -70
+    if kind == "integers":  # row sums that cancel to zero, midpoints
+        val, b = np.rint(val * 4), np.rint(b * 2)
+    if kind == "huge":  # products near the top of the range
+        val, b = val * 2.0 ** 500, b * 2.0 ** 400
+    iters = 5
+    xr, hr, _ = oracle.dcg(make_flags(sumMode=1), val, colind, rowptr, b, np.zeros(n), iters, 0.0)
+    handle.sumMode, handle.verbose = 1, 1
+
+    def dev(a):
+        return cuda.from_numpy(np.ascontiguousarray(a)).cuda()
+
+    dx = cuda.zeros(n, dtype=cuda.float64, device="cuda")
+    h1, h2 = np.zeros(iters + 1), np.zeros(iters + 1)
+    ozb.dcg(handle, "n", n, len(val), dev(val), dev(colind), dev(rowptr), dev(b), dx, iters, 0.0, h1, h2)
+    assert bits_equal(h1, hr), first_diff(h1, hr)
+    assert bits_equal(dx.cpu().numpy(), xr), first_diff(dx.cpu().numpy(), xr)
+
+
 @pytest.mark.parametrize("n,lo,hi", [(1, 1, 1), (3000, 0, 2), (700, 1, 7), (500, 0, 40), (300, 20, 40), (200, 30, 199)])
 def test_row_split_widths(n, lo, hi, oracle, handle, ozb, cuda):
     """x off the predicted chain: the rows' slices come from the row split, at each number of lanes per row."""
