@@ -71,12 +71,12 @@ __device__ __forceinline__ void di_transpose4(uint32_t w0, uint32_t w1, uint32_t
     }
 }
 
-// Cut E consecutive elements into all kDotLevels levels (levels past the
-// plan only fill rows that are never read) and write their digit rows (row
+// Cut E consecutive elements into the plan's L levels (four at least; rows
+// past the plan are never read) and write their digit rows (row
 // s D + j below `rows`, K bytes E u .. E u + E - 1; `rows` is the chunk's first
 // row plus this thread's byte offset, `ub16` its 16-byte chunk index times 16,
-// before the swizzle).  sk[s] = sigma_s + K g_s with K = 0x80808080: t = base
-// + sk[s] is rounded on the same grid, and its low word is (RN_{g_s}(base) /
+// before the swizzle).  sk_s = sigma_s + K g_s with K = 0x80808080: t = base
+// + sk_s is rounded on the same grid, and its low word is (RN_{g_s}(base) /
 // g_s + K) mod 2^32, so w = lo(t_s) - lo(t_{s-1}) * 2^d + K * 2^d is a_s + K
 // (at a group start lo(t_{s-1}) is taken as K); the bytes of w are the
 // balanced digits of a_s plus 0x80 each, removed after the byte transpose.
@@ -84,11 +84,12 @@ __device__ __forceinline__ void di_transpose4(uint32_t w0, uint32_t w1, uint32_t
 // for their proof (`pending`) are voted on with |a_s|.  No branch depends on
 // data or on the plan inside the level loop.
 template <int D, int E, int G, bool VOTE>
-__device__ __forceinline__ void di_digits(const double (&v)[E], const double *sk, int d, const int *ith,
+__device__ __forceinline__ void di_digits(const double (&v)[E], double sk0, int d, int L, const int *ith,
                                           uint32_t rows, unsigned pending, unsigned &prov) {
     static_assert(E == 4 || E == 8, "4 or 8 elements per thread");
     constexpr uint32_t K = 0x80808080u;
     const uint32_t kd = K << d;
+    const int skhi = __double2hiint(sk0), sklo = __double2loint(sk0);
     // the 128-byte swizzle XORs bits 4-6 of the address with the row's low 3
     // bits; `rows` has its own 16-byte chunk index there and row multiples of
     // 1024 above, so row r's address is (rows ^ ((r & 7) << 4)) + r * 128
@@ -101,9 +102,10 @@ __device__ __forceinline__ void di_digits(const double (&v)[E], const double *sk
     for (int e = 0; e < E; e++) base[e] = v[e];
 #pragma unroll
     for (int s = 0; s < kDotLevels; s++) {
-        const double sg = sk[s];
+        if (s >= 4 && s >= L) break;  // uniform: the plan has no such level
+        const double sg = __hiloint2double(skhi - s * (d << 20), sklo);
         if (s > 0 && s % G == 0) {  // compile-time: the next group cuts the remainder
-            const double sp = sk[s - 1];
+            const double sp = __hiloint2double(skhi - (s - 1) * (d << 20), sklo);
 #pragma unroll
             for (int e = 0; e < E; e++) base[e] = base[e] - (tprev[e] - sp);
         }
@@ -163,24 +165,34 @@ __device__ __forceinline__ void di_load(const double *__restrict__ v, int64_t i0
     }
 }
 
-// The pairs from the digit sums, the scale check, then FSum / NearSum (one
-// thread of the last CTA).
+// The pairs from the digit sums (a thread each: in one thread they were a
+// chain of 256 L2 loads, 20 us behind a pass of 125), the scale check, then
+// FSum / NearSum by one thread.  The last CTA, all threads.
 __device__ void di_finish(DotScratch *sc, const TreePlan &pl, bool same, int sum_mode, int D, double *Pv,
                           double *tmp) {
+    __shared__ int ok_sh;
+    const int t = threadIdx.x;
     const int nA = pl.ns[0], nB = same ? pl.ns[0] : pl.ns[1];
     const int gx0 = pl.G0[0], gy0 = same ? pl.G0[0] : pl.G0[1];
-    int ok = __ldcg(&sc->err) == 0;
-    for (int i = 0; i < kDotLevels * kDotLevels; i++) Pv[i] = 0.0;
-    for (int ia = 0; ia < nA; ia++)
-        for (int ib = 0; ib < nB; ib++) {
+    if (t == 0) ok_sh = __ldcg(&sc->err) == 0;
+    __syncthreads();
+    if (t < kDotLevels * kDotLevels) {
+        const int ia = t / kDotLevels, ib = t % kDotLevels;
+        double v = 0.0;
+        if (ia < nA && ib < nB) {
             long long S = 0;
             for (int i = 0; i < D; i++)
                 for (int j = 0; j < D; j++)
                     S += __ldcg(&sc->T[(ia * D + i) * kDotDigitRows + ib * D + j]) * (1LL << (8 * (i + j)));
             const int e = (gx0 - ia * pl.d) + (gy0 - ib * pl.d);
-            if (e < -1074 || e > 971 || S > (1LL << 53) || S < -(1LL << 53)) ok = 0;
-            Pv[ia * kDotLevels + ib] = (double)S * pow2(e);
+            if (e < -1074 || e > 971 || S > (1LL << 53) || S < -(1LL << 53)) ok_sh = 0;
+            v = (double)S * pow2(e);
         }
+        Pv[t] = v;
+    }
+    __syncthreads();
+    if (t != 0) return;
+    const int ok = ok_sh;
     // why a result is not used (traced by the host): 1 plan, 2 wait, 4 scale, 8 / 16 proof of x / y
     int why = (pl.valid ? 0 : 1) | (__ldcg(&sc->err) ? 2 : 0) | (ok || __ldcg(&sc->err) ? 0 : 4);
     for (int v = 0; v < (same ? 1 : 2); v++)
@@ -192,15 +204,15 @@ __device__ void di_finish(DotScratch *sc, const TreePlan &pl, bool same, int sum
     sc->out.status = valid;
     if (!valid) return;
     const int maxlevel = nA + nB - 2;  // DOT: fastMode is ignored (src/cpu/ozblas_gemm.cpp:26-29)
-    double t = 0.0;
+    double sum = 0.0;
     if (sum_mode == 1) {
         int np = 0;
         for_each_pair(nA, nB, maxlevel, [&](int ia, int ib) { tmp[np++] = Pv[ia * kDotLevels + ib]; });
-        t = nearsum(np, tmp, 1);
+        sum = nearsum(np, tmp, 1);
     } else {
-        for_each_pair(nA, nB, maxlevel, [&](int ia, int ib) { t += Pv[ia * kDotLevels + ib]; });
+        for_each_pair(nA, nB, maxlevel, [&](int ia, int ib) { sum += Pv[ia * kDotLevels + ib]; });
     }
-    sc->out.result = fma(1.0, t, 0.0 * 0.0);  // alpha = 1, beta = 0 as the DOT driver passes them
+    sc->out.result = fma(1.0, sum, 0.0 * 0.0);  // alpha = 1, beta = 0 as the DOT driver passes them
 }
 
 // RP digit rows per chunk of 128 elements: 16 (two digits, up to 8 levels) or
@@ -224,15 +236,12 @@ __global__ void __launch_bounds__(kDiThreads, 1)
     __shared__ double fin[2][kDotLevels * kDotLevels];
     __shared__ int last;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    __shared__ double sk[2][kDotLevels];
     plan_in_block(&sc->vs, rho, maxS, SAME, pl);
     for (int i = t; i < RP * RP; i += kDiThreads) red[i] = 0ull;
     __syncthreads();
-    if (t < 2 * kDotLevels) {  // sigma_s + 0x80808080 g_s: exact (an integer below 2^53 times g_s)
-        const int v = t / kDotLevels, s = t % kDotLevels;
-        sk[v][s] = pl.sig[v][s] + 2155905152.0 * pow2(pl.G0[v] - s * pl.d);
-    }
-    __syncthreads();
+    // sigma_0 + 0x80808080 g_0: exact (an integer below 2^53 times g_0)
+    const double sk0[2] = {pl.sig[0][0] + 2155905152.0 * pow2(pl.G0[0]),
+                           pl.sig[1][0] + 2155905152.0 * pow2(pl.G0[1])};
     const int L = pl.L;
     const bool work = pl.valid != 0 && L * D <= RP;  // (L * D > RP cannot happen for a valid plan)
     // (the group size G is the plan's, chain_group(rho, 4); the launch picks it)
@@ -267,6 +276,8 @@ __global__ void __launch_bounds__(kDiThreads, 1)
         };
         const uint32_t idesc = tc::idesc_i8(128, 128);
         const uint32_t acc = tmem_base + 128 * quad;  // this group's accumulator columns
+        const int wq = __shfl_sync(0xffffffffu, tq >> 5, 0);  // the warp within the group
+        const bool lead = tc::elect_one();
         // job k of this group (i = quad + k * kDiQuads), elements in xv / yv;
         // thread 0 of the group issues the group's MMAs once all its warps
         // have written the stage (group barrier 1 + quad)
@@ -289,24 +300,29 @@ __global__ void __launch_bounds__(kDiThreads, 1)
                 }
                 const unsigned before = prov[v];
                 if (pend)
-                    di_digits<D, E, G, true>(v ? yv : xv, sk[v], d, pl.ith[v], ra + v * kDiTile, pend, prov[v]);
+                    di_digits<D, E, G, true>(v ? yv : xv, sk0[v], d, L, pl.ith[v], ra + v * kDiTile, pend, prov[v]);
                 else
-                    di_digits<D, E, G, false>(v ? yv : xv, sk[v], d, pl.ith[v], ra + v * kDiTile, 0u, prov[v]);
+                    di_digits<D, E, G, false>(v ? yv : xv, sk0[v], d, L, pl.ith[v], ra + v * kDiTile, 0u, prov[v]);
                 if (lane == 0 && prov[v] != before) atomicOr(&sc->proven[v], prov[v]);  // share at once
             }
             tc::fence_proxy_async();
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&full[st]);
-            // the group's issuer, once all four warps have written the stage; on a
-            // timeout it issues nothing (the abort flag then stops every wait)
-            if (tq == 0 && tc::mbar_wait(&full[st], (k >> 1) & 1, &abort_flag, &sc->err, 2, kDiWaitNs)) {
-                tc::fence_after_sync();
-                const uint32_t sa = tc::smem_u32(tileA), sb = SAME ? sa : sa + kDiTile;
-                const uint64_t adesc = tc::smem_desc_k_sw128(sa), bdesc = tc::smem_desc_k_sw128(sb);
+            // the group's first warp issues once all four warps have written the
+            // stage (whole warp, one elected lane's predicate: under a branch on the
+            // lane an MMA takes 80 cycles, not 64, and FP64 stands still meanwhile);
+            // on a timeout it issues nothing (the abort flag then stops every wait)
+            if (wq == 0) {
+                const bool got = tc::mbar_wait(&full[st], (k >> 1) & 1, &abort_flag, &sc->err, 2, kDiWaitNs);
+                if (__all_sync(0xffffffffu, got)) {
+                    tc::fence_after_sync();
+                    const uint32_t sa = tc::smem_u32(tileA), sb = SAME ? sa : sa + kDiTile;
+                    const uint64_t adesc = tc::smem_desc_k_sw128(sa), bdesc = tc::smem_desc_k_sw128(sb);
 #pragma unroll
-                for (int kk = 0; kk < 4; kk++)  // +32 bytes along K = +2 in 16-byte units
-                    tc::mma_i8(acc, adesc + 2 * kk, bdesc + 2 * kk, idesc, (k > 0 || kk > 0) ? 1u : 0u);
-                tc::mma_commit(&empty[st]);
+                    for (int kk = 0; kk < 4; kk++)  // +32 bytes along K = +2 in 16-byte units
+                        tc::mma_i8_if(lead, acc, adesc + 2 * kk, bdesc + 2 * kk, idesc, (k > 0 || kk > 0) ? 1u : 0u);
+                    tc::mma_commit_if(lead, &empty[st]);
+                }
             }
             return true;
         };
@@ -331,8 +347,9 @@ __global__ void __launch_bounds__(kDiThreads, 1)
             }
             if (!produce(k + 1, xb, yb)) break;
         }
-        if (tq == 0) {
-            tc::mma_commit(&done);  // also when nothing was issued or the group gave up
+        __syncwarp();
+        if (wq == 0) {
+            tc::mma_commit_if(lead, &done);  // also when nothing was issued or the group gave up
             // every MMA of this group completes before TMEM is released (bounded)
             const uint64_t t0 = tc::globaltimer();
             while (!tc::mbar_try_wait(&done, 0) && tc::globaltimer() - t0 < 100000000ull) {
@@ -390,7 +407,7 @@ __global__ void __launch_bounds__(kDiThreads, 1)
     __syncthreads();
     if (!last) return;
     __threadfence();
-    if (t == 0) di_finish(sc, pl, SAME, sum_mode, D, fin[0], fin[1]);
+    di_finish(sc, pl, SAME, sum_mode, D, fin[0], fin[1]);
     __syncthreads();
     // leave the accumulators zeroed for the next use (replayed graphs skip the memset)
     for (int i = t; i < kDotDigitRows * kDotDigitRows; i += kDiThreads) sc->T[i] = 0;
