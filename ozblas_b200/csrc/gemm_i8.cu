@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int ntiles = p.tiles_m * p.tiles_n;
     const uint64_t wait_ns = g_i8_wait_ns;
 
@@ -169,15 +169,21 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        // The whole warp walks the groups and one elected lane's predicate issues
+        // (under a branch on the lane index an MMA takes 80 cycles, not 64).
+        {
+            const bool lead = tc::elect_one();
+            auto wait = [&](uint64_t *b, uint32_t parity) {
+                return __all_sync(0xffffffffu,
+                                  tc::mbar_wait(b, parity, &abort_flag, p.err, ERR_TIMEOUT_MMA, wait_ns)) != 0;
+            };
             const uint32_t idesc = tc::idesc_i8(I8_BM, I8_BN);
             uint32_t stage = 0, phase = 0, abuf = 0, aphase = 0;
             bool ok = true, issued = false;
             for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
                 for (int g = 0; g < p.n_groups && ok; g++) {
                     const int4 grp = p.groups[g];
-                    if (!tc::mbar_wait(&acc_empty[abuf], aphase ^ 1, &abort_flag, p.err, ERR_TIMEOUT_MMA,
-                                       wait_ns)) {
+                    if (!wait(&acc_empty[abuf], aphase ^ 1)) {
                         ok = false;
                         break;
                     }
@@ -187,8 +193,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
                     for (int it = grp.x; it < grp.y && ok; it++) {
                         const int4 item = p.items[it];
                         for (int kb = item.z; kb < item.w; kb++) {
-                            if (!tc::mbar_wait(&full[stage], phase, &abort_flag, p.err, ERR_TIMEOUT_MMA,
-                                               wait_ns)) {
+                            if (!wait(&full[stage], phase)) {
                                 ok = false;
                                 break;
                             }
@@ -198,11 +203,11 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
 #pragma unroll
                             for (int kk = 0; kk < I8_BK / 32; kk++) {
                                 // +32 bytes along K inside the 128-byte swizzle row = +2 in 16-byte units
-                                tc::mma_i8(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
+                                tc::mma_i8_if(lead, tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
                                 accumulate = 1;
                             }
                             issued = true;
-                            tc::mma_commit(&empty[stage]);
+                            tc::mma_commit_if(lead, &empty[stage]);
                             if (++stage == I8_NST) {
                                 stage = 0;
                                 phase ^= 1;
@@ -210,13 +215,13 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
                         }
                     }
                     if (!ok) break;
-                    tc::mma_commit(&acc_full[abuf]);
+                    tc::mma_commit_if(lead, &acc_full[abuf]);
                     abuf ^= 1;
                     if (abuf == 0) aphase ^= 1;
                 }
             }
             if (!ok && issued) {  // drain MMAs still in flight before TMEM is released
-                tc::mma_commit(drain);
+                tc::mma_commit_if(lead, drain);
                 const uint64_t t0 = tc::globaltimer();
                 while (!tc::mbar_try_wait(drain, 0) && tc::globaltimer() - t0 < 100000000ull) {
                 }
