@@ -450,7 +450,8 @@ __device__ inline void xparts_round(const XPart *parts, int np, double *sh, doub
 #pragma unroll
     for (int j = 0; j <= kXK2; j++) terms[j] = __shfl_sync(0xffffffffu, slot, j);
     terms[kXK2 + 1] = t == 0 ? -D : D;
-    const int flagged = s_flags;
+    // (with the top bin at the end of the range the layout's first grid overflows)
+    const int flagged = s_flags || Bt > kXBmax + 1;
     double r = 0.0;
     if (t < 2 && !flagged) {
         CrSum cs;
