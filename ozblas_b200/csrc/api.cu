@@ -24,6 +24,8 @@ int csrmv_presplit(cuozblasHandle_t *h, int m, int n, double alpha, const double
                    const int *colind, const int *rowptr, const double *x, double beta, double *y);
 int dot_fused(cuozblasHandle_t *h, int n, const double *x, const double *y, double *ret, bool *done, int *nA,
               int *nB);
+int dot_small(cuozblasHandle_t *h, int n, const double *x, const double *y, double *ret, bool *done, int *nA,
+              int *nB);
 int dot_exact(cuozblasHandle_t *h, int n, const double *x, const double *y, double *ret, bool *done, int *nA,
               int *nB);
 int csrmv_fused(cuozblasHandle_t *h, int m, int n, double alpha, const double *val, const int *colind,
@@ -109,13 +111,15 @@ static int finish(cuozblasHandle_t *h, double t0) {
     cudaError_t e = cudaStreamSynchronize(state(h)->stream);
     h->t_total = (float)(wall() - t0);
     State *st = state(h);
-    if (st->plain_timers && e == cudaSuccess) {  // the plain form's phases (src/cpu/ozblas_gemm.cpp timers)
+    if (st->span_timer && e == cudaSuccess) {
+        h->t_comp = ev_ms(h, 2, 3) * 1e-3f;
+    } else if (st->plain_timers && e == cudaSuccess) {  // the plain form's phases (src/cpu/ozblas_gemm.cpp timers)
         h->t_SplitA = ev_ms(h, 0, 1) * 1e-3f;
         h->t_SplitB = ev_ms(h, 1, 2) * 1e-3f;
         h->t_comp = ev_ms(h, 2, 3) * 1e-3f;
         h->t_sum = ev_ms(h, 3, 4) * 1e-3f;
     }
-    st->plain_timers = false;
+    st->plain_timers = st->span_timer = false;
     if (e != cudaSuccess) {
         fprintf(stderr, "cuozblas: CUDA error %s\n", cudaGetErrorString(e));
         return CUOZBLAS_STATUS_CUDA_ERROR;
@@ -128,8 +132,10 @@ static int dot_impl(cuozblasHandle_t *h, int n, const double *x, const double *y
     State *st = state(h);
     bool done = false;
     int nA = 0, nB = 0;
+    // up to a few thousand elements: one launch
+    if (h->splitEpsMode == 0) OZB_TRY(dot_small(h, n, x, y, ret, &done, &nA, &nB));
     // NearSum: one pass over x and y (exact dot, certified rounding, proven split counts)
-    if (h->splitEpsMode == 0 && h->sumMode == 1 && !st->env.dot_two_pass)
+    if (h->splitEpsMode == 0 && !done && h->sumMode == 1 && !st->env.dot_two_pass)
         OZB_TRY(dot_exact(h, n, x, y, ret, &done, &nA, &nB));
     if (h->splitEpsMode == 0 && !done) OZB_TRY(dot_fused(h, n, x, y, ret, &done, &nA, &nB));
     if (done) {

@@ -58,6 +58,7 @@ struct State {
     int64_t splitA_ld = 0;        // slice stride of the pre-split A (cuozblasDcsrmvSplitA)
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // phase timers (split A/B, products, sum)
     bool plain_timers = false;    // ev[0..4] hold a plain-form call's phases, read at the call's end
+    bool span_timer = false;      // ev[2..3] hold the span of the call's kernels, its only phase
     uint64_t launches = 0;        // kernels this handle has launched (cuozblasGetLaunchCount)
     // Device scratch that lives as long as the handle (zeroed at create; every
     // kernel that uses it leaves it zeroed): the one-pass DOT's statistics,
@@ -82,22 +83,24 @@ inline void counted(cuozblasHandle_t *h) { state(h)->launches++; }
 
 // Phase timers of the reference handle (t_SplitA, t_SplitB, t_comp), taken
 // with CUDA events on the handle's stream; read after the call's final sync.
-inline void ev_record(cuozblasHandle_t *h, int i) { cudaEventRecord(state(h)->ev[i], state(h)->stream); }
+// (event 1 ends a split: the call has phases, whatever path declined before)
+inline void ev_record(cuozblasHandle_t *h, int i) {
+    if (i == 1) state(h)->span_timer = false;
+    cudaEventRecord(state(h)->ev[i], state(h)->stream);
+}
 inline float ev_ms(cuozblasHandle_t *h, int a, int b) {
     float ms = 0.f;
     if (cudaEventElapsedTime(&ms, state(h)->ev[a], state(h)->ev[b]) != cudaSuccess) return 0.f;
     return ms;
 }
 
-// The device span of a call's kernels as the exec info's t_comp (events 0-2
-// before the first launch, 3-4 after the last, read at the call's end).
-inline void span_begin(cuozblasHandle_t *h) {
-    for (int i = 0; i < 3; i++) ev_record(h, i);
-}
+// The device span of a call's kernels as the exec info's t_comp (event 2
+// before the first launch, 3 after the last, read at the call's end); such a
+// call has no other phase, and five events cost a short call 10 us of its 57.
+inline void span_begin(cuozblasHandle_t *h) { ev_record(h, 2); }
 inline void span_end(cuozblasHandle_t *h) {
     ev_record(h, 3);
-    ev_record(h, 4);
-    state(h)->plain_timers = true;
+    state(h)->span_timer = true;
 }
 
 // Pinned staging of a handle, for host -> device uploads of schedules: a copy
