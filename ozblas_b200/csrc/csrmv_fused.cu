@@ -1066,7 +1066,7 @@ __global__ void __launch_bounds__(kCsrThreads, 4)
 // coalesced (values, columns, then the gathers of x, eight of each in flight
 // per thread), leaves each one's TwoProd in shared memory, and then one thread
 // adds each row.  What is left of the bound is half memory (84 MB for 10^6
-// rows of 7: 13 us), half the rows' TwoSum cascades.  10^6 rows: 36 us; the
+// rows of 7: 13 us), half the rows' TwoSum cascades.  10^6 rows: 34 us; the
 // kernel above, which also splits each row, 53.
 constexpr int kReadyRows = 256;
 
@@ -1107,12 +1107,28 @@ __global__ void __launch_bounds__(kReadyRows, 4)
     int slsb = 0, sbad = 0;
     bool wide = false;  // a product outside the range TwoProd keeps exact
     const int ntiles = (m + kReadyRows - 1) / kReadyRows;
+    // a tile's entries [first, last) and this thread's row in it, read a tile ahead
+    struct Rows {
+        int first, last, lo, hi;
+    };
+    auto rows_of = [&](int tile) {
+        Rows r{0, 0, 0, 0};
+        if (tile < ntiles) {
+            const int r0 = tile * kReadyRows, row = r0 + t;
+            r.first = rowptr[r0];
+            r.last = rowptr[m - r0 < kReadyRows ? m : r0 + kReadyRows];
+            r.lo = row < m ? rowptr[row] : 0;
+            r.hi = row < m ? rowptr[row + 1] : 0;
+        }
+        return r;
+    };
+    Rows next = rows_of(blockIdx.x);
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int r0 = tile * kReadyRows, row = r0 + t;
-        const int rend = m - r0 < kReadyRows ? m : r0 + kReadyRows;
-        const int base = rowptr[r0], end = rowptr[rend];
+        const Rows rw = next;
+        next = rows_of(tile + gridDim.x);
+        const int row = tile * kReadyRows + t, base = rw.first, end = rw.last;
         const bool active = row < m;
-        const int lo = active ? rowptr[row] - base : 0, len = active ? rowptr[row + 1] - base - lo : 0;
+        const int lo = rw.lo - base, len = rw.hi - rw.lo;
         const double yold = active ? y[row] : 0.0;
         double v[kCsrRowMax], xv[kCsrRowMax];
         int c[kCsrRowMax];
