@@ -184,8 +184,10 @@ __device__ __forceinline__ int g_line_e(const int *e, int l) {
     return CG ? __ldcg(e + l) : e[l];
 }
 
-// One block of 512 threads cuts block bk of operand o.  CG: the line
+// One block of G_ST threads cuts block bk of operand o.  CG: the line
 // exponents were written by other blocks of the same launch.
+constexpr int G_ST = 256;
+
 template <bool CG>
 __device__ __forceinline__ void g_digits_tile(const int4 bk, const GOp &o) {
     const int l0 = bk.y * G_T, k0 = bk.z * G_T;
@@ -196,21 +198,21 @@ __device__ __forceinline__ void g_digits_tile(const int4 bk, const GOp &o) {
     int f[16];
     uint32_t neg[4];
     if (!o.kcontig) {
-        // thread: row r, k quarter q (two halves of 16 values); lines contiguous across threads
-        const int r = t & 127, q = t >> 7, l = l0 + r;
+        // thread: row r, every other 16 k values; lines contiguous across threads
+        const int r = t & 127, l = l0 + r;
         const int E = l < o.lines ? g_line_e<CG>(o.e, l) : 0;
-        for (int hh = 0; hh < 2; hh++) {
+        for (int c16 = t >> 7; c16 < G_T / 16; c16 += G_ST / 128) {
             neg[0] = neg[1] = neg[2] = neg[3] = 0u;
 #pragma unroll
             for (int j = 0; j < 16; j++) {
-                const int kk = k0 + 32 * q + 16 * hh + j;
+                const int kk = k0 + 16 * c16 + j;
                 const double v = (l < o.lines && kk < o.k) ? o.X[(size_t)l + (size_t)kk * o.ld] : 0.0;
                 const DigitCut c = digit_cut(v, E);
                 m7[j] = c.m7;
                 f[j] = c.f;
                 if (v < 0.0) neg[j >> 2] |= 0xffu << (8 * (j & 3));
             }
-            const int ch = (2 * q + hh) ^ (r & 7);
+            const int ch = c16 ^ (r & 7);
             for (int s = 0; s < o.S; s++) {
                 uint32_t w[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
@@ -225,14 +227,15 @@ __device__ __forceinline__ void g_digits_tile(const int4 bk, const GOp &o) {
             }
         }
     } else {
-        // warp: rows w + 16 i (two passes of four rows); lane: k 4 lane .. 4 lane + 3 (k contiguous)
+        // warp: rows w + NW i (passes of four rows); lane: k 4 lane .. 4 lane + 3 (k contiguous)
+        constexpr int NW = G_ST / 32;
         const int w = t >> 5, lane = t & 31;
-        for (int pass = 0; pass < 2; pass++) {
+        for (int pass = 0; pass < G_T / (4 * NW); pass++) {
             int E[4];
             neg[0] = neg[1] = neg[2] = neg[3] = 0u;
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const int l = l0 + w + 16 * (4 * pass + i);
+                const int l = l0 + w + NW * (4 * pass + i);
                 E[i] = l < o.lines ? g_line_e<CG>(o.e, l) : 0;
 #pragma unroll
                 for (int qq = 0; qq < 4; qq++) {
@@ -247,7 +250,7 @@ __device__ __forceinline__ void g_digits_tile(const int4 bk, const GOp &o) {
             for (int s = 0; s < o.S; s++) {
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    const int r = w + 16 * (4 * pass + i);
+                    const int r = w + NW * (4 * pass + i);
                     uint32_t word = 0u;
 #pragma unroll
                     for (int qq = 0; qq < 4; qq++) {
@@ -263,7 +266,7 @@ __device__ __forceinline__ void g_digits_tile(const int4 bk, const GOp &o) {
     }
 }
 
-__global__ void __launch_bounds__(512) k_g_digits(const int4 *__restrict__ blocks, const GOp *__restrict__ ops) {
+__global__ void __launch_bounds__(G_ST) k_g_digits(const int4 *__restrict__ blocks, const GOp *__restrict__ ops) {
     const int4 bk = blocks[blockIdx.x];
     g_digits_tile<false>(bk, ops[bk.x]);
 }
@@ -316,61 +319,67 @@ __device__ __forceinline__ bool g_grid_barrier(unsigned *ctr, int *err) {
     return ok_sh != 0;
 }
 
-// Statistics of one block with 512 threads (as k_g_stats).
-__device__ __forceinline__ void g_stats_tile512(const int4 bk, const GOp &o, double *smx, int *slsb) {
+// Statistics of one block with G_ST threads (as k_g_stats), 32 loads of a
+// thread in flight together.
+__device__ __forceinline__ void g_stats_tile(const int4 bk, const GOp &o, double *smx, int *slsb) {
     const int l0 = bk.y * G_T, k0 = bk.z * G_T;
     const int t = threadIdx.x;
     if (!o.kcontig) {
-        const int l = l0 + (t & 127), kh = k0 + (t >> 7) * 32;
+        const int l = l0 + (t & 127);
         double mx = 0.0;
         int lsb = 0x7fffffff;
         if (l < o.lines) {
-            double v[32];  // every load in flight before the first use
+            for (int c32 = t >> 7; c32 < G_T / 32; c32 += G_ST / 128) {
+                double v[32];
 #pragma unroll
-            for (int j = 0; j < 32; j++) {
-                const int kk = kh + j;
-                v[j] = kk < o.k ? o.X[(size_t)l + (size_t)kk * o.ld] : 0.0;
+                for (int j = 0; j < 32; j++) {
+                    const int kk = k0 + 32 * c32 + j;
+                    v[j] = kk < o.k ? o.X[(size_t)l + (size_t)kk * o.ld] : 0.0;
+                }
+#pragma unroll
+                for (int j = 0; j < 32; j++) g_stat(v[j], mx, lsb);
             }
-#pragma unroll
-            for (int j = 0; j < 32; j++) g_stat(v[j], mx, lsb);
         }
         smx[t] = mx;
         slsb[t] = lsb;
         __syncthreads();
         if (t < 128 && l < o.lines) {
-            mx = ref_max(ref_max(smx[t], smx[t + 128]), ref_max(smx[t + 256], smx[t + 384]));
-            lsb = min(min(slsb[t], slsb[t + 128]), min(slsb[t + 256], slsb[t + 384]));
+            mx = ref_max(smx[t], smx[t + 128]);
+            lsb = min(slsb[t], slsb[t + 128]);
             if (mx > 0.0) atomicMax(&o.mx[l], (unsigned long long)__double_as_longlong(mx));
             if (lsb != 0x7fffffff) atomicMin(&o.lsb[l], lsb);
         }
         __syncthreads();
     } else {
+        constexpr int NW = G_ST / 32, RB = 8;  // rows per batch
         const int w = t >> 5, lane = t & 31;
-        double v[G_T / 16][4];  // every load of the thread in flight together
+        for (int i0 = 0; i0 < G_T / NW; i0 += RB) {
+            double v[RB][4];
 #pragma unroll
-        for (int i = 0; i < G_T / 16; i++) {
-            const int l = l0 + w + 16 * i;
+            for (int i = 0; i < RB; i++) {
+                const int l = l0 + w + NW * (i0 + i);
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int kk = k0 + 4 * lane + q;
-                v[i][q] = (l < o.lines && kk < o.k) ? o.X[(size_t)l * o.ld + kk] : 0.0;
+                for (int q = 0; q < 4; q++) {
+                    const int kk = k0 + 4 * lane + q;
+                    v[i][q] = (l < o.lines && kk < o.k) ? o.X[(size_t)l * o.ld + kk] : 0.0;
+                }
             }
-        }
 #pragma unroll
-        for (int i = 0; i < G_T / 16; i++) {
-            const int l = l0 + w + 16 * i;
-            if (l >= o.lines) break;  // uniform per warp
-            double mx = 0.0;
-            int lsb = 0x7fffffff;
+            for (int i = 0; i < RB; i++) {
+                const int l = l0 + w + NW * (i0 + i);
+                if (l >= o.lines) break;  // uniform per warp
+                double mx = 0.0;
+                int lsb = 0x7fffffff;
 #pragma unroll
-            for (int q = 0; q < 4; q++) g_stat(v[i][q], mx, lsb);
-            for (int sft = 16; sft > 0; sft >>= 1) {
-                mx = ref_max(mx, __shfl_xor_sync(0xffffffffu, mx, sft));
-                lsb = min(lsb, __shfl_xor_sync(0xffffffffu, lsb, sft));
-            }
-            if (lane == 0) {
-                if (mx > 0.0) atomicMax(&o.mx[l], (unsigned long long)__double_as_longlong(mx));
-                if (lsb != 0x7fffffff) atomicMin(&o.lsb[l], lsb);
+                for (int q = 0; q < 4; q++) g_stat(v[i][q], mx, lsb);
+                for (int sft = 16; sft > 0; sft >>= 1) {
+                    mx = ref_max(mx, __shfl_xor_sync(0xffffffffu, mx, sft));
+                    lsb = min(lsb, __shfl_xor_sync(0xffffffffu, lsb, sft));
+                }
+                if (lane == 0) {
+                    if (mx > 0.0) atomicMax(&o.mx[l], (unsigned long long)__double_as_longlong(mx));
+                    if (lsb != 0x7fffffff) atomicMin(&o.lsb[l], lsb);
+                }
             }
         }
     }
@@ -396,14 +405,68 @@ __device__ __forceinline__ int g_next_block(unsigned *ctr, int *slot) {
     return *slot;
 }
 
-__global__ void __launch_bounds__(512, 1) k_g_split(const GSplitArgs a) {
-    __shared__ double smx[512];
-    __shared__ int slsb[512];
+// Digit counts and buffers of all operands (the host carves the same ones),
+// one block: a thread per operand, the offsets by a scan of each chunk.
+__device__ __forceinline__ void g_carve(const GSplitArgs &a, unsigned long long *wsum) {
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    unsigned long long off0 = 0;
+    for (int i0 = 0; i0 < a.nops; i0 += G_ST) {
+        const int i = i0 + t;
+        unsigned long long bytes = 0;
+        int S = 0;
+        if (i < a.nops) {
+            S = __ldcg(&a.need[i]);
+            S = S < 1 ? 1 : S;
+            if (a.cap > 0 && S > a.cap) S = a.cap;
+            bytes = g_digit_bytes(S, a.ops[i].tiles_l, a.ops[i].nkb);
+        }
+        unsigned long long incl = bytes;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        if (lane == 31) wsum[w] = incl;
+        __syncthreads();
+        unsigned long long before = off0, total = off0;
+        for (int j = 0; j < G_ST / 32; j++) {
+            if (j < w) before += wsum[j];
+            total += wsum[j];
+        }
+        if (i < a.nops) {
+            a.ops[i].S = S;
+            a.ops[i].digits = a.dig_base + (before + incl - bytes);
+            if (a.mail) ((volatile int *)a.mail)[2 + i] = S;
+        }
+        off0 = total;
+        __syncthreads();
+    }
+    if (t == 0 && off0 > a.dig_capacity) atomicExch(a.err, 2);
+    if (!a.mail) return;
+    __threadfence_system();  // post the counts: the host builds the schedules while the digits are cut
+    __syncthreads();
+    if (t == 0) {
+        ((volatile int *)a.mail)[1] = *(volatile int *)a.err;
+        __threadfence_system();
+        ((volatile int *)a.mail)[0] = a.tag;
+        __threadfence_system();
+    }
+}
+
+// Bound by memory (both passes read the operands, the second writes S bytes
+// per element) about as much as by issuing the cuts, so two blocks of 256
+// threads share an SM and one loads while the other cuts: one block of 512
+// did these in turn and its operands' buffers were carved by one thread (512
+// operands: 350 us).  256 problems of 256..1024, 6.8 GB moved: 2340 -> 1980 us (three
+// blocks of 80 registers: 2100).
+__global__ void __launch_bounds__(G_ST, 2) k_g_split(const GSplitArgs a) {
+    __shared__ double smx[G_ST];
+    __shared__ int slsb[G_ST];
+    __shared__ unsigned long long wsum[G_ST / 32];
     __shared__ int next_sh;
     // 1: per-line max and lowest set bit
     for (int b = g_next_block(&a.bar[3], &next_sh); b < a.nblocks; b = g_next_block(&a.bar[3], &next_sh)) {
         const int4 bk = a.blocks[b];
-        g_stats_tile512(bk, a.ops[bk.x], smx, slsb);
+        g_stats_tile(bk, a.ops[bk.x], smx, slsb);
     }
     if (!g_grid_barrier(&a.bar[0], a.err)) return;
     // 2: line exponents and each operand's digit need
@@ -424,26 +487,7 @@ __global__ void __launch_bounds__(512, 1) k_g_split(const GSplitArgs a) {
         if (mx > 0.0) atomicMax(&a.need[lo], (E - __ldcg(&o.lsb[l]) + 6) / 7);
     }
     if (!g_grid_barrier(&a.bar[1], a.err)) return;
-    // digit counts and buffers (the host carves the same ones)
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        unsigned long long off = 0;
-        for (int i = 0; i < a.nops; i++) {
-            int S = __ldcg(&a.need[i]);
-            S = S < 1 ? 1 : S;
-            if (a.cap > 0 && S > a.cap) S = a.cap;
-            a.ops[i].S = S;
-            a.ops[i].digits = a.dig_base + off;
-            off += g_digit_bytes(S, a.ops[i].tiles_l, a.ops[i].nkb);
-        }
-        if (off > a.dig_capacity) atomicExch(a.err, 2);
-        if (a.mail) {  // post the counts: the host builds the schedules while the digits are cut
-            for (int i = 0; i < a.nops; i++) ((volatile int *)a.mail)[2 + i] = a.ops[i].S;
-            ((volatile int *)a.mail)[1] = *(volatile int *)a.err;
-            __threadfence_system();
-            ((volatile int *)a.mail)[0] = a.tag;
-            __threadfence_system();
-        }
-    }
+    if (blockIdx.x == 0) g_carve(a, wsum);
     if (!g_grid_barrier(&a.bar[2], a.err)) return;
     // 3: digits
     for (int b = g_next_block(&a.bar[4], &next_sh); b < a.nblocks; b = g_next_block(&a.bar[4], &next_sh)) {
@@ -804,7 +848,7 @@ int gemm_i8_batched(cuozblasHandle_t *h, char ta, char tb, int count, const int 
         if (occ == 0) {
             int coop = 0;
             if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_g_split, 512, 0) == cudaSuccess && occ > 0) {
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_g_split, G_ST, 0) == cudaSuccess && occ > 0) {
                 if (dev >= 0 && dev < 64) occ_cache[dev].store(occ);
             } else {
                 cudaGetLastError();
@@ -856,7 +900,7 @@ int gemm_i8_batched(cuozblasHandle_t *h, char ta, char tb, int count, const int 
         ga.tag = st->mail_seq;
         void *args[] = {&ga};
         counted(h);
-        if (cudaLaunchCooperativeKernel((const void *)k_g_split, dim3(coop_grid), dim3(512), args, 0, s) !=
+        if (cudaLaunchCooperativeKernel((const void *)k_g_split, dim3(coop_grid), dim3(G_ST), args, 0, s) !=
             cudaSuccess) {
             cudaGetLastError();  // not launched: the three-launch split
             fused = false;
@@ -935,7 +979,7 @@ int gemm_i8_batched(cuozblasHandle_t *h, char ta, char tb, int count, const int 
     if (!carved && !blocks.empty()) {
         OZB_CHECK(stage_upload(st, d_ops, ops.data(), sizeof(GOp) * nops, staged));
         counted(h);
-        k_g_digits<<<(unsigned)blocks.size(), 512, 0, s>>>(d_blocks, d_ops);
+        k_g_digits<<<(unsigned)blocks.size(), G_ST, 0, s>>>(d_blocks, d_ops);
         OZB_CHECK(cudaGetLastError());
     }
     ev_record(h, 1);
