@@ -635,11 +635,11 @@ __device__ __forceinline__ int lean_tau(unsigned mh, const double (&r)[kCsrRowMa
 }
 
 // The row's own chain (src/cpu/ozblas_split.cpp:779-815) as row_chain
-// computes it, keeping the slices.  Returns false when the row needs more
+// computes it, keeping the sigmas.  Returns false when the row needs more
 // than NA levels (and nSplitMax allows more) or holds Inf / NaN.
 template <int NA>
 __device__ __forceinline__ bool lean_chain(double (&r)[kCsrRowMax], int len, int shift, int epsmode, int maxS,
-                                           double (&sa)[kCsrRowMax][NA], int &na, int &z) {
+                                           double (&sig)[NA], int &na, int &z) {
     na = 0;
     z = 0;
     unsigned mh = 0u;
@@ -651,21 +651,19 @@ __device__ __forceinline__ bool lean_chain(double (&r)[kCsrRowMax], int len, int
     bool fin = len <= 0;
     double sg = 1.0;
     // Levels after the first zero remainder cut zeros into +0 slices (with the
-    // last sigma), which is what the products need there; only levels beyond
-    // nSplitMax are set to zero explicitly.
+    // last sigma), which is what the products need there.
 #pragma unroll
     for (int s = 0; s < NA; s++) {
         if (s < maxS) {  // uniform
-            if (!fin) sg = shift_sigma(0.75 * pow2(rho + lean_tau(mh, r)), shift);
-            unsigned nh = 0u;
-#pragma unroll
-            for (int e = 0; e < kCsrRowMax; e++) {
-                const double sl = (r[e] + sg) - sg;
-                r[e] = r[e] - sl;
-                sa[e][s] = sl;
-                nh = max(nh, hi_abs(r[e]));
-            }
             if (!fin) {
+                sg = shift_sigma(0.75 * pow2(rho + lean_tau(mh, r)), shift);
+                unsigned nh = 0u;
+#pragma unroll
+                for (int e = 0; e < kCsrRowMax; e++) {
+                    const double sl = (r[e] + sg) - sg;
+                    r[e] = r[e] - sl;
+                    nh = max(nh, hi_abs(r[e]));
+                }
                 na = s + 1;
                 bool zero = false;
                 if (nh == 0u) {
@@ -678,19 +676,20 @@ __device__ __forceinline__ bool lean_chain(double (&r)[kCsrRowMax], int len, int
                     z = s;
                     fin = true;
                 }
+                mh = nh;
             }
-            mh = nh;
-        } else {
-#pragma unroll
-            for (int e = 0; e < kCsrRowMax; e++) sa[e][s] = 0.0;
         }
+        sig[s] = sg;
     }
     return fin || na >= maxS;
 }
 
+// The entries are cut again along the row's sigmas (12 additions of some 55
+// operations per entry): kept slices would be 64 more registers, and with 12
+// warps per SM instead of 20 the chains' latency bounds the kernel.
 template <int SUM_MODE, int NA, int NB, int GX>
-__device__ __forceinline__ double lean_products(const double (&sa)[kCsrRowMax][NA], const double (&xv)[kCsrRowMax],
-                                                int len, int na, const double *xsig) {
+__device__ __forceinline__ double lean_products(const double (&v)[kCsrRowMax], const double (&sig)[NA], int maxS,
+                                                const double (&xv)[kCsrRowMax], int len, int na, const double *xsig) {
     double P[NA][NB];
 #pragma unroll
     for (int i = 0; i < NA; i++)
@@ -699,12 +698,18 @@ __device__ __forceinline__ double lean_products(const double (&sa)[kCsrRowMax][N
 #pragma unroll
     for (int e = 0; e < kCsrRowMax; e++) {
         if (e < len) {
-            double sx[NB];
+            double sa[NA], sx[NB], r = v[e];
+#pragma unroll
+            for (int s = 0; s < NA; s++) {
+                const double sl = (r + sig[s]) - sig[s];
+                r = r - sl;
+                sa[s] = s < maxS ? sl : 0.0;  // (uniform)
+            }
             cut_tree<GX, NB - 1>(xv[e], xsig, sx);
 #pragma unroll
             for (int ia = 0; ia < NA; ia++)
 #pragma unroll
-                for (int ib = 0; ib < NB; ib++) P[ia][ib] = fma(sa[e][ia], sx[ib], P[ia][ib]);
+                for (int ib = 0; ib < NB; ib++) P[ia][ib] = fma(sa[ia], sx[ib], P[ia][ib]);
         }
     }
     if (SUM_MODE == 0) {
@@ -734,7 +739,7 @@ __device__ __forceinline__ double lean_products(const double (&sa)[kCsrRowMax][N
 }
 
 template <int SUM_MODE, int NA, int GX>
-__global__ void __launch_bounds__(kCsrThreads, NA >= 4 ? 3 : 4)
+__global__ void __launch_bounds__(kCsrThreads, 4)
     k_csrmv_lean(int m, int n, const double *__restrict__ val, const int *__restrict__ colind,
                  const int *__restrict__ rowptr, const double *__restrict__ x, int shift, int epsmode, int maxS,
                  double alpha, double beta, double *__restrict__ y, CsrScratch *__restrict__ sc,
@@ -824,12 +829,12 @@ __global__ void __launch_bounds__(kCsrThreads, NA >= 4 ? 3 : 4)
         bool defer = active && len > kCsrRowMax;
         const bool work = active && !defer;
         const double yold = active ? S.yold[t] : 0.0;
-        double sa[kCsrRowMax][NA];
+        double sig[NA];
         int na = 0, z = 0;
         if (work) {
             double r[kCsrRowMax];
             lean_read(S.val, t, r);
-            if (!lean_chain<NA>(r, len, shift, epsmode, maxS, sa, na, z)) defer = true;
+            if (!lean_chain<NA>(r, len, shift, epsmode, maxS, sig, na, z)) defer = true;
         }
         if (defer && append_slow) slow_rows[atomicAdd(&sc->nslow, 1)] = row;
         if (work && !defer) zmax = z > zmax ? z : zmax;
@@ -840,18 +845,19 @@ __global__ void __launch_bounds__(kCsrThreads, NA >= 4 ? 3 : 4)
         cp_async_commit();
         // ---- phase 2: products and sums
         if (work && !defer) {
-            double xv[kCsrRowMax];
+            double v[kCsrRowMax], xv[kCsrRowMax];
+            lean_read(S.val, t, v);
             lean_read(S.xg, t, xv);
             double tsum;
             switch (nB) {  // uniform
-                case 1: tsum = lean_products<SUM_MODE, NA, 1, GX>(sa, xv, len, na, xs_sigma); break;
-                case 2: tsum = lean_products<SUM_MODE, NA, 2, GX>(sa, xv, len, na, xs_sigma); break;
-                case 3: tsum = lean_products<SUM_MODE, NA, 3, GX>(sa, xv, len, na, xs_sigma); break;
-                case 4: tsum = lean_products<SUM_MODE, NA, 4, GX>(sa, xv, len, na, xs_sigma); break;
-                case 5: tsum = lean_products<SUM_MODE, NA, 5, GX>(sa, xv, len, na, xs_sigma); break;
-                case 6: tsum = lean_products<SUM_MODE, NA, 6, GX>(sa, xv, len, na, xs_sigma); break;
-                case 7: tsum = lean_products<SUM_MODE, NA, 7, GX>(sa, xv, len, na, xs_sigma); break;
-                default: tsum = lean_products<SUM_MODE, NA, 8, GX>(sa, xv, len, na, xs_sigma); break;
+                case 1: tsum = lean_products<SUM_MODE, NA, 1, GX>(v, sig, maxS, xv, len, na, xs_sigma); break;
+                case 2: tsum = lean_products<SUM_MODE, NA, 2, GX>(v, sig, maxS, xv, len, na, xs_sigma); break;
+                case 3: tsum = lean_products<SUM_MODE, NA, 3, GX>(v, sig, maxS, xv, len, na, xs_sigma); break;
+                case 4: tsum = lean_products<SUM_MODE, NA, 4, GX>(v, sig, maxS, xv, len, na, xs_sigma); break;
+                case 5: tsum = lean_products<SUM_MODE, NA, 5, GX>(v, sig, maxS, xv, len, na, xs_sigma); break;
+                case 6: tsum = lean_products<SUM_MODE, NA, 6, GX>(v, sig, maxS, xv, len, na, xs_sigma); break;
+                case 7: tsum = lean_products<SUM_MODE, NA, 7, GX>(v, sig, maxS, xv, len, na, xs_sigma); break;
+                default: tsum = lean_products<SUM_MODE, NA, 8, GX>(v, sig, maxS, xv, len, na, xs_sigma); break;
             }
             const double ynew = fma(alpha, tsum, beta * yold);
             y[row] = ynew;
@@ -1017,10 +1023,10 @@ __global__ void __launch_bounds__(kCsrThreads, 4)
         if (work) {
             // len 2^(106 - rho_A - rho_x + log2 shift) < 2^53 in product-grid units
             if (len > 0 && ceil_log2_small(len) + 106 - rho_rule(len, epsmode) - rho_x + lg_shift > 53) defer = true;
-            double r[kCsrRowMax], sa[kCsrRowMax][NA];
+            double r[kCsrRowMax], sig[NA];
             lean_read(S.val, t, r);
             int na = 0, z = 0;
-            if (!lean_chain<NA>(r, len, shift, epsmode, maxS, sa, na, z))
+            if (!lean_chain<NA>(r, len, shift, epsmode, maxS, sig, na, z))
                 listed = true;  // more levels than held, or Inf / NaN
             else if (len > 0 && z >= maxS)
                 defer = true;   // an incomplete split
