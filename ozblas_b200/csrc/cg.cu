@@ -449,7 +449,7 @@ int cg_graph(cuozblasHandle_t *h, int n, const double *val, const int *colind, c
     }
     CG_CHECK(ce);
     CG_CHECK(cudaGraphInstantiate(&exec, graph, 0));
-    const int per_iter = (fused_dots ? (no_proof ? 4 : 5) : 8) + (nslow > 0 ? (nslow + 8191) / 8192 : 0);
+    const int per_iter = (fused_dots ? (no_proof ? 4 : 5) : 8) + (nslow > 0 ? (h->sumMode == 1 ? (nslow + 8191) / 8192 : 1) : 0);
     // device clock against the host's, for the elapsed-time history
     k_cg_stamp<<<1, 1, 0, s>>>(stamp_dev + maxiter + 1);
     unsigned long long dev0 = 0;

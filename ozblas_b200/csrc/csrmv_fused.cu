@@ -348,7 +348,13 @@ __device__ __forceinline__ double slice_at(double v, const double *sig, int lv) 
 }
 
 // General per-row kernel for the deferred rows: any length, any level count;
-// slices recomputed on the fly; NearSum terms in `terms` (slot x maxS*kCsrLv).
+// slices recomputed on the fly.  SUM_MODE 0: FSum; 1: NearSum, its terms in
+// `terms` (slot x maxS*kCsrLv); 2: NearSum as the terms come (CrSum), rows it
+// cannot certify listed in `again` (sc->nslow counts them) and not written.
+// A row is a chain of some 10^5 dependent cycles, so modes 0 and 2, which need
+// no terms in memory, take all rows in one launch; mode 1 takes kCsrSlowChunk
+// rows at a time, a third of the chip.  200 000 rows of 9 to 12 entries, FSum:
+// 25 launches of 107 us -> one of 422; 72 000 with NearSum: 9 of 120 -> one of 166.
 template <int SUM_MODE>
 __global__ void __launch_bounds__(128) k_csrmv_slow(int nrows, const int *__restrict__ rows,
                                                     const double *__restrict__ val, const int *__restrict__ colind,
@@ -356,7 +362,8 @@ __global__ void __launch_bounds__(128) k_csrmv_slow(int nrows, const int *__rest
                                                     int shift, int epsmode, int maxS, double alpha, double beta,
                                                     double *__restrict__ y, CsrScratch *__restrict__ sc,
                                                     double *__restrict__ terms, VecStats *__restrict__ ystats,
-                                                    int ystats_index, const int *__restrict__ gate) {
+                                                    int ystats_index, const int *__restrict__ gate,
+                                                    int *__restrict__ again = nullptr) {
     if (gate && *gate == 0) return;  // uniform
     if (!sc->valid) return;          // uniform: x's chain is not proven
     __shared__ double red[4];
@@ -396,7 +403,8 @@ __global__ void __launch_bounds__(128) k_csrmv_slow(int nrows, const int *__rest
         atomicMax((int *)&sc->zmax, z);
         double tsum = 0.0;
         int np = 0;
-        double *tm = terms + (size_t)slot * kMaxSplitDefault * kCsrLv;
+        CrSum cs;
+        double *tm = SUM_MODE == 1 ? terms + (size_t)slot * kMaxSplitDefault * kCsrLv : nullptr;
         const int maxlevel = na + nB - 2;
         for (int ik = 0; ik <= maxlevel; ik++) {
             const int ia0 = ik - (nB - 1) > 0 ? ik - (nB - 1) : 0, ia1 = ik < na - 1 ? ik : na - 1;
@@ -407,14 +415,20 @@ __global__ void __launch_bounds__(128) k_csrmv_slow(int nrows, const int *__rest
                     p = fma(slice_at(val[i], sa, ia), slice_at(x[colind[i]], sc->sigma, ib), p);
                 if (SUM_MODE == 1)
                     tm[np] = p;
+                else if (SUM_MODE == 2)
+                    cs.add(p);
                 else
                     tsum += p;
                 np++;
             }
         }
         if (SUM_MODE == 1) tsum = nearsum(np, tm, 1);
-        ynew = fma(alpha, tsum, beta * y[row]);
-        y[row] = ynew;
+        if (SUM_MODE == 2 && !cs.finish(tsum)) {
+            again[atomicAdd(&sc->nslow, 1)] = row;
+        } else {
+            ynew = fma(alpha, tsum, beta * y[row]);
+            y[row] = ynew;
+        }
     }
     if (ystats) {
         double mx = 0.0;
@@ -1345,8 +1359,9 @@ int csr_rows_launch(cudaStream_t s, const CsrmvArgs &a, CsrScratch *sc, int *slo
         else
             launch_lean<0, 4>(gx, rb, s, a, sc, slow, append, ystats, ystats_index, gate);
     }
-    for (int c0 = 0; c0 < fixed_slow; c0 += kCsrSlowChunk) {
-        const int nr = fixed_slow - c0 < kCsrSlowChunk ? fixed_slow - c0 : kCsrSlowChunk;
+    const int chunk = a.sum_mode == 1 ? kCsrSlowChunk : fixed_slow;  // FSum keeps no terms
+    for (int c0 = 0; c0 < fixed_slow; c0 += chunk) {
+        const int nr = fixed_slow - c0 < chunk ? fixed_slow - c0 : chunk;
         if (a.sum_mode == 1)
             k_csrmv_slow<1><<<(nr + 127) / 128, 128, 0, s>>>(nr, slow + c0, a.val, a.colind, a.rowptr, a.x, a.shift,
                                                             a.epsmode, a.maxS, a.alpha, a.beta, a.y, sc, terms,
@@ -1412,17 +1427,36 @@ int csrmv_fused(cuozblasHandle_t *h, int m, int n, double alpha, const double *v
     if (nslow > 0) {
         double *terms = ar.take<double>((uint64_t)kCsrSlowChunk * kMaxSplitDefault * kCsrLv);
         if (!ar.ok) return CUOZBLAS_STATUS_WORKSPACE;
-        for (int c0 = 0; c0 < nslow; c0 += kCsrSlowChunk) {
-            const int nr = nslow - c0 < kCsrSlowChunk ? nslow - c0 : kCsrSlowChunk;
+        const int grid = (nslow + 127) / 128;
+        int nagain = nslow;  // NearSum rows left for the kernel that keeps its terms
+        const int *list = slow;
+        if (h->sumMode == 0) {
             counted(h);
-            if (h->sumMode == 1)
-                k_csrmv_slow<1><<<(nr + 127) / 128, 128, 0, s>>>(nr, slow + c0, val, colind, rowptr, x, shift,
-                                                                h->splitEpsMode, maxS, alpha, beta, y, sc, terms,
-                                                                nullptr, 0, nullptr);
-            else
-                k_csrmv_slow<0><<<(nr + 127) / 128, 128, 0, s>>>(nr, slow + c0, val, colind, rowptr, x, shift,
-                                                                h->splitEpsMode, maxS, alpha, beta, y, sc, terms,
-                                                                nullptr, 0, nullptr);
+            k_csrmv_slow<0><<<grid, 128, 0, s>>>(nslow, slow, val, colind, rowptr, x, shift, h->splitEpsMode, maxS,
+                                                 alpha, beta, y, sc, nullptr, nullptr, 0, nullptr);
+            OZB_CHECK(cudaGetLastError());
+            nagain = 0;
+        } else {
+            int *again = ar.take<int>(nslow);
+            if (ar.ok) {
+                OZB_CHECK(cudaMemsetAsync(&sc->nslow, 0, sizeof(int), s));
+                counted(h);
+                k_csrmv_slow<2><<<grid, 128, 0, s>>>(nslow, slow, val, colind, rowptr, x, shift, h->splitEpsMode,
+                                                     maxS, alpha, beta, y, sc, nullptr, nullptr, 0, nullptr, again);
+                OZB_CHECK(cudaGetLastError());
+                OZB_CHECK(cudaMemcpyAsync(&nagain, &sc->nslow, sizeof(int), cudaMemcpyDeviceToHost, s));
+                OZB_CHECK(cudaStreamSynchronize(s));
+                list = again;
+            } else {  // no room for the list: every row with its terms
+                ar.ok = true;
+            }
+        }
+        for (int c0 = 0; c0 < nagain; c0 += kCsrSlowChunk) {
+            const int nr = nagain - c0 < kCsrSlowChunk ? nagain - c0 : kCsrSlowChunk;
+            counted(h);
+            k_csrmv_slow<1><<<(nr + 127) / 128, 128, 0, s>>>(nr, list + c0, val, colind, rowptr, x, shift,
+                                                            h->splitEpsMode, maxS, alpha, beta, y, sc, terms,
+                                                            nullptr, 0, nullptr);
             OZB_CHECK(cudaGetLastError());
         }
         OZB_CHECK(cudaMemcpyAsync(&res[3], &sc->zmax, sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -93,3 +93,29 @@ def test_exact_reduction_bins(n, kind, oracle, handle, ozb, cuda):
     r, info = oracle.ddot(make_flags(sumMode=1), x, y)
     assert np.float64(d).view(np.int64) == np.float64(r).view(np.int64), (d, r)
     assert (handle.nSplitA, handle.nSplitB) == (info.nSplitA, info.nSplitB)
+
+
+@pytest.mark.parametrize("sm", [0, 1])
+def test_many_deferred_rows(sm, oracle, handle, ozb, cuda):
+    """More rows of over 8 entries than one launch with terms in memory takes, some with sums that need NearSum itself."""
+    rng = np.random.default_rng(3)
+    n = 20000
+    lens = np.where(np.arange(n) % 2 == 0, 10, 3)
+    rowptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    colind = rng.integers(0, n, int(rowptr[-1])).astype(np.int32)
+    val = oracle.phi_vector(len(colind), 1.0, 7)
+    x, y0 = oracle.phi_vector(n, 1.0, 8), oracle.phi_vector(n, 1.0, 9)
+    for r in range(0, n, 40):  # entries that cancel in pairs: zero sums, which the certified sum leaves to NearSum
+        lo = rowptr[r]
+        colind[lo + 5:lo + 10] = colind[lo:lo + 5]
+        val[lo + 5:lo + 10] = -val[lo:lo + 5]
+    ref, info = oracle.dcsrmv(make_flags(sumMode=sm), n, n, 0.5, val, colind, rowptr, x, -2.0, y0)
+
+    def dev(a):
+        return cuda.from_numpy(np.ascontiguousarray(a)).cuda()
+
+    handle.sumMode = sm
+    dy = dev(y0)
+    ozb.dcsrmv(handle, "n", n, n, len(val), 0.5, dev(val), dev(colind), dev(rowptr), dev(x), -2.0, dy)
+    assert bits_equal(dy.cpu().numpy(), ref), first_diff(dy.cpu().numpy(), ref)
+    assert (handle.nSplitA, handle.nSplitB) == (info.nSplitA, info.nSplitB)
