@@ -654,7 +654,7 @@ def config1_extras(ozb, torch, cpu=True, n=1024):
     h.close()
     flops = 2.0 * n ** 3
     peaks, _ = measured_peaks()
-    digits = (53 - int(ozb.rule_rho(n, 0)) + 1 + 6) // 7  # int8 digit planes per FP64 slice
+    digits = (53 - int(ozb.rule_rho(n, 0)) + 1 + 7) // 8  # balanced int8 digit planes per FP64 slice
     kern = min(kms[1:])
     i8_ops = pairs * digits * digits * flops
     rec = {"ms": ms, "TFLOPS": flops / ms / 1e9, "slices": [nA, nB], "pairs": pairs,

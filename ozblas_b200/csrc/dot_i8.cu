@@ -32,9 +32,11 @@
 //
 // CTA (one per SM): 3 producer groups of 4 warps, two 32 KiB stages per group.
 // Each group cuts its jobs into its stages in turn, loading the next job's
-// elements before cutting the current one; one thread of the group waits for
+// elements before cutting the current one; the group's first warp waits for
 // its four warps (a per-stage mbarrier) and issues the group's MMAs into the
-// group's own 128-column TMEM accumulator, so no other thread touches it.
+// group's own 128-column TMEM accumulator, so no other warp touches it.
+// 2^24 elements: 115 us; 144 with eight levels cut whatever the plan, the pairs
+// formed by one thread and single-lane issue.
 // Proven levels are shared through DotScratch::proven at once, so warps stop
 // voting on them.  The first group sums the three accumulators at the end.
 // Every wait is bounded and every warp collective is reached by all lanes

@@ -791,7 +791,7 @@ __global__ void __launch_bounds__(kPpThreads, 1)
                     }
                     if (!__all_sync(0xffffffffu, ok)) return false;
                     __syncwarp();
-                    const auto *from = reinterpret_cast<const decltype(&t[0])>(p.pbuf) +
+                    const auto *from = reinterpret_cast<decltype(&t[0])>(p.pbuf) +
                                        (size_t)(blockIdx.x - 1) * (128 * S::BN) + (size_t)(half * CW) * 128 + row;
 #pragma unroll
                     for (int c = 0; c < (FUSED ? CW : 1); c++) t[c] = __ldcg(from + c * 128);
