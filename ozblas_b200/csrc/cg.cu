@@ -97,11 +97,26 @@ __global__ void __launch_bounds__(256) k_cg_update_p(int n, double *__restrict__
     const double be = d->beta;
     double mx = 0.0;
     int lsb = 0, bad = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        // p = beta p, then p = fma(1, r, p): two roundings, never contracted into one fma
-        const double pi = fma(1.0, r[i], __dmul_rn(be, p[i]));
-        p[i] = pi;
-        scan_elem(pi, mx, lsb, bad);
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    constexpr int U = 4;  // elements per step, their loads in flight together
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += U * stride) {
+        double rv[U], pv[U];
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            const int64_t e = i + k * stride;
+            rv[k] = e < n ? r[e] : 0.0;
+            pv[k] = e < n ? p[e] : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            const int64_t e = i + k * stride;
+            if (e < n) {
+                // p = beta p, then p = fma(1, r, p): two roundings, never contracted into one fma
+                const double pi = fma(1.0, rv[k], __dmul_rn(be, pv[k]));
+                p[e] = pi;
+                scan_elem(pi, mx, lsb, bad);
+            }
+        }
     }
     scan_commit(ps_a, 0, mx, lsb, bad, red);
     scan_commit(ps_b, 0, mx, lsb, bad, red);
@@ -238,7 +253,7 @@ __global__ void __launch_bounds__(256) k_cg_xr_rr(int n, double *__restrict__ x,
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t iw = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31);
     // U elements per lane per step, their four loads each in flight together
-    constexpr int U = 2;
+    constexpr int U = 4;
     const int64_t steps = iw < n ? ((int64_t)n - iw + U * stride - 1) / (U * stride) : 0;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (int64_t s = 0; s < steps; s++, i += U * stride) {
@@ -267,7 +282,7 @@ __global__ void __launch_bounds__(256) k_cg_xr_rr(int n, double *__restrict__ x,
         xacc_fit(acc, __reduce_max_sync(0xffffffffu, hi));
 #pragma unroll
         for (int k = 0; k < U; k++) xacc_product(acc, rv[k], rv[k]);
-        if ((s & 31) == 31) xacc_normalize(acc);  // every 64 products per lane
+        if ((s & 15) == 15) xacc_normalize(acc);  // every 64 products per lane
     }
     scan_commit(rs, 0, mx, lsb, bad, red);
     if (!xreduce_finish(acc, xr, &res_sh, &cert_sh)) return;
@@ -440,7 +455,7 @@ int cg_graph(cuozblasHandle_t *h, int n, const double *val, const int *colind, c
                 cap = dot_tree_launch(s, nsm, n, r, r, rho, maxS, h->sumMode, drr, &d->gate, state(h)->env.dot_tree);
             k_cg_beta<<<1, 1, 0, s>>>(d, drr, res_dev, stamp_dev);
         }
-        k_cg_update_p<<<ub, 256, 0, s>>>(n, p, r, d, &cs->vs, &dpq->vs);
+        k_cg_update_p<<<ub < nsm * 4 ? ub : nsm * 4, 256, 0, s>>>(n, p, r, d, &cs->vs, &dpq->vs);
     }
     const cudaError_t ce = cudaStreamEndCapture(s, &graph);
     if (cap) {
