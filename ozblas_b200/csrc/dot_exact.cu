@@ -256,7 +256,8 @@ __device__ void dot_ring_publish(DotScratch *sc, DotExactScratch *xs, int rho, i
 template <int G, bool SAME>
 __global__ void __launch_bounds__(kXThreads) k_dot_exact_ring(int n, const double *__restrict__ x,
                                                               const double *__restrict__ y, DotScratch *__restrict__ sc,
-                                                              DotExactScratch *__restrict__ xs, int rho, int maxS) {
+                                                              DotExactScratch *__restrict__ xs, int rho, int maxS,
+                                                              DotStatus *mail) {
     constexpr int V = SAME ? 1 : 2;
     static_assert(dot_ring_bytes<SAME>() >= 256 * (kXK2 + 3) * (int)sizeof(double), "ring too small for the scratch");
     extern __shared__ __align__(16) double2 dring[];
@@ -381,6 +382,7 @@ __global__ void __launch_bounds__(kXThreads) k_dot_exact_ring(int n, const doubl
         xs->certified = cert_sh;
     }
     dot_ring_publish<G, SAME>(sc, xs, rho, maxS, res_sh, cert_sh);
+    if (t == 0) dot_post(sc, mail);
 }
 
 template <int G, bool SAME>
@@ -505,6 +507,8 @@ int dot_exact(cuozblasHandle_t *h, int n, const double *x, const double *y, doub
         return CUOZBLAS_STATUS_SUCCESS;
     };
     DotStatus res{};
+    DotStatus *mail = reinterpret_cast<DotStatus *>(st->d_mail);
+    memcpy(st->h_mail, &res, sizeof(res));
     bool need_prove = true;
     if (aligned) {
         // one wave of the ring kernel: its resident blocks per SM x SMs
@@ -536,9 +540,9 @@ int dot_exact(cuozblasHandle_t *h, int n, const double *x, const double *y, doub
 #define OZB_RING(GG)                                                                                          \
     do {                                                                                                    \
         if (same)                                                                                           \
-            k_dot_exact_ring<GG, true><<<rb, kXThreads, smem, st->stream>>>(n, x, y, sc, xs, rho, maxS);     \
+            k_dot_exact_ring<GG, true><<<rb, kXThreads, smem, st->stream>>>(n, x, y, sc, xs, rho, maxS, mail); \
         else                                                                                                \
-            k_dot_exact_ring<GG, false><<<rb, kXThreads, smem, st->stream>>>(n, x, y, sc, xs, rho, maxS);    \
+            k_dot_exact_ring<GG, false><<<rb, kXThreads, smem, st->stream>>>(n, x, y, sc, xs, rho, maxS, mail); \
     } while (0)
         switch (G) {
             case 1: OZB_RING(1); break;
@@ -551,7 +555,8 @@ int dot_exact(cuozblasHandle_t *h, int n, const double *x, const double *y, doub
         span_end(h);
         // the ring kernel's last block proved the chains from its candidates (status 1),
         // found the one-pass result unusable (0), or left levels for the proof kernel (2)
-        OZB_TRY(read_status(res));
+        OZB_CHECK(cudaStreamSynchronize(st->stream));
+        memcpy(&res, st->h_mail, sizeof(res));
         need_prove = res.status == 2;
     } else {
         if (same)

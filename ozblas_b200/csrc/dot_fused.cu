@@ -183,7 +183,7 @@ template <int G, bool SAME, bool ALIGNED>
 __global__ void __launch_bounds__(kDotThreads, 1) k_dot_tree(int n, const double *__restrict__ x,
                                                              const double *__restrict__ y, int rho, int maxS,
                                                              int sum_mode, DotScratch *__restrict__ sc,
-                                                             const int *__restrict__ gate) {
+                                                             const int *__restrict__ gate, DotStatus *mail) {
     if (gate && *gate == 0) return;  // uniform: a captured solver step that is switched off
     __shared__ TreePlan pl;
     extern __shared__ __align__(16) double2 ring_raw[];  // [kDotStages][SAME ? 1 : 2][kDotThreads]
@@ -281,7 +281,10 @@ __global__ void __launch_bounds__(kDotThreads, 1) k_dot_tree(int n, const double
     double *Pv = &red[0][0], *tmp = &red[1][0];
     if (t < kDotLevels * kDotLevels) Pv[t] = __ldcg(&sc->P[t]);
     __syncthreads();
-    if (t == 0) dot_finish(sc, pl, rho, SAME, sum_mode, Pv, tmp);
+    if (t == 0) {
+        dot_finish(sc, pl, rho, SAME, sum_mode, Pv, tmp);
+        if (mail) dot_post(sc, mail);
+    }
     __syncthreads();
     // leave the accumulators zeroed for the next use (replayed graphs skip the memset)
     if (t < kDotLevels * kDotLevels) sc->P[t] = 0.0;
@@ -294,15 +297,15 @@ __global__ void __launch_bounds__(kDotThreads, 1) k_dot_tree(int n, const double
 
 template <int G, bool SAME>
 static int launch_tree(bool aligned, int grid, cudaStream_t s, int n, const double *x, const double *y, int rho,
-                       int maxS, int sum_mode, DotScratch *sc, const int *gate) {
+                       int maxS, int sum_mode, DotScratch *sc, const int *gate, DotStatus *mail) {
     if (aligned) {
         const int smem = kDotStages * (SAME ? 1 : 2) * kDotThreads * (int)sizeof(double2);
         static std::atomic<uint64_t> attr{0};  // devices already opted in, per instantiation
         if (smem_optin((const void *)k_dot_tree<G, SAME, true>, smem, attr) != cudaSuccess)
             return CUOZBLAS_STATUS_CUDA_ERROR;
-        k_dot_tree<G, SAME, true><<<grid, kDotThreads, smem, s>>>(n, x, y, rho, maxS, sum_mode, sc, gate);
+        k_dot_tree<G, SAME, true><<<grid, kDotThreads, smem, s>>>(n, x, y, rho, maxS, sum_mode, sc, gate, mail);
     } else {
-        k_dot_tree<G, SAME, false><<<grid, kDotThreads, 0, s>>>(n, x, y, rho, maxS, sum_mode, sc, gate);
+        k_dot_tree<G, SAME, false><<<grid, kDotThreads, 0, s>>>(n, x, y, rho, maxS, sum_mode, sc, gate, mail);
     }
     return CUOZBLAS_STATUS_SUCCESS;
 }
@@ -344,7 +347,7 @@ int dot_scan_launch(cudaStream_t s, int nsm, int n, const double *x, const doubl
 }
 
 int dot_tree_launch(cudaStream_t s, int nsm, int n, const double *x, const double *y, int rho, int maxS,
-                    int sum_mode, DotScratch *sc, const int *gate, bool tree_only) {
+                    int sum_mode, DotScratch *sc, const int *gate, bool tree_only, DotStatus *mail) {
     const int G = chain_group(rho, 4);  // levels cut from one base value
     const bool same = (x == y);
     const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u) == 0;
@@ -352,27 +355,27 @@ int dot_tree_launch(cudaStream_t s, int nsm, int n, const double *x, const doubl
     // level take the tensor-core pass (it holds every valid plan; below that
     // length its fixed costs outweigh the FP64 tree pass, which takes the rest)
     if (aligned && n >= (1 << 22) && dot_i8_digits(rho) > 0 && !tree_only)
-        return dot_i8_launch(s, nsm, n, x, y, rho, maxS, sum_mode, sc, gate);
+        return dot_i8_launch(s, nsm, n, x, y, rho, maxS, sum_mode, sc, gate, mail);
     int fblocks = (int)(((int64_t)n + 2 * kDotThreads - 1) / (2 * kDotThreads));
     if (fblocks > nsm) fblocks = nsm;  // ~250 registers per thread: one 256-thread block per SM
     if (fblocks < 1) fblocks = 1;
     int ls;
     switch (G) {
         case 1:
-            ls = same ? launch_tree<1, true>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate)
-                      : launch_tree<1, false>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate);
+            ls = same ? launch_tree<1, true>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate, mail)
+                      : launch_tree<1, false>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate, mail);
             break;
         case 2:
-            ls = same ? launch_tree<2, true>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate)
-                      : launch_tree<2, false>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate);
+            ls = same ? launch_tree<2, true>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate, mail)
+                      : launch_tree<2, false>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate, mail);
             break;
         case 3:
-            ls = same ? launch_tree<3, true>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate)
-                      : launch_tree<3, false>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate);
+            ls = same ? launch_tree<3, true>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate, mail)
+                      : launch_tree<3, false>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate, mail);
             break;
         default:
-            ls = same ? launch_tree<4, true>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate)
-                      : launch_tree<4, false>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate);
+            ls = same ? launch_tree<4, true>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate, mail)
+                      : launch_tree<4, false>(aligned, fblocks, s, n, x, y, rho, maxS, sum_mode, sc, gate, mail);
             break;
     }
     if (ls) return ls;
@@ -386,26 +389,34 @@ int dot_fused(cuozblasHandle_t *h, int n, const double *x, const double *y, doub
               int *nB) {
     State *st = state(h);
     *done = false;
-    Arena ar(h);
-    const uint64_t mk = ar.mark();
-    DotScratch *sc = ar.take<DotScratch>(1);
-    if (!ar.ok) return CUOZBLAS_STATUS_WORKSPACE;
+    {  // the smallest workspace a DOT is accepted with
+        Arena ar(h);
+        const uint64_t mk = ar.mark();
+        ar.take<DotScratch>(1);
+        if (!ar.ok) return CUOZBLAS_STATUS_WORKSPACE;
+        ar.release(mk);
+    }
+    // the handle's persistent scratch, left zeroed by every kernel that uses it
+    DotScratch *sc = reinterpret_cast<DotScratch *>(st->d_persist);
+    DotStatus *mail = reinterpret_cast<DotStatus *>(st->d_mail);
     const int maxS = h->nSplitMax > 0 ? h->nSplitMax : kMaxSplitDefault;
     const int rho = rho_rule(n, h->splitEpsMode);
-    OZB_CHECK(cudaMemsetAsync(sc, 0, sizeof(DotScratch), st->stream));
     const int nsm = sm_count();
+    DotStatus res{};
+    memcpy(st->h_mail, &res, sizeof(res));
     span_begin(h);
     counted(h);
-    OZB_TRY(dot_scan_launch(st->stream, nsm, n, x, y, sc));
+    int launched = dot_scan_launch(st->stream, nsm, n, x, y, sc);
     counted(h);
-    OZB_TRY(dot_tree_launch(st->stream, nsm, n, x, y, rho, maxS, h->sumMode, sc, nullptr, st->env.dot_tree));
+    if (!launched)
+        launched = dot_tree_launch(st->stream, nsm, n, x, y, rho, maxS, h->sumMode, sc, nullptr, st->env.dot_tree, mail);
+    if (launched) {
+        cudaMemsetAsync(sc, 0, sizeof(DotScratch), st->stream);
+        return launched;
+    }
     span_end(h);
-    static_assert(sizeof(DotStatus) == 24, "status block layout");
-    OZB_CHECK(cudaMemcpyAsync(st->h_dbl, &sc->out, sizeof(DotStatus), cudaMemcpyDeviceToHost, st->stream));
     OZB_CHECK(cudaStreamSynchronize(st->stream));
-    ar.release(mk);
-    DotStatus res;
-    memcpy(&res, st->h_dbl, sizeof(res));
+    memcpy(&res, st->h_mail, sizeof(res));
     if (res.status != 1 && state(h)->env.dot_trace)
         fprintf(stderr, "cuozblas: dot fused not used (n=%d, reason bits %d)\n", n, res.pad);
     if (res.status == 1) {

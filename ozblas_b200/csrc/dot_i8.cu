@@ -222,7 +222,7 @@ __device__ void di_finish(DotScratch *sc, const TreePlan &pl, bool same, int sum
 template <bool SAME, int D, int RP, int G>
 __global__ void __launch_bounds__(kDiThreads, 1)
     k_dot_i8(int n, const double *__restrict__ x, const double *__restrict__ y, int rho, int maxS, int sum_mode,
-             DotScratch *__restrict__ sc, const int *__restrict__ gate) {
+             DotScratch *__restrict__ sc, const int *__restrict__ gate, DotStatus *mail) {
     constexpr int CH = 128 / RP;   // chunks per job
     constexpr int JOB = 128 * CH;  // elements per job
     constexpr int E = CH;          // elements per producer thread (128 threads per job)
@@ -410,6 +410,7 @@ __global__ void __launch_bounds__(kDiThreads, 1)
     if (!last) return;
     __threadfence();
     di_finish(sc, pl, SAME, sum_mode, D, fin[0], fin[1]);
+    if (t == 0 && mail) dot_post(sc, mail);
     __syncthreads();
     // leave the accumulators zeroed for the next use (replayed graphs skip the memset)
     for (int i = t; i < kDotDigitRows * kDotDigitRows; i += kDiThreads) sc->T[i] = 0;
@@ -431,12 +432,12 @@ int dot_i8_digits(int rho) {
 
 template <bool SAME, int D, int G>
 static int launch_i8(int grid, cudaStream_t s, int n, const double *x, const double *y, int rho, int maxS,
-                     int sum_mode, DotScratch *sc, const int *gate) {
+                     int sum_mode, DotScratch *sc, const int *gate, DotStatus *mail) {
     constexpr int RP = D == 2 ? 16 : 32;
     static std::atomic<uint64_t> attr{0};  // devices already opted in, per instantiation
     if (smem_optin((const void *)k_dot_i8<SAME, D, RP, G>, kDiSmem, attr) != cudaSuccess)
         return CUOZBLAS_STATUS_CUDA_ERROR;
-    k_dot_i8<SAME, D, RP, G><<<grid, kDiThreads, kDiSmem, s>>>(n, x, y, rho, maxS, sum_mode, sc, gate);
+    k_dot_i8<SAME, D, RP, G><<<grid, kDiThreads, kDiSmem, s>>>(n, x, y, rho, maxS, sum_mode, sc, gate, mail);
     return cudaGetLastError() == cudaSuccess ? CUOZBLAS_STATUS_SUCCESS : CUOZBLAS_STATUS_CUDA_ERROR;
 }
 
@@ -456,16 +457,16 @@ int dot_i8_prepare() {
 
 template <bool SAME>
 static int launch_i8_g(int D, int G, int grid, cudaStream_t s, int n, const double *x, const double *y, int rho,
-                       int maxS, int sum_mode, DotScratch *sc, const int *gate) {
-    if (D == 2 && G == 3) return launch_i8<SAME, 2, 3>(grid, s, n, x, y, rho, maxS, sum_mode, sc, gate);
-    if (D == 2 && G == 4) return launch_i8<SAME, 2, 4>(grid, s, n, x, y, rho, maxS, sum_mode, sc, gate);
-    if (D == 3 && G == 2) return launch_i8<SAME, 3, 2>(grid, s, n, x, y, rho, maxS, sum_mode, sc, gate);
-    if (D == 3 && G == 3) return launch_i8<SAME, 3, 3>(grid, s, n, x, y, rho, maxS, sum_mode, sc, gate);
+                       int maxS, int sum_mode, DotScratch *sc, const int *gate, DotStatus *mail) {
+    if (D == 2 && G == 3) return launch_i8<SAME, 2, 3>(grid, s, n, x, y, rho, maxS, sum_mode, sc, gate, mail);
+    if (D == 2 && G == 4) return launch_i8<SAME, 2, 4>(grid, s, n, x, y, rho, maxS, sum_mode, sc, gate, mail);
+    if (D == 3 && G == 2) return launch_i8<SAME, 3, 2>(grid, s, n, x, y, rho, maxS, sum_mode, sc, gate, mail);
+    if (D == 3 && G == 3) return launch_i8<SAME, 3, 3>(grid, s, n, x, y, rho, maxS, sum_mode, sc, gate, mail);
     return CUOZBLAS_STATUS_INVALID_VALUE;
 }
 
 int dot_i8_launch(cudaStream_t s, int nsm, int n, const double *x, const double *y, int rho, int maxS,
-                  int sum_mode, DotScratch *sc, const int *gate) {
+                  int sum_mode, DotScratch *sc, const int *gate, DotStatus *mail) {
     const int D = dot_i8_digits(rho);
     const int G = chain_group(rho, 4);  // levels cut from one base value, as the tree pass
     const int job = D == 2 ? 1024 : 512;
@@ -474,8 +475,8 @@ int dot_i8_launch(cudaStream_t s, int nsm, int n, const double *x, const double 
     const int64_t need = (njobs + kDiMaxJobs - 1) / kDiMaxJobs;
     if (grid < need) grid = need;
     if (grid < 1) grid = 1;
-    return x == y ? launch_i8_g<true>(D, G, (int)grid, s, n, x, y, rho, maxS, sum_mode, sc, gate)
-                  : launch_i8_g<false>(D, G, (int)grid, s, n, x, y, rho, maxS, sum_mode, sc, gate);
+    return x == y ? launch_i8_g<true>(D, G, (int)grid, s, n, x, y, rho, maxS, sum_mode, sc, gate, mail)
+                  : launch_i8_g<false>(D, G, (int)grid, s, n, x, y, rho, maxS, sum_mode, sc, gate, mail);
 }
 
 }  // namespace ozb

@@ -202,8 +202,15 @@ int dot_small(cuozblasHandle_t *h, int n, const double *x, const double *y, doub
               int *nB) {
     State *st = state(h);
     *done = false;
-    if (n < 1 || n > kDotSmallMax || st->h_mail == nullptr || st->env.dot_tree || st->env.dot_two_pass)
+    if (n < 1 || n > kDotSmallMax || st->env.dot_tree || st->env.dot_two_pass)
         return CUOZBLAS_STATUS_SUCCESS;
+    if (h->sumMode == 0) {  // the smallest workspace an FSum DOT is accepted with (dot_fused.cu)
+        Arena ar(h);
+        const uint64_t mk = ar.mark();
+        ar.take<DotScratch>(1);
+        if (!ar.ok) return CUOZBLAS_STATUS_WORKSPACE;
+        ar.release(mk);
+    }
     const int maxS = h->nSplitMax > 0 ? h->nSplitMax : kMaxSplitDefault;
     const int rho = rho_rule(n, h->splitEpsMode);
     DotStatus res{};
