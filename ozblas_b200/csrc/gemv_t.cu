@@ -57,7 +57,9 @@ __device__ __forceinline__ uint64_t mag_bits(double v) {  // |v| in order; 0 for
 }
 
 // The block's largest |v| over C values per thread (NaN skipped): by high
-// words, the low words only where the rule for tau or a zero depends on them.
+// words, the low words only where the rule for tau or a zero depends on them:
+// in normal numbers just above a power of two, in subnormal ones (whose leading
+// bit may be any bit of the high word) always.
 template <int C>
 __device__ __forceinline__ double block_max_abs(const double (&v)[C], unsigned *red) {  // red: 2 x 32, used in turn
     unsigned hm = 0;
@@ -72,7 +74,7 @@ __device__ __forceinline__ double block_max_abs(const double (&v)[C], unsigned *
     __syncthreads();
     hm = __reduce_max_sync(0xffffffffu, l < nw ? red[l] : 0u);
     unsigned lm = 1;
-    if ((hm & 0xfffffu) == 0) {  // uniform: at a power of two, or subnormal, or zero
+    if ((hm & 0xfffffu) == 0 || hm < 0x100000u) {  // uniform: at a power of two, or subnormal, or zero
         lm = 0;
 #pragma unroll
         for (int c = 0; c < C; c++)
