@@ -96,7 +96,7 @@ typedef enum {
     CUOZBLAS_STATUS_WORKSPACE = 3,      /* the arena given at create is too small */
     CUOZBLAS_STATUS_NOT_SUPPORTED = 4,  /* e.g. Dot2 for GEMM/GEMV, NearSum in the mixed and quad forms */
     CUOZBLAS_STATUS_INT32_BOUND = 5,    /* INT8 form: k beyond the exact INT32 bound */
-    CUOZBLAS_STATUS_DEVICE_TIMEOUT = 6, /* a bounded device-side wait gave up */
+    CUOZBLAS_STATUS_DEVICE_TIMEOUT = 6, /* a bounded device-side wait gave up; the output may be partly written */
     CUOZBLAS_STATUS_CUDA_ERROR = 7
 } cuozblasStatus_t;
 
@@ -279,7 +279,9 @@ int cuozblasDgemmI8Static(char transa, char transb, int32_t m, int32_t n, int32_
  * default 2 s) and, with hold_copies != 0, a producer that issues no copies,
  * so that the tensor-core issuer's wait runs out and cuozblasDgemmI8 returns
  * CUOZBLAS_STATUS_DEVICE_TIMEOUT; the kernel releases its tensor memory
- * first and the context stays usable.  Call (0, 0) to restore. */
+ * first and the context stays usable.  The product kernel of the plain, the
+ * <float,double,double> and the quad GEMM obeys it too.  Call (0, 0) to
+ * restore. */
 int cuozblasSetI8WaitTest(uint64_t ns, int32_t hold_copies);
 
 /* Rule checks exported for the host-side tests (same code the kernels use). */

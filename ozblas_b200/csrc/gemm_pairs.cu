@@ -1088,7 +1088,9 @@ int pair_status(cuozblasHandle_t *h) {
 // fifteen instructions (with the list found per term and both forms of it
 // inlined a term took 74, and the code did not fit the instruction cache).
 // Entries of pairs that the product kernel skipped hold anything: the lines'
-// marks at those levels make them zeros.
+// marks at those levels make them zeros.  *err: a wait of the product kernel ran
+// out, so the buffer is not complete and C stays as it is (the word is read
+// first and tested last, behind the loads of the pairs).
 constexpr int kPsRows = 256, kPsCols = 2, kPsIn = 16;
 constexpr int kPsLevels = 12, kPsPairs = 144;  // held in shared memory; k_pair_sum_any beyond
 
@@ -1112,7 +1114,8 @@ template <bool FLOATS>
 __global__ void __launch_bounds__(kPsRows, 4)
     k_pair_sum(int m, int n, int col0, int cn, int nA, int nB, int np, const double *__restrict__ pbuf,
                const short *__restrict__ ea, const short *__restrict__ eb, int bias, double alpha, double beta,
-               void *__restrict__ Cv, int ldc) {
+               void *__restrict__ Cv, int ldc, const int *__restrict__ err) {
+    const int failed = *err;
     __shared__ short sA[kPsLevels][kPsRows];
     __shared__ int2 sP[kPsCols][kPsPairs];  // A level, B level's tau
     const int rb = (m + kPsRows - 1) / kPsRows, tr = threadIdx.x;
@@ -1160,7 +1163,7 @@ __global__ void __launch_bounds__(kPsRows, 4)
                 }
             }
         }
-        pair_out<FLOATS>(Cv, (size_t)(c0 + c) * ldc + row, alpha, beta, t, tf);
+        if (failed == 0) pair_out<FLOATS>(Cv, (size_t)(c0 + c) * ldc + row, alpha, beta, t, tf);
     }
 }
 
@@ -1169,7 +1172,8 @@ template <bool FLOATS>
 __global__ void __launch_bounds__(256)
     k_pair_sum_any(int m, int n, int col0, int cn, int nA, int nB, int maxlevel, int np, double *__restrict__ pbuf,
                    const short *__restrict__ ea, const short *__restrict__ eb, int bias, int sum_mode, double alpha,
-                   double beta, void *__restrict__ Cv, int ldc) {
+                   double beta, void *__restrict__ Cv, int ldc, const int *__restrict__ err) {
+    const int failed = *err;
     const int rb = (m + 255) / 256;
     const int row = (int)(blockIdx.x % rb) * 256 + threadIdx.x, col = col0 + (int)(blockIdx.x / rb);
     if (row >= m) return;
@@ -1190,7 +1194,7 @@ __global__ void __launch_bounds__(256)
             t = __dadd_rn(t, term);
     });
     if (!FLOATS && sum_mode == 1) t = nearsum(np, pe, (int64_t)count);
-    pair_out<FLOATS>(Cv, (size_t)col * ldc + row, alpha, beta, t, tf);
+    if (failed == 0) pair_out<FLOATS>(Cv, (size_t)col * ldc + row, alpha, beta, t, tf);
 }
 
 // C = alpha op(A) op(B) + beta C with m, n > 1 in the plain form (T = double)
@@ -1334,11 +1338,12 @@ int gemm_pairs_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
             if (!near && c.nA <= kPsLevels && npu <= kPsPairs)
                 k_pair_sum<kFloats><<<(unsigned)((int64_t)((m + kPsRows - 1) / kPsRows) * ((c.cn + kPsCols - 1) / kPsCols)),
                                       kPsRows, 0, st->stream>>>(m, n, c0, c.cn, c.nA, c.nB, npu, c.pbuf, op[0].exps,
-                                                                op[1].exps, c.bias, alpha, beta, C, ldc);
+                                                                op[1].exps, c.bias, alpha, beta, C, ldc,
+                                                                st->d_ints + kPairErrInt);
             else
                 k_pair_sum_any<kFloats><<<(unsigned)((int64_t)((m + 255) / 256) * c.cn), 256, 0, st->stream>>>(
                     m, n, c0, c.cn, c.nA, c.nB, c.maxlevel, npu, c.pbuf, op[0].exps, op[1].exps, c.bias, h->sumMode,
-                    alpha, beta, C, ldc);
+                    alpha, beta, C, ldc, st->d_ints + kPairErrInt);
             OZB_CHECK(cudaGetLastError());
         }
     } else {

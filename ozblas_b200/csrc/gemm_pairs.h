@@ -56,7 +56,9 @@ int pair_split(cuozblasHandle_t *h, int k, int k_pad, const T *X, int ldx, int r
                int tile_lines, const PairOperand &op, int *zmax_dev);
 
 // The products of every pair (ia, ib), ia + ib <= maxlevel, ia < nA, ib < nB.
-// A bounded wait that runs out is reported by pair_status.
+// A bounded wait that runs out sets the handle's error word (kPairErrInt): a sum
+// over the pair buffer must leave C alone then (kPairFsum and kPairSd have stored
+// the tiles that were complete), and pair_status reports it.
 struct PairCall {
     int m, n, k_pad, nA, nB, maxlevel;
     int bias = 0;  // a pair product is 2^(bias + tauA + tauB) sum q q (kPairStore: for the sum that reads pbuf)

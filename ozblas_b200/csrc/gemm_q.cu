@@ -150,13 +150,15 @@ __global__ void __launch_bounds__(256) k_split_lines_q_digits(int k, int nl, con
 
 // General GEMM sum: element e = col * m + row of a block of nc columns from
 // c0; pbuf[p * count + e] exact FP64 products of pair dp[p].
-// INT: the entries are 64-bit integers V below 2^53, the product V 2^vbias.
+// INT: the entries are 64-bit integers V below 2^53, the product V 2^vbias, and C
+// stays as it is when *err says that they are not complete.
 template <bool INT>
 __global__ void k_sum_pairs_q(int m, int n, int64_t count, int c0, int np, const double *__restrict__ pbuf, int vbias,
                               const int2 *__restrict__ dp, const short *__restrict__ Ea,
-                              const short *__restrict__ Eb, Q128 alpha, Q128 beta, Q128 *__restrict__ C, int ldc) {
+                              const short *__restrict__ Eb, Q128 alpha, Q128 beta, Q128 *__restrict__ C, int ldc,
+                              const int *__restrict__ err) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= count) return;
+    if (e >= count || (INT && *err != 0)) return;
     const int row = (int)(e % m), col = c0 + (int)(e / m);
     Q128 t = q_zero(0);
     for (int p = 0; p < np; p++) {
@@ -331,7 +333,8 @@ int gemm_q_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, cons
             const int64_t count = (int64_t)m * n;
             counted(h);
             k_sum_pairs_q<true><<<(unsigned)((count + 255) / 256), 256, 0, st->stream>>>(m, n, count, 0, np, pbuf, pc.bias, dp, Ea,
-                                                                                  Eb, alpha, beta, C, ldc);
+                                                                                  Eb, alpha, beta, C, ldc,
+                                                                                  st->d_ints + kPairErrInt);
             OZB_CHECK(cudaGetLastError());
             ev_record(h, 3);
             ev_record(h, 4);
@@ -369,7 +372,7 @@ int gemm_q_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, cons
         const int64_t count = (int64_t)m * nc;
         counted(h);
         k_sum_pairs_q<false><<<(unsigned)((count + 255) / 256), 256, 0, st->stream>>>(m, n, count, (int)c0, np, pbuf, 0, dp, Ea,
-                                                                              Eb, alpha, beta, C, ldc);
+                                                                              Eb, alpha, beta, C, ldc, nullptr);
         OZB_CHECK(cudaGetLastError());
     }
     ev_record(h, 3);  // products and sum interleave per column block here
