@@ -1308,12 +1308,13 @@ int gemm_pairs_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
     c.epi = kFloats ? kPairSd : kPairFsum;
     const PairStorePlan sp = pair_store_plan(m, n, k_pad, npu, pd.D);
     if (near || sp.us < pair_fused_us(m, n, k_pad, npu, pd.D)) {
-        // in column blocks: as many as the plan asks for, or as the arena does
+        // in column blocks: as many as the plan asks for, or as the arena does.  A block is whole tiles:
+        // the plan's rounded up, or what the arena holds rounded down.
         const uint64_t avail = h->workSizeBytes - ((ar.mark() + 255) / 256 * 256);
         int64_t cols = (n + sp.blocks - 1) / sp.blocks;
         const int64_t most = (int64_t)(avail / (sizeof(double) * (uint64_t)npu * (uint64_t)m));
-        if (cols > most) cols = most;
-        if (cols < n) cols = (cols + (sp.blocks > 1 && cols < most ? tile[1] - 1 : 0)) / tile[1] * tile[1];
+        if (cols < n) cols = (cols + tile[1] - 1) / tile[1] * tile[1];
+        if (cols > most) cols = most / tile[1] * tile[1];
         if (cols > 0) {
             c.cn = (int)cols;
             c.pbuf = ar.take<double>((uint64_t)npu * m * cols);
