@@ -664,10 +664,11 @@ int cuozblasDcsrmv(cuozblasHandle_t *h, char trans, int32_t m, int32_t n, int32_
     Arena ar(h);
     const int64_t ld = splitA_ld(nnz);
     int nA = 0;
-    OZB_TRY(split_csr_count(h, m, val, rowptr, h->splitEpsMode, 1, maxS, &nA));
+    CsrSplitRows rows;
+    OZB_TRY(split_csr_count(h, m, val, rowptr, h->splitEpsMode, 1, maxS, &nA, &rows));
     double *As = ar.take<double>((uint64_t)nA * ld);
     if (!ar.ok) return CUOZBLAS_STATUS_WORKSPACE;
-    OZB_TRY(split_csr_write(h, m, nnz, val, rowptr, h->splitEpsMode, 1, nA, As, ld));
+    OZB_TRY(split_csr_write(h, m, nnz, val, rowptr, h->splitEpsMode, 1, nA, As, ld, rows));
     OZB_TRY(csrmv_presplit(h, m, n, alpha, As, nA, ld, colind, rowptr, x, beta, y));
     return finish(h, t0);
 }
@@ -683,17 +684,18 @@ int cuozblasDcsrmvSplitA(cuozblasHandle_t *h, char trans, int32_t m, int32_t n, 
     const double t0 = wall();
     // tuning of splitShift (src/cuda/cuozblas_csrmv.cu:186-201), counts only
     int s = 0;
-    OZB_TRY(split_csr_count(h, m, val, rowptr, h->splitEpsMode, 1, maxS, &s));
+    CsrSplitRows rows;
+    OZB_TRY(split_csr_count(h, m, val, rowptr, h->splitEpsMode, 1, maxS, &s, &rows));
     int shift = 1;
     if (h->nSplitMax == 0) {
         int sold;
         do {
             sold = s;
             shift *= 2;
-            OZB_TRY(split_csr_count(h, m, val, rowptr, h->splitEpsMode, shift, maxS, &s));
+            OZB_TRY(split_csr_count(h, m, val, rowptr, h->splitEpsMode, shift, maxS, &s, &rows));
         } while (sold == s && shift < 512);
         if (sold == s) shift = 1;
-        OZB_TRY(split_csr_count(h, m, val, rowptr, h->splitEpsMode, shift, maxS, &s));
+        OZB_TRY(split_csr_count(h, m, val, rowptr, h->splitEpsMode, shift, maxS, &s, &rows));
     }
     // the preserved region starts at the arena base
     State *st = state(h);
@@ -702,7 +704,7 @@ int cuozblasDcsrmvSplitA(cuozblasHandle_t *h, char trans, int32_t m, int32_t n, 
     const int64_t ld = splitA_ld(nnz);
     double *As = ar.take<double>((uint64_t)s * ld);
     if (!ar.ok) return CUOZBLAS_STATUS_WORKSPACE;
-    OZB_TRY(split_csr_write(h, m, nnz, val, rowptr, h->splitEpsMode, shift, s, As, ld));
+    OZB_TRY(split_csr_write(h, m, nnz, val, rowptr, h->splitEpsMode, shift, s, As, ld, rows));
     h->memMaskSplitA = st->off;
     h->splitShift = shift;
     h->nSplitA_ = s;

@@ -235,11 +235,16 @@ int transpose(cuozblasHandle_t *h, int rows, int cols, const double *A, int lda,
 constexpr int kSplitVectorSmallMax = 16384;
 int split_vector_small(cuozblasHandle_t *h, int n, const double *x, int rho, int maxS, double *out, int ldo, int *ns);
 int split_vector(cuozblasHandle_t *h, int n, const double *x, int rho, int maxS, double *out, int ldo, int *ns);
-// CSR row split; slices laid out ns x nnz.  shift divides sigma.
+// CSR row split; slices laid out ns x nnz.  shift divides sigma.  The count
+// says how the write takes the rows.
+struct CsrSplitRows {
+    int lanes = 0;       // per row (0: from the write's nnz)
+    bool longer = true;  // some row is too long for them
+};
 int split_csr_count(cuozblasHandle_t *h, int m, const double *val, const int *rowptr, int epsmode, int shift,
-                    int maxS, int *ns);
+                    int maxS, int *ns, CsrSplitRows *rows);
 int split_csr_write(cuozblasHandle_t *h, int m, int nnz, const double *val, const int *rowptr, int epsmode,
-                    int shift, int ns, double *out, int64_t ld);
+                    int shift, int ns, double *out, int64_t ld, const CsrSplitRows &rows);
 
 // Copy n elements of esz (4, 8 or 16) bytes, `stride` elements apart, to a
 // contiguous array (csrmv.cu).

@@ -402,51 +402,100 @@ int split_vector_f32(cuozblasHandle_t *h, int n, const double *x, int rho, int m
 // z in *zmax, the write pass writes `levels` slices of nnz.
 //
 // W lanes hold a row and kCsrHeld entries each in registers, W so that this
-// covers twice the mean row length (a longer row keeps its remainders in
-// `rem`, nnz doubles): the level's sigma is computed by every lane of a row,
-// so wider rows only repeat it.  The counts are folded per block: one atomic
-// per row on the one counter was the bound (10^6 rows of 7 with it and a warp
-// per row: 675 us, of which the 56 MB of values account for 9; 8 lanes per
+// covers twice the mean row length: the level's sigma is computed by every lane
+// of a row, so wider rows only repeat it.  The counts are folded per block: one
+// atomic per row on the one counter was the bound (10^6 rows of 7 with it and a
+// warp per row: 675 us, of which the 56 MB of values account for 9; 8 lanes per
 // row 94, 4 lanes 55; the writing pass 385 -> 63).
+//
+// Longer rows keep their remainders in `rem` (nnz doubles).  Its own lanes walk a
+// row of up to kCsrWalk entries each.  Beyond that a row stands out (at most one
+// in 8 does): the block lists those and its warps share them at the end, up to
+// csr_block_row entries.  The rest is left to k_split_csr_long, which the count
+// pass asks for when it meets one: a launch and a host wait more, 25 us a pass.
+// 10^6 rows of 3 with 1000 of 600, cuozblasDcsrmvSplitA: 0.45 ms (1.2 in their two
+// lanes, 1.5 in k_split_csr_long, 4.0 with a warp for every row).
 // ---------------------------------------------------------------------------
-constexpr int kCsrHeld = 4;  // entries of a row per lane in registers
+constexpr int kCsrHeld = 4;   // entries of a row per lane in registers
+constexpr int kCsrWalk = 16;  // entries per lane that the row's own lanes walk (W < 32)
+constexpr int kCsrList = 512;
+__host__ __device__ constexpr int csr_block_row(int lanes) { return lanes < 32 ? 1024 : 8192; }
+
+// The split of the row of n entries from lo by W lanes of a warp (`mask`; this
+// one is `sub`), the remainders in memory, the loads of four steps in flight.
+// Returns the first level that leaves nothing.
+template <bool WRITE, int W>
+__device__ __forceinline__ int split_row_rem(int lo, int n, int sub, unsigned mask, const double *__restrict__ val,
+                                             int epsmode, int shift, int levels, double *__restrict__ rem,
+                                             double *__restrict__ out, int64_t ldo) {
+    constexpr int U = 4;
+    val += lo;
+    rem += lo;
+    if (WRITE) out += lo;
+    double mx = 0.0;
+    for (int i = sub; i < n; i += W) mx = ref_max(mx, fabs(val[i]));
+    for (int o = W / 2; o > 0; o >>= 1) mx = ref_max(mx, __shfl_xor_sync(mask, mx, o));
+    const int rho = rho_rule(n, epsmode);
+    for (int s = 0; s < levels; s++) {
+        const double sigma = shift_sigma(0.75 * pow2(rho + tau_rule(mx)), shift);
+        const double *from = s == 0 ? val : rem;
+        double nm = 0.0;
+        for (int i0 = sub; i0 < n; i0 += U * W) {
+            double v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) v[u] = i0 + u * W < n ? from[i0 + u * W] : 0.0;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int i = i0 + u * W;
+                if (i < n) {
+                    const double sl = (v[u] + sigma) - sigma;
+                    const double r = v[u] - sl;
+                    rem[i] = r;
+                    nm = ref_max(nm, fabs(r));
+                    if (WRITE) out[(size_t)s * ldo + i] = sl;
+                }
+            }
+        }
+        for (int o = W / 2; o > 0; o >>= 1) nm = ref_max(nm, __shfl_xor_sync(mask, nm, o));
+        mx = nm;
+        if (!WRITE && mx == 0.0) return s;
+    }
+    return levels;
+}
 
 template <bool WRITE, int W>
 __global__ void __launch_bounds__(256) k_split_csr(int m, const double *__restrict__ val,
                                                    const int *__restrict__ rowptr, int epsmode, int shift,
                                                    int levels, double *__restrict__ rem, double *__restrict__ out,
-                                                   int64_t ldo, int *__restrict__ zmax) {
-    __shared__ int zsh[8];
+                                                   int64_t ldo, int *__restrict__ zmax, int *__restrict__ longer) {
+    __shared__ int zsh[8], list[kCsrList], nlist;
     const int lane = threadIdx.x & 31, sub = lane % W;
     const unsigned rows_lanes = W == 32 ? 0xffffffffu : ((1u << W) - 1u) << (lane - sub);  // this row's lanes
     const int64_t nrows = (int64_t)gridDim.x * (256 / W);
     int zbest = 0;
-    for (int64_t row = (int64_t)blockIdx.x * (256 / W) + threadIdx.x / W; row < m; row += nrows) {
-        const int lo = rowptr[row], hi = rowptr[row + 1];
-        if (hi <= lo) continue;  // z = 0
-        const bool held = hi - lo <= kCsrHeld * W;  // uniform over the row's lanes
-        double r[kCsrHeld], mx = 0.0;
-        if (held) {
+    if (W < 32) {
+        if (threadIdx.x == 0) nlist = 0;
+        __syncthreads();
+    }
+    // base: the warp's first row
+    for (int64_t base = ((int64_t)blockIdx.x * 256 + (threadIdx.x & ~31)) / W; base < m; base += nrows) {
+        const int64_t row = base + lane / W;
+        const int lo = row < m ? rowptr[row] : 0, hi = row < m ? rowptr[row + 1] : 0;
+        const int len = hi - lo;  // uniform over the row's lanes; an empty row has z = 0
+        if (len > 0 && len <= kCsrHeld * W) {
+            double r[kCsrHeld], mx = 0.0;
 #pragma unroll
             for (int e = 0; e < kCsrHeld; e++) {
                 const int i = lo + e * W + sub;
                 r[e] = i < hi ? val[i] : 0.0;
                 mx = ref_max(mx, fabs(r[e]));
             }
-        } else {
-            for (int i = lo + sub; i < hi; i += W) {
-                const double v = val[i];
-                rem[i] = v;
-                mx = ref_max(mx, fabs(v));
-            }
-        }
-        for (int o = W / 2; o > 0; o >>= 1) mx = ref_max(mx, __shfl_xor_sync(rows_lanes, mx, o));
-        int z = levels;
-        const int rho = rho_rule(hi - lo, epsmode);
-        for (int s = 0; s < levels; s++) {
-            const double sigma = shift_sigma(0.75 * pow2(rho + tau_rule(mx)), shift);
-            double nm = 0.0;
-            if (held) {
+            for (int o = W / 2; o > 0; o >>= 1) mx = ref_max(mx, __shfl_xor_sync(rows_lanes, mx, o));
+            int z = levels;
+            const int rho = rho_rule(len, epsmode);
+            for (int s = 0; s < levels; s++) {
+                const double sigma = shift_sigma(0.75 * pow2(rho + tau_rule(mx)), shift);
+                double nm = 0.0;
 #pragma unroll
                 for (int e = 0; e < kCsrHeld; e++) {
                     const int i = lo + e * W + sub;
@@ -457,24 +506,38 @@ __global__ void __launch_bounds__(256) k_split_csr(int m, const double *__restri
                         if (WRITE) out[(size_t)s * ldo + i] = sl;
                     }
                 }
-            } else {
-                for (int i = lo + sub; i < hi; i += W) {
-                    double v = rem[i];
-                    const double sl = (v + sigma) - sigma;
-                    v = v - sl;
-                    rem[i] = v;
-                    nm = ref_max(nm, fabs(v));
-                    if (WRITE) out[(size_t)s * ldo + i] = sl;
+                for (int o = W / 2; o > 0; o >>= 1) nm = ref_max(nm, __shfl_xor_sync(rows_lanes, nm, o));
+                mx = nm;
+                if (!WRITE && mx == 0.0) {
+                    z = s;
+                    break;
                 }
             }
-            for (int o = W / 2; o > 0; o >>= 1) nm = ref_max(nm, __shfl_xor_sync(rows_lanes, nm, o));
-            mx = nm;
-            if (!WRITE && mx == 0.0) {
-                z = s;
-                break;
+            zbest = z > zbest ? z : zbest;
+        } else if (len > csr_block_row(W)) {
+            if (!WRITE && sub == 0) *longer = 1;
+        } else if (len > 0) {
+            bool own = W == 32 || len <= kCsrWalk * W;
+            if (!own) {
+                int at = sub == 0 ? atomicAdd(&nlist, 1) : 0;
+                at = __shfl_sync(rows_lanes, at, lane - sub);
+                own = at >= kCsrList;  // no room
+                if (!own && sub == 0) list[at] = (int)row;
+            }
+            if (own) {
+                const int z = split_row_rem<WRITE, W>(lo, len, sub, rows_lanes, val, epsmode, shift, levels, rem, out, ldo);
+                zbest = z > zbest ? z : zbest;
             }
         }
-        zbest = z > zbest ? z : zbest;
+    }
+    if (W < 32) {
+        __syncthreads();
+        const int n = nlist < kCsrList ? nlist : kCsrList;
+        for (int k = threadIdx.x >> 5; k < n; k += 8) {
+            const int lo = rowptr[list[k]], len = rowptr[list[k] + 1] - lo;
+            const int z = split_row_rem<WRITE, 32>(lo, len, lane, 0xffffffffu, val, epsmode, shift, levels, rem, out, ldo);
+            zbest = z > zbest ? z : zbest;
+        }
     }
     if (!WRITE) {
         const int zw = __reduce_max_sync(0xffffffffu, zbest);
@@ -488,36 +551,110 @@ __global__ void __launch_bounds__(256) k_split_csr(int m, const double *__restri
     }
 }
 
+// The rows of more than `over` entries, a block per row.  Row r belongs to block
+// r % gridDim.x, so long rows that stand together are spread over the chip; a
+// block finds its own 1024 at a time.  cuozblasDcsrmvSplitA (a count per shift and
+// the write) of 10^6 rows of 3 with one of 10^5: 1.65 ms (in a row's own two lanes
+// 347, with a warp for every row 13.7); with 1000 of 5000 side by side 1.6 (15.8,
+// 6.5); without such rows 0.75 (8.2).
+constexpr int kCsrLongThreads = 1024;
+
 template <bool WRITE>
-static int split_csr_launch(cuozblasHandle_t *h, int m, int nnz, const double *val, const int *rowptr, int epsmode,
-                            int shift, int levels, double *rem, double *out, int64_t ldo, int *zmax) {
+__global__ void __launch_bounds__(kCsrLongThreads) k_split_csr_long(int m, int over, const double *__restrict__ val,
+                                                                    const int *__restrict__ rowptr, int epsmode,
+                                                                    int shift, int levels, double *__restrict__ rem,
+                                                                    double *__restrict__ out, int64_t ldo,
+                                                                    int *__restrict__ zmax) {
+    __shared__ int list[kCsrLongThreads], nlist;
+    __shared__ double red[kCsrLongThreads / 32];
+    const int t = threadIdx.x;
+    int zbest = 0;
+    for (int64_t r0 = blockIdx.x; r0 < m; r0 += (int64_t)gridDim.x * kCsrLongThreads) {
+        __syncthreads();
+        if (t == 0) nlist = 0;
+        __syncthreads();
+        const int64_t row = r0 + (int64_t)gridDim.x * t;
+        if (row < m && rowptr[row + 1] - rowptr[row] > over) list[atomicAdd(&nlist, 1)] = (int)row;
+        __syncthreads();
+        for (int k = 0; k < nlist; k++) {
+            const int lo = rowptr[list[k]];
+            const int64_t n = rowptr[list[k] + 1] - lo;
+            double *r = rem + lo;
+            double mx = 0.0;
+            for (int64_t i = t; i < n; i += kCsrLongThreads) mx = ref_max(mx, fabs(val[lo + i]));
+            mx = block_max_nonneg(mx, red);
+            int z = levels;
+            const int rho = rho_rule((int)n, epsmode);
+            for (int s = 0; s < levels; s++) {
+                const double sigma = shift_sigma(0.75 * pow2(rho + tau_rule(mx)), shift);
+                const double *from = s == 0 ? val + lo : r;
+                double nm = 0.0;
+                for (int64_t i = t; i < n; i += kCsrLongThreads) {
+                    double v = from[i];
+                    const double sl = (v + sigma) - sigma;
+                    v = v - sl;
+                    r[i] = v;
+                    nm = ref_max(nm, fabs(v));
+                    if (WRITE) out[(size_t)s * ldo + lo + i] = sl;
+                }
+                mx = block_max_nonneg(nm, red);
+                if (!WRITE && mx == 0.0) {  // uniform
+                    z = s;
+                    break;
+                }
+            }
+            zbest = z > zbest ? z : zbest;
+        }
+    }
+    if (!WRITE && t == 0 && zbest > 0) atomicMax(zmax, zbest);
+}
+
+// Lanes per row (see above).
+static int split_csr_lanes(int m, int nnz) {
+    const int64_t mean = m > 0 ? ((int64_t)nnz + m - 1) / m : 0;
+    return mean <= 4 ? 2 : mean <= 8 ? 4 : mean <= 16 ? 8 : mean <= 32 ? 16 : 32;
+}
+
+template <bool WRITE>
+static int split_csr_launch(cuozblasHandle_t *h, int m, int lanes, const double *val, const int *rowptr, int epsmode,
+                            int shift, int levels, double *rem, double *out, int64_t ldo, int *zmax, int *longer) {
     if (m <= 0) return CUOZBLAS_STATUS_SUCCESS;
     cudaStream_t s = state(h)->stream;
-    const int64_t mean = ((int64_t)nnz + m - 1) / m;
     auto go = [&](auto width) {
         constexpr int W = decltype(width)::value;
+        // one resident wave, so that the counts fold; a few waves of one row per warp as they come
         const int64_t need = ((int64_t)m + 256 / W - 1) / (256 / W), cap = (int64_t)sm_count() * 8;
-        k_split_csr<WRITE, W><<<(int)(need < cap ? need : cap), 256, 0, s>>>(m, val, rowptr, epsmode, shift, levels,
-                                                                             rem, out, ldo, zmax);
+        k_split_csr<WRITE, W><<<(int)(need < (W < 32 ? cap : 8 * cap) ? need : cap), 256, 0, s>>>(m, val, rowptr, epsmode, shift, levels,
+                                                                             rem, out, ldo, zmax, longer);
     };
     counted(h);
-    if (mean <= 4)
-        go(std::integral_constant<int, 2>{});
-    else if (mean <= 8)
-        go(std::integral_constant<int, 4>{});
-    else if (mean <= 16)
-        go(std::integral_constant<int, 8>{});
-    else if (mean <= 32)
-        go(std::integral_constant<int, 16>{});
-    else
-        go(std::integral_constant<int, 32>{});
+    switch (lanes) {
+        case 2: go(std::integral_constant<int, 2>{}); break;
+        case 4: go(std::integral_constant<int, 4>{}); break;
+        case 8: go(std::integral_constant<int, 8>{}); break;
+        case 16: go(std::integral_constant<int, 16>{}); break;
+        default: go(std::integral_constant<int, 32>{}); break;
+    }
+    OZB_CHECK(cudaGetLastError());
+    return CUOZBLAS_STATUS_SUCCESS;
+}
+
+template <bool WRITE>
+static int split_csr_long_launch(cuozblasHandle_t *h, int m, int lanes, const double *val, const int *rowptr,
+                                 int epsmode, int shift, int levels, double *rem, double *out, int64_t ldo, int *zmax) {
+    if (m <= 0) return CUOZBLAS_STATUS_SUCCESS;
+    const int cap = sm_count() * 2;
+    counted(h);
+    k_split_csr_long<WRITE><<<m < cap ? m : cap, kCsrLongThreads, 0, state(h)->stream>>>(
+        m, csr_block_row(lanes), val, rowptr, epsmode, shift, levels, rem, out, ldo, zmax);
     OZB_CHECK(cudaGetLastError());
     return CUOZBLAS_STATUS_SUCCESS;
 }
 
 int split_csr_count(cuozblasHandle_t *h, int m, const double *val, const int *rowptr, int epsmode, int shift,
-                    int maxS, int *ns) {
+                    int maxS, int *ns, CsrSplitRows *rows) {
     State *st = state(h);
+    *rows = CsrSplitRows{};  // not looked at
     if (maxS <= 1) {
         *ns = 1;
         return CUOZBLAS_STATUS_SUCCESS;
@@ -526,14 +663,24 @@ int split_csr_count(cuozblasHandle_t *h, int m, const double *val, const int *ro
     OZB_CHECK(cudaMemcpyAsync(st->h_ints, rowptr + m, sizeof(int), cudaMemcpyDeviceToHost, st->stream));
     OZB_CHECK(cudaStreamSynchronize(st->stream));
     nnz = st->h_ints[0];
+    rows->lanes = split_csr_lanes(m, nnz);
     Arena ar(h);
     const uint64_t mk = ar.mark();
     double *rem = ar.take<double>(nnz > 0 ? nnz : 1);
     if (!ar.ok) return CUOZBLAS_STATUS_WORKSPACE;
-    OZB_CHECK(cudaMemsetAsync(st->d_ints, 0, sizeof(int), st->stream));
-    OZB_TRY(split_csr_launch<false>(h, m, nnz, val, rowptr, epsmode, shift, maxS - 1, rem, nullptr, 0, st->d_ints));
-    OZB_CHECK(cudaMemcpyAsync(st->h_ints, st->d_ints, sizeof(int), cudaMemcpyDeviceToHost, st->stream));
+    int *res = st->d_ints;  // the largest z, whether a row was left out as too long
+    OZB_CHECK(cudaMemsetAsync(res, 0, 2 * sizeof(int), st->stream));
+    OZB_TRY(split_csr_launch<false>(h, m, rows->lanes, val, rowptr, epsmode, shift, maxS - 1, rem, nullptr, 0, res,
+                                    res + 1));
+    OZB_CHECK(cudaMemcpyAsync(st->h_ints, res, 2 * sizeof(int), cudaMemcpyDeviceToHost, st->stream));
     OZB_CHECK(cudaStreamSynchronize(st->stream));
+    rows->longer = st->h_ints[1] != 0;
+    if (rows->longer) {
+        OZB_TRY(split_csr_long_launch<false>(h, m, rows->lanes, val, rowptr, epsmode, shift, maxS - 1, rem, nullptr, 0,
+                                             res));
+        OZB_CHECK(cudaMemcpyAsync(st->h_ints, res, sizeof(int), cudaMemcpyDeviceToHost, st->stream));
+        OZB_CHECK(cudaStreamSynchronize(st->stream));
+    }
     const int zmax = st->h_ints[0];
     const int c = (zmax < 1 ? 1 : zmax) + 1;
     *ns = c < maxS ? c : maxS;
@@ -542,12 +689,15 @@ int split_csr_count(cuozblasHandle_t *h, int m, const double *val, const int *ro
 }
 
 int split_csr_write(cuozblasHandle_t *h, int m, int nnz, const double *val, const int *rowptr, int epsmode,
-                    int shift, int ns, double *out, int64_t ld) {
+                    int shift, int ns, double *out, int64_t ld, const CsrSplitRows &rows) {
+    const int lanes = rows.lanes > 0 ? rows.lanes : split_csr_lanes(m, nnz);
     Arena ar(h);
     const uint64_t mk = ar.mark();
     double *rem = ar.take<double>(nnz > 0 ? nnz : 1);
     if (!ar.ok) return CUOZBLAS_STATUS_WORKSPACE;
-    OZB_TRY(split_csr_launch<true>(h, m, nnz, val, rowptr, epsmode, shift, ns, rem, out, ld, nullptr));
+    OZB_TRY(split_csr_launch<true>(h, m, lanes, val, rowptr, epsmode, shift, ns, rem, out, ld, nullptr, nullptr));
+    if (rows.longer)
+        OZB_TRY(split_csr_long_launch<true>(h, m, lanes, val, rowptr, epsmode, shift, ns, rem, out, ld, nullptr));
     ar.release(mk);
     return CUOZBLAS_STATUS_SUCCESS;
 }
