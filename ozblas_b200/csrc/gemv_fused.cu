@@ -33,6 +33,7 @@ constexpr int kGvCols = 64;    // columns per warp per pass
 constexpr int kGvWarps = 8;    // warps per block (same 32 rows, different column chunks)
 constexpr int kGvMaxLevels = 8;
 constexpr int kRowBad = 1 << 20;  // above every kLsbBias - lsb
+enum { kRowProven = 0, kRowOpen = 1, kRowExact = 2 };  // a row's state; kRowExact: left to the exact passes
 
 // Pass p: M[p * m + row] = max |r_p| over the row (r_0 = a), with
 // sigma_l = 0.75 2^(rho + tau(M[l * m + row])) for l < p.  M zeroed before.
@@ -374,8 +375,8 @@ __global__ void __launch_bounds__(256, NB <= 4 ? 2 : 1)
     __shared__ int abort_flag, never;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int row0 = blockIdx.x * 32, row = row0 + lane;
-    const bool active = row < m && state[row] != 0;
-    if (!__syncthreads_or(active)) return;  // block-uniform: every row is proven
+    const bool active = row < m && state[row] == kRowOpen;
+    if (!__syncthreads_or(active)) return;  // block-uniform: no row for this pass
     const int c0 = blockIdx.y * cpb;
     const int cend = c0 + cpb < n ? c0 + cpb : n;
     const int nt = (cend - c0 + kGtCols - 1) / kGtCols;
@@ -406,7 +407,7 @@ __global__ void __launch_bounds__(256, NB <= 4 ? 2 : 1)
         tc::prefetch_tmap(&tmA);
         for (; issued < nt && issued < kGtStages; issued++) load(issued);
     }
-    // this row's chain and level count (rows past m or proven: none)
+    // this row's chain and level count (rows that are not this pass's: none)
     const int z = active ? Z[row] : 0;
     double sig[kGvMaxLevels], acc[kGvMaxLevels][NB];
     unsigned hm[kGvMaxLevels], thr[kGvMaxLevels];
@@ -421,8 +422,7 @@ __global__ void __launch_bounds__(256, NB <= 4 ? 2 : 1)
         for (int b = 0; b < NB; b++) acc[l][b] = 0.0;
     }
     thr[kGvMaxLevels - 1] = 0u;
-    int L = __reduce_max_sync(0xffffffffu, z + 1);
-    if (L > kGvMaxLevels) L = kGvMaxLevels;  // such a row is not proven: the exact pass decides
+    const int L = __reduce_max_sync(0xffffffffu, z + 1);  // at most kGvMaxLevels
     bool track = true;
     int consumed = 0;
     for (int t = 0; t < nt; t++) {
@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(256, NB <= 4 ? 2 : 1)
 #pragma unroll
             for (int w = 0; w < kGvWarps; w++) v += ps[w * NB * 32 + i];
             const int rr = row0 + (i & 31);
-            if (rr < m && state[rr] != 0) atomicAdd(&P[((size_t)l * nB + (i >> 5)) * m + rr], v);
+            if (rr < m && state[rr] == kRowOpen) atomicAdd(&P[((size_t)l * nB + (i >> 5)) * m + rr], v);
         }
     }
     if (active)
@@ -519,17 +519,21 @@ __global__ void __launch_bounds__(256, NB <= 4 ? 2 : 1)
 // with the tau that the chain has for it (or nothing: then z was too large).
 // A row whose chain breaks at level l gets the true tau_l, a prediction beyond
 // it, the z that follows and another pass.  Rows without a z within the levels
-// held, or whose tau depends on a low word, are left to the exact pass (Z =
-// kGvMaxLevels).  out[0] = the largest
-// z of the proven rows, out[open] counts the others.
+// held, or whose tau depends on a low word, are left to the exact passes
+// (kRowExact).  out[0] = the largest z of the proven rows, out[open] counts the
+// others.
 __global__ void k_gemv_check(int m, int rho, unsigned *__restrict__ W, int *__restrict__ T, int *__restrict__ Z,
                              const int *__restrict__ key, int *__restrict__ state, double *__restrict__ P, int np,
                              int *__restrict__ out, int open) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= m || state[row] == 0) return;
+    if (row >= m || state[row] == kRowProven) return;
+    if (state[row] == kRowExact) {
+        atomicAdd(&out[open], 1);
+        return;
+    }
     int z = Z[row], bad = -1;
     unsigned h = 0;
-    for (int l = 1; l <= z && z < kGvMaxLevels; l++) {
+    for (int l = 1; l <= z; l++) {
         h = W[(size_t)l * m + row];
         if (h == 0) {  // grids are normal, so nothing hides below the high word
             z = l - 1;
@@ -540,8 +544,8 @@ __global__ void k_gemv_check(int m, int rho, unsigned *__restrict__ W, int *__re
             break;
         }
     }
-    if (z < kGvMaxLevels && bad < 0) {
-        state[row] = 0;
+    if (bad < 0) {
+        state[row] = kRowProven;
         atomicMax(&out[0], z);
         return;
     }
@@ -552,7 +556,7 @@ __global__ void k_gemv_check(int m, int rho, unsigned *__restrict__ W, int *__re
     // usual case: a last level with one bit left); otherwise tau is open.
     const int e = (int)(h >> 20) - 1023, low = kLsbBias - key[row];
     const bool power = (h & 0xfffffu) == 0;
-    if (bad > 0 && (!power || low >= e - 20)) {
+    if (!power || low >= e - 20) {
         const int d = 54 - rho;
         int tau = power ? e : e + 1;
         const int G = rho + tau - 53, num = G - low;
@@ -561,14 +565,20 @@ __global__ void k_gemv_check(int m, int rho, unsigned *__restrict__ W, int *__re
         if (nz < kGvMaxLevels)
             for (int l = bad; l < kGvMaxLevels; l++, tau -= d) T[(size_t)l * m + row] = tau;
     }
+    if (nz == kGvMaxLevels) state[row] = kRowExact;
     Z[row] = nz;
     for (int l = 1; l < kGvMaxLevels; l++) W[(size_t)l * m + row] = 0;
     for (int i = 0; i < np; i++) P[(size_t)i * m + row] = 0.0;
 }
 
-// it < 0: the predicted chains T from the row maxima Ma[0..m), every row
-// unproven (state 1), and Z[row] the first all-zero level that the lowest set
-// bit in keys[row] gives (kGvMaxLevels where the prediction does not apply).  it >= 0: the proof after products pass `it` (see above).  out[0]
+// it < 0: the predicted chains T from the row maxima Ma[0..m), and Z[row] the
+// first all-zero level that the lowest set bit in keys[row] gives.  Rows that
+// have none within the levels held, or to which the prediction does not apply,
+// go to the exact passes at once, and with them the 32 rows of their block: an
+// exact pass over the block takes the same time for one row as for all, and the
+// fast ones would be on top of it (a call of 4096 x 4096 with one such row in
+// eight: 2.54 ms with fast passes for all rows, 2.37 with this).
+// it >= 0: the proof after products pass `it` (see above).  out[0]
 // = max over proven rows of z - 1 (z = the first level with a zero remainder
 // maximum), out[1] = 1 when a row has no zero level within the capacity,
 // out[2] is the wait-error flag of the passes, out[4 + it] = rows whose
@@ -577,20 +587,25 @@ __global__ void k_gemv_chain(int m, int rho, int it, double *__restrict__ Ma, in
                              int *__restrict__ state, int *__restrict__ Z, const int *__restrict__ keys,
                              double *__restrict__ P, int np, int *__restrict__ out) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= m) return;
     if (it < 0) {
-        int tau = tau_rule(Ma[row]);
-        const int key = keys[row], d = 54 - rho, G0 = rho + tau - 53;
-        const int num = key == 0 ? 0 : G0 - (kLsbBias - key);
-        int z = num <= 0 ? 0 : (num + d - 1) / d;
-        // sigma, every grid and every threshold normal
-        if (key >= kRowBad || rho + tau > 1000 || G0 - z * d < -1000 || z > kGvMaxLevels) z = kGvMaxLevels;
-        Z[row] = z;
-        for (int l = 0; l < kGvMaxLevels; l++, tau += rho - 54) T[(size_t)l * m + row] = tau;
-        state[row] = 1;
+        bool exact = false;
+        if (row < m) {
+            int tau = tau_rule(Ma[row]);
+            const int key = keys[row], d = 54 - rho, G0 = rho + tau - 53;
+            const int num = key == 0 ? 0 : G0 - (kLsbBias - key);
+            int z = num <= 0 ? 0 : (num + d - 1) / d;
+            // sigma, every grid and every threshold normal
+            if (key >= kRowBad || rho + tau > 1000 || G0 - z * d < -1000 || z > kGvMaxLevels) z = kGvMaxLevels;
+            Z[row] = z;
+            for (int l = 0; l < kGvMaxLevels; l++, tau += rho - 54) T[(size_t)l * m + row] = tau;
+            exact = z == kGvMaxLevels;
+        }
+        exact = __any_sync(0xffffffffu, exact);
+        if (row < m) state[row] = exact ? kRowExact : kRowOpen;
         return;
     }
-    if (state[row] == 0) return;
+    if (row >= m) return;
+    if (state[row] == kRowProven) return;
     int z = -1, bad = -1;
     for (int l = 1; l < kGvMaxLevels + 1; l++) {
         const double v = Ma[(size_t)l * m + row];
@@ -611,7 +626,7 @@ __global__ void k_gemv_chain(int m, int rho, int it, double *__restrict__ Ma, in
         atomicAdd(&out[4 + it], 1);
         return;
     }
-    state[row] = 0;
+    state[row] = kRowProven;
     if (z < 0) atomicExch(&out[1], 1);
     else atomicMax(&out[0], z - 1);
 }
@@ -734,14 +749,14 @@ int gemv_fused_n(cuozblasHandle_t *h, int m, int n, const double *A, int lda, co
                                                                       flags, 4 + it);
                 OZB_CHECK(cudaGetLastError());
             }
-            // The sum where the second pass proves the rest, and one host read; exact passes only when
-            // it does not.  The sum runs over every level held (those past nA add zeros), so it needs
-            // no count.
+            // The sum where the second pass proves the rest, and one host read; the exact passes (those
+            // that find nothing open return at once) and a second read only when it does not.  The sum
+            // runs over every level held (those past nA add zeros), so it needs no count.
             const int lv = maxS < kGvMaxLevels ? maxS : kGvMaxLevels;
             const bool early = fastMode == 0;
-            for (int it = 0; it <= kGtIters; it++) {
-                const int open = 5 + it;  // rows left by the second fast pass, by the exact passes
-                if (it > 0) {
+            for (int round = 0; round < 2; round++) {
+                const int open = round == 0 ? 5 : 5 + kGtIters;  // rows left by the second fast pass, by the last exact one
+                for (int it = 1; round > 0 && it <= kGtIters; it++) {
                     counted(h);
                     OZB_TRY(launch_gt_pred(nB, g2, st->stream, tm, m, n, rho, cpb, T, rstate, xs, ldx, P, Ma, err));
                     counted(h);
@@ -754,7 +769,11 @@ int gemv_fused_n(cuozblasHandle_t *h, int m, int n, const double *A, int lda, co
                                           st->stream));
                 OZB_CHECK(cudaStreamSynchronize(st->stream));
                 if (st->h_ints[2] != 0) return CUOZBLAS_STATUS_DEVICE_TIMEOUT;
-                if (st->h_ints[1] != 0) break;  // a row has no zero level within the capacity
+                if (st->h_ints[1] != 0) {  // a row's true chain has no zero level within the levels held
+                    if (maxS <= kGvMaxLevels) break;
+                    ar.release(mk);
+                    return CUOZBLAS_STATUS_NOT_SUPPORTED;  // nor have the level passes: that call 1.89 ms without them
+                }
                 if (st->h_ints[open] != 0) continue;
                 const int zmax = st->h_ints[0];  // every chain proven
                 const int c = (zmax < 1 ? 1 : zmax) + 1;  // the lines rule's count
