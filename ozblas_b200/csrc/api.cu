@@ -93,6 +93,7 @@ int counter_init(cuozblasHandle_t *h) {
     h->n_comp = 0.f;
     state(h)->off = h->memMaskSplitA;
     h->memAddr = h->memMaskSplitA;
+    state(h)->plain_timers = state(h)->span_timer = false;
     return CUOZBLAS_STATUS_SUCCESS;
 }
 
@@ -665,11 +666,13 @@ int cuozblasDcsrmv(cuozblasHandle_t *h, char trans, int32_t m, int32_t n, int32_
     const int64_t ld = splitA_ld(nnz);
     int nA = 0;
     CsrSplitRows rows;
+    span_begin(h);  // of this path's kernels (one that declined has left its own)
     OZB_TRY(split_csr_count(h, m, val, rowptr, h->splitEpsMode, 1, maxS, &nA, &rows));
     double *As = ar.take<double>((uint64_t)nA * ld);
     if (!ar.ok) return CUOZBLAS_STATUS_WORKSPACE;
     OZB_TRY(split_csr_write(h, m, nnz, val, rowptr, h->splitEpsMode, 1, nA, As, ld, rows));
     OZB_TRY(csrmv_presplit(h, m, n, alpha, As, nA, ld, colind, rowptr, x, beta, y));
+    span_end(h);
     return finish(h, t0);
 }
 

@@ -285,7 +285,7 @@ int gemm_f32_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, do
     // rho >= 47 (k > 1024): every slice is an int8 times a power of two, and the
     // exact slice products run on the INT8 tensor cores (same bits)
     if (!dot && !skinny_n && rho >= 47 && !state(h)->env.ds_simt) {
-        st->plain_timers = true;
+        phases_begin(h);
         int nA = 0, nB = 0, np = 0;
         OZB_TRY(gemm_ds_i8_core(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, rho, fastMode, &nA, &nB,
                                 &np));
@@ -298,8 +298,7 @@ int gemm_f32_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, do
     }
 
     // ---- split ----  (phase events 0..4: start, A split, B split, products, sum)
-    ev_record(h, 0);
-    st->plain_timers = true;
+    phases_begin(h);
     float *Sa = nullptr, *Sb = nullptr;
     short *Ea = nullptr, *Eb = nullptr;
     int nA = 0, nB = 0;

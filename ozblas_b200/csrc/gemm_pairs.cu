@@ -1233,8 +1233,7 @@ int gemm_pairs_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
             return CUOZBLAS_STATUS_SUCCESS;
         }
         const uint64_t mark1 = ar.mark();
-        ev_record(h, 0);
-        st->plain_timers = true;
+        phases_begin(h);
         OZB_CHECK(cudaMemsetAsync(st->d_ints, 0, (kPairErrInt + 1) * sizeof(int), st->stream));
         for (int o = 0; o < 2; o++) {
             const bool strided = o == 0 ? !is_trans(ta) : is_trans(tb);

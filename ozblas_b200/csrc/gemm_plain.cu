@@ -442,8 +442,7 @@ int gemm_plain_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
     const int ldk = dot || skinny_n ? ceil_to(k > 0 ? k : 1, 2) : ceil_to(k > 0 ? k : 1, kBK);
 
     // ---- split ----  (phase events 0..4: start, A split, B split, products, sum)
-    ev_record(h, 0);
-    st->plain_timers = true;
+    phases_begin(h);
     // GEMV 'n' with NearSum: correctly rounded exact row dots, A read once
     if (skinny_n && !dot && !is_trans(ta) && h->sumMode == 1 && fastMode == 0 && h->splitEpsMode == 0 &&
         !state(h)->env.gemv_split && !state(h)->env.gemv_slices) {
@@ -459,7 +458,7 @@ int gemm_plain_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
             h->nbk = n;
             return CUOZBLAS_STATUS_SUCCESS;  // gemv_rn_n recorded the span of its kernels (t_comp)
         }
-        ev_record(h, 0);
+        phases_begin(h);
     }
     // GEMV 't' (lines contiguous): split and products in registers
     if (skinny_n && !dot && is_trans(ta) && fastMode == 0 && h->splitEpsMode == 0 && !st->env.gemv_split) {
@@ -475,7 +474,7 @@ int gemm_plain_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
             h->nbk = n;
             return CUOZBLAS_STATUS_SUCCESS;
         }
-        ev_record(h, 0);
+        phases_begin(h);
     }
     // GEMV 'n' (rows of A strided): fused split and products, A read nA + 2 times
     if (skinny_n && !dot && !is_trans(ta) && !state(h)->env.gemv_split) {
@@ -505,13 +504,13 @@ int gemm_plain_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
         }
         if (fr != CUOZBLAS_STATUS_NOT_SUPPORTED) return fr;
         ar.release(mk0);  // more levels than the fused kernel holds: the materialised path
-        ev_record(h, 0);
+        phases_begin(h);
     }
     if (!dot && !skinny_n && !st->env.plain_dmma) {
         bool done = false;
         OZB_TRY(gemm_pairs_core<double>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, fastMode, rho, &done));
         if (done) return CUOZBLAS_STATUS_SUCCESS;
-        ev_record(h, 0);
+        phases_begin(h);
     }
     double *Sa = nullptr, *Sb = nullptr;
     int nA = 0, nB = 0;
@@ -755,15 +754,14 @@ int gemm_sd_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, flo
     const bool skinny_n = (n == 1);
     const int ldk = dot || skinny_n ? ceil_to(k > 0 ? k : 1, 2) : ceil_to(k > 0 ? k : 1, kBK);
 
-    ev_record(h, 0);
-    st->plain_timers = true;
+    phases_begin(h);
     // for rho >= 2 (k > 128) x + sigma stays in sigma's binade: every slice is q 2^(rho - 24)
     if (!dot && !skinny_n && rho >= 2 && !st->env.sd_dmma) {
         bool done = false;
         OZB_TRY(gemm_pairs_core<float>(h, ta, tb, m, n, k, (double)alpha, A, lda, B, ldb, (double)beta, C, ldc, fastMode,
                                        rho, &done));
         if (done) return CUOZBLAS_STATUS_SUCCESS;
-        ev_record(h, 0);
+        phases_begin(h);
     }
     double *Sa = nullptr, *Sb = nullptr;
     short *Ea = nullptr, *Eb = nullptr;

@@ -241,8 +241,7 @@ int gemm_q_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, cons
     const bool skinny_n = (n == 1);
     const int ldk = dot || skinny_n ? ceil_to(k > 0 ? k : 1, 2) : ceil_to(k > 0 ? k : 1, 16);
 
-    ev_record(h, 0);
-    st->plain_timers = true;
+    phases_begin(h);
     double *Sa = nullptr, *Sb = nullptr;
     short *Ea = nullptr, *Eb = nullptr;
     int nA = 0, nB = 0;

@@ -83,10 +83,12 @@ inline void counted(cuozblasHandle_t *h) { state(h)->launches++; }
 
 // Phase timers of the reference handle (t_SplitA, t_SplitB, t_comp), taken
 // with CUDA events on the handle's stream; read after the call's final sync.
-// (event 1 ends a split: the call has phases, whatever path declined before)
-inline void ev_record(cuozblasHandle_t *h, int i) {
-    if (i == 1) state(h)->span_timer = false;
-    cudaEventRecord(state(h)->ev[i], state(h)->stream);
+inline void ev_record(cuozblasHandle_t *h, int i) { cudaEventRecord(state(h)->ev[i], state(h)->stream); }
+// Event 0 of a call with phases, whatever path of it declined before.
+inline void phases_begin(cuozblasHandle_t *h) {
+    state(h)->span_timer = false;
+    state(h)->plain_timers = true;
+    ev_record(h, 0);
 }
 inline float ev_ms(cuozblasHandle_t *h, int a, int b) {
     float ms = 0.f;

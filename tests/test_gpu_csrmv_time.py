@@ -1,0 +1,19 @@
+"""The exec info's times of a call whose first path declined are those of the path that computed the result."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def test_csrmv_general_path_time(handle, ozb, cuda):
+    """x off the predicted chain: t_comp spans the split and the products of the general path, most of the call."""
+    n, w = 400000, 6
+    gen = cuda.Generator(device="cuda").manual_seed(1)
+    rowptr = cuda.arange(0, (n + 1) * w, w, dtype=cuda.int32, device="cuda")
+    colind = cuda.randint(0, n, (n * w,), dtype=cuda.int32, device="cuda", generator=gen)
+    val = cuda.randn(n * w, dtype=cuda.float64, device="cuda", generator=gen)
+    x = cuda.randn(n, dtype=cuda.float64, device="cuda", generator=gen) * 2.0 ** -40
+    x[n // 2] = 1.0
+    y = cuda.zeros(n, dtype=cuda.float64, device="cuda")
+    for _ in range(3):
+        ozb.dcsrmv(handle, "n", n, n, n * w, 1.0, val, colind, rowptr, x, 0.0, y)
+    assert 0.5 * handle.t_total < handle.t_comp <= handle.t_total, (handle.t_comp, handle.t_total)
