@@ -1,6 +1,9 @@
-"""The slice-pair product's plans, against other paths of the same bits."""
+"""The slice-pair product's plans: arenas that force column blocks, leading dimensions above the sizes, and the sum
+inside the product kernel with three and four digits, against other paths of the same bits."""
 import numpy as np
 import pytest
+
+from tests.conftest import bits_equal, first_diff
 
 pytestmark = pytest.mark.gpu
 
@@ -43,3 +46,39 @@ def test_column_blocks(sm, m, n, k, digits, tile, handle, ozb, cuda):
         block = min(-(-half // tile), cols // tile) * tile
         assert launches == 2 + 2 * -(-n // block), cols
         assert cuda.equal(out, ref), cols
+
+
+@pytest.mark.parametrize("form,ta,tb,m,n,k,mode", [
+    ("d", "n", "t", 200, 150, 300, 0), ("d", "t", "n", 130, 300, 128, 0), ("d", "n", "n", 2100, 1700, 200, 0),
+    ("d", "t", "n", 1300, 1100, 128, 0), ("d", "n", "t", 2100, 1700, 90, 0), ("d", "t", "t", 1, 300, 200, 0),
+    ("sd", "n", "t", 200, 150, 300, 0), ("sd", "t", "n", 2100, 1700, 129, 0), ("sd", "n", "n", 1100, 900, 70000, 9)])
+def test_leading_dimensions(form, ta, tb, m, n, k, mode, handle, ozb, cuda, monkeypatch):
+    """lda, ldb and ldc above the sizes, a few lines that need more levels than the rest; the memory between the lines
+    is NaN and stays so in C.  The last case has four digits in the mixed form."""
+    gen = cuda.Generator(device="cuda").manual_seed(m + n + k)
+    dt = cuda.float64 if form == "d" else cuda.float32
+
+    def mat(lines, length, pad):
+        full = cuda.full((lines, length + pad), float("nan"), dtype=dt, device="cuda")
+        u = cuda.rand((lines, length), dtype=cuda.float64, device="cuda", generator=gen) - 0.5
+        full[:, :length] = (u * cuda.randn((lines, length), dtype=cuda.float64, device="cuda", generator=gen).exp()).to(dt)
+        return full
+
+    A = mat(k, m, 5) if ta == "n" else mat(m, k, 3)
+    B = mat(n, k, 1) if tb == "n" else mat(k, n, 2)
+    if ta == "t" and m > 3:
+        A[3, :k] *= cuda.exp2(cuda.randint(-40, 40, (k,), device="cuda", generator=gen).to(dt))
+    C0 = mat(n, m, 7)
+    handle.splitEpsMode = mode
+    call = ozb.dgemm if form == "d" else ozb.sdgemm
+    outs = []
+    for dmma in (False, True):
+        if dmma:
+            monkeypatch.setenv("OZBLAS_PLAIN_DMMA" if form == "d" else "OZBLAS_SD_DMMA", "1")
+            handle.read_env()
+        C = C0.clone()
+        call(handle, ta, tb, m, n, k, 1.25, A, A.shape[1], B, B.shape[1], -0.5, C, C.shape[1])
+        outs.append(C.cpu().numpy())
+    got, want = (o[:, :m].astype(np.float64) for o in outs)
+    assert bits_equal(got, want), first_diff(got, want)
+    assert np.isnan(outs[0][:, m:]).all()
