@@ -1089,8 +1089,9 @@ int pair_status(cuozblasHandle_t *h) {
 // inlined a term took 74, and the code did not fit the instruction cache).
 // Entries of pairs that the product kernel skipped hold anything: the lines'
 // marks at those levels make them zeros.  *err: a wait of the product kernel ran
-// out, so the buffer is not complete and C stays as it is (the word is read
-// first and tested last, behind the loads of the pairs).
+// out, so the buffer is not complete and C stays as it is (a warp without a part
+// in the lists reads the word: by every thread into a register, or by the first
+// warp, it cost 3 us of the 278 of a call at 1024^3).
 constexpr int kPsRows = 256, kPsCols = 2, kPsIn = 16;
 constexpr int kPsLevels = 12, kPsPairs = 144;  // held in shared memory; k_pair_sum_any beyond
 
@@ -1115,7 +1116,7 @@ __global__ void __launch_bounds__(kPsRows, 4)
     k_pair_sum(int m, int n, int col0, int cn, int nA, int nB, int np, const double *__restrict__ pbuf,
                const short *__restrict__ ea, const short *__restrict__ eb, int bias, double alpha, double beta,
                void *__restrict__ Cv, int ldc, const int *__restrict__ err) {
-    const int failed = *err;
+    __shared__ int failed;
     __shared__ short sA[kPsLevels][kPsRows];
     __shared__ int2 sP[kPsCols][kPsPairs];  // A level, B level's tau
     const int rb = (m + kPsRows - 1) / kPsRows, tr = threadIdx.x;
@@ -1123,6 +1124,7 @@ __global__ void __launch_bounds__(kPsRows, 4)
     const int nc = min(kPsCols, col0 + cn - c0);
     if (row < m)
         for (int s = 0; s < nA; s++) sA[s][tr] = ea[(size_t)s * m + row];
+    if (tr == kPsRows - 1) failed = *err;  // beside the first warps' lists
     for (int i = tr; i < np * nc; i += kPsRows) {
         const int q = i / nc, c = i - q * nc;
         int ia, ib;
