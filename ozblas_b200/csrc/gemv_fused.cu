@@ -572,12 +572,12 @@ __global__ void k_gemv_check(int m, int rho, unsigned *__restrict__ W, int *__re
 }
 
 // it < 0: the predicted chains T from the row maxima Ma[0..m), and Z[row] the
-// first all-zero level that the lowest set bit in keys[row] gives.  Rows that
+// first all-zero level that the lowest set bit in keys[row] gives; rows that
 // have none within the levels held, or to which the prediction does not apply,
-// go to the exact passes at once, and with them the 32 rows of their block: an
-// exact pass over the block takes the same time for one row as for all, and the
-// fast ones would be on top of it (a call of 4096 x 4096 with one such row in
-// eight: 2.54 ms with fast passes for all rows, 2.37 with this).
+// go to the exact passes at once (the fast ones would cut all 8 levels of theirs,
+// and of the rows beside them, in vain).  The other rows of their blocks keep
+// the fast passes: with the block left to the exact ones, whose predictions are
+// corrected a level a pass, 3000 x 2000 with one infinity took 270 us, 224 so.
 // it >= 0: the proof after products pass `it` (see above).  out[0]
 // = max over proven rows of z - 1 (z = the first level with a zero remainder
 // maximum), out[1] = 1 when a row has no zero level within the capacity,
@@ -587,24 +587,19 @@ __global__ void k_gemv_chain(int m, int rho, int it, double *__restrict__ Ma, in
                              int *__restrict__ state, int *__restrict__ Z, const int *__restrict__ keys,
                              double *__restrict__ P, int np, int *__restrict__ out) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row >= m) return;
     if (it < 0) {
-        bool exact = false;
-        if (row < m) {
-            int tau = tau_rule(Ma[row]);
-            const int key = keys[row], d = 54 - rho, G0 = rho + tau - 53;
-            const int num = key == 0 ? 0 : G0 - (kLsbBias - key);
-            int z = num <= 0 ? 0 : (num + d - 1) / d;
-            // sigma, every grid and every threshold normal
-            if (key >= kRowBad || rho + tau > 1000 || G0 - z * d < -1000 || z > kGvMaxLevels) z = kGvMaxLevels;
-            Z[row] = z;
-            for (int l = 0; l < kGvMaxLevels; l++, tau += rho - 54) T[(size_t)l * m + row] = tau;
-            exact = z == kGvMaxLevels;
-        }
-        exact = __any_sync(0xffffffffu, exact);
-        if (row < m) state[row] = exact ? kRowExact : kRowOpen;
+        int tau = tau_rule(Ma[row]);
+        const int key = keys[row], d = 54 - rho, G0 = rho + tau - 53;
+        const int num = key == 0 ? 0 : G0 - (kLsbBias - key);
+        int z = num <= 0 ? 0 : (num + d - 1) / d;
+        // sigma, every grid and every threshold normal
+        if (key >= kRowBad || rho + tau > 1000 || G0 - z * d < -1000 || z > kGvMaxLevels) z = kGvMaxLevels;
+        Z[row] = z;
+        for (int l = 0; l < kGvMaxLevels; l++, tau += rho - 54) T[(size_t)l * m + row] = tau;
+        state[row] = z < kGvMaxLevels ? kRowOpen : kRowExact;
         return;
     }
-    if (row >= m) return;
     if (state[row] == kRowProven) return;
     int z = -1, bad = -1;
     for (int l = 1; l < kGvMaxLevels + 1; l++) {
@@ -749,14 +744,16 @@ int gemv_fused_n(cuozblasHandle_t *h, int m, int n, const double *A, int lda, co
                                                                       flags, 4 + it);
                 OZB_CHECK(cudaGetLastError());
             }
-            // The sum where the second pass proves the rest, and one host read; the exact passes (those
-            // that find nothing open return at once) and a second read only when it does not.  The sum
-            // runs over every level held (those past nA add zeros), so it needs no count.
+            // The sum where the second pass proves the rest, and one host read; an exact pass and a
+            // second read only when it does not, the other exact passes together and a third read
+            // when rows are left after that.  The sum runs over every level held (those past nA add
+            // zeros), so it needs no count.
             const int lv = maxS < kGvMaxLevels ? maxS : kGvMaxLevels;
             const bool early = fastMode == 0;
-            for (int round = 0; round < 2; round++) {
-                const int open = round == 0 ? 5 : 5 + kGtIters;  // rows left by the second fast pass, by the last exact one
-                for (int it = 1; round > 0 && it <= kGtIters; it++) {
+            int it = 0;  // exact passes enqueued
+            for (const int upto : {0, 1, kGtIters}) {
+                while (it < upto) {
+                    it++;
                     counted(h);
                     OZB_TRY(launch_gt_pred(nB, g2, st->stream, tm, m, n, rho, cpb, T, rstate, xs, ldx, P, Ma, err));
                     counted(h);
@@ -764,6 +761,7 @@ int gemv_fused_n(cuozblasHandle_t *h, int m, int n, const double *A, int lda, co
                                                                           kGvMaxLevels * nB, flags);
                     OZB_CHECK(cudaGetLastError());
                 }
+                const int open = 5 + it;  // rows left by the second fast pass, by the last exact one
                 if (early) OZB_TRY(sum_rows_if_launch(h, m, lv, nB, lv + nB - 2, P, m, alpha, beta, y, scratch, flags, open));
                 OZB_CHECK(cudaMemcpyAsync(st->h_ints, flags, sizeof(int) * (6 + kGtIters), cudaMemcpyDeviceToHost,
                                           st->stream));
@@ -772,7 +770,7 @@ int gemv_fused_n(cuozblasHandle_t *h, int m, int n, const double *A, int lda, co
                 if (st->h_ints[1] != 0) {  // a row's true chain has no zero level within the levels held
                     if (maxS <= kGvMaxLevels) break;
                     ar.release(mk);
-                    return CUOZBLAS_STATUS_NOT_SUPPORTED;  // nor have the level passes: that call 1.89 ms without them
+                    return CUOZBLAS_STATUS_NOT_SUPPORTED;  // nor have the level passes
                 }
                 if (st->h_ints[open] != 0) continue;
                 const int zmax = st->h_ints[0];  // every chain proven
