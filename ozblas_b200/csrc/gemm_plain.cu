@@ -461,10 +461,11 @@ int gemm_plain_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
         phases_begin(h);
     }
     // GEMV 't' (lines contiguous): split and products in registers
+    VecSlices kept;  // x's slices from it
     if (skinny_n && !dot && is_trans(ta) && fastMode == 0 && h->splitEpsMode == 0 && !st->env.gemv_split) {
         bool done = false;
         int nAv = 0, nBv = 0;
-        OZB_TRY(gemv_t_fused(h, m, k, A, lda, B, alpha, beta, C, &done, &nAv, &nBv));
+        OZB_TRY(gemv_t_fused(h, m, k, A, lda, B, alpha, beta, C, &done, &nAv, &nBv, &kept));
         if (done) {
             const int ml = (nAv - 1) + (nBv - 1);
             h->nSplitA = (float)nAv;
@@ -513,7 +514,7 @@ int gemm_plain_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
         phases_begin(h);
     }
     double *Sa = nullptr, *Sb = nullptr;
-    int nA = 0, nB = 0;
+    int nA = 0, nB = 0, ldb_s = ldk;
     if (dot) {
         Sa = ar.take<double>((uint64_t)maxS * ldk);
         if (!ar.ok) return CUOZBLAS_STATUS_WORKSPACE;
@@ -523,7 +524,11 @@ int gemm_plain_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
         OZB_TRY(split_operand(h, !is_trans(ta), m, k, A, lda, rho, maxS, ldk, &Sa, &nA, ar));
     }
     ev_record(h, 1);
-    if (skinny_n) {
+    if (kept.xs) {
+        Sb = kept.xs;
+        nB = kept.ns;
+        ldb_s = kept.ld;
+    } else if (skinny_n) {
         Sb = ar.take<double>((uint64_t)maxS * ldk);
         if (!ar.ok) return CUOZBLAS_STATUS_WORKSPACE;
         OZB_TRY(split_vector(h, k, B, rho, maxS, Sb, ldk, &nB));
@@ -584,7 +589,7 @@ int gemm_plain_core(cuozblasHandle_t *h, char ta, char tb, int m, int n, int k, 
                 } else {
                     const int blocks = (int)(((int64_t)m * 32 + 255) / 256);
                     counted(h);
-                    k_pair_gemv<<<blocks, 256, 0, st->stream>>>(m, k, na, nb, ia0, ib0, nB, Sa, ldk, Sb, ldk, P,
+                    k_pair_gemv<<<blocks, 256, 0, st->stream>>>(m, k, na, nb, ia0, ib0, nB, Sa, ldk, Sb, ldb_s, P,
                                                                 ldp);
                 }
                 OZB_CHECK(cudaGetLastError());

@@ -16,9 +16,10 @@
 // the ordered sum over the pairs follows, per line.  What bounds it is the FP64
 // pipe: per element 3 L + L nB operations for L levels of the line against
 // nB slices of x (28 for 4 x 4), 18 T a second on the chip.
-// Lines with more than kGtLevels levels, Inf / NaN or exponents near the ends
-// of the range, and x with more than kGtLevels slices, leave the call to the
-// slice path (nothing is written).
+// Lines with more than kGtLevels levels or with Inf / NaN are listed and done by
+// a block each, level by level (k_gemv_t_deep).  Exponents near the ends of the
+// range, and x with Inf / NaN or more than kGtLevels slices, leave the call to
+// the slice path (nothing is written; x's slices are kept for it).
 //
 // 6001 x 3001 (phi = 1, 5 x 4 levels), one B200: the materialised path 853 us a
 // call (split 309, products 466, x's split 19), this one 206 (statistics 35,
@@ -161,11 +162,12 @@ int split_vector_small(cuozblasHandle_t *h, int n, const double *x, int rho, int
 struct GemvTStatus {  // zeroed before the launch
     int declined;     // some line (or x) needs the slice path: y is not written
     int zmax;         // the largest first all-zero level of a line
+    int ndeep;        // lines listed for k_gemv_t_deep
 };
 
 struct GtPlan {
     double sig[kGtLevels];
-    int L, z, bad;
+    int L, z, bad;  // L above kGtLevels: a deep line
 };
 
 // A (part of a) line's statistics from the first pass: the largest |v| (+inf
@@ -183,19 +185,21 @@ __device__ __forceinline__ GtPlan gt_predict(int tau0, int lb, int rho, int maxS
     p.z = num <= 0 ? 0 : (num + d - 1) / d;
     p.L = p.z + 1 < maxS ? p.z + 1 : maxS;
     // every sigma and grid normal, every slice product on a representable grid
-    p.bad = p.L > kGtLevels || rho + tau0 > 1000 || G0 - p.z * d < -1000 || G0 - (p.L - 1) * d + glast < -1060;
+    p.bad = rho + tau0 > 1000 || G0 - p.z * d < -1000 || G0 - (p.L - 1) * d + glast < -1060;
 #pragma unroll
     for (int s = 0; s < kGtLevels; s++) p.sig[s] = 0.75 * pow2(rho + tau0 - s * d);
     return p;
 }
 
-// Pass 1: one warp per (line, part of it).
+// Pass 1: one warp per (line, part of it), ended after its first loads when x
+// leaves the call to the slice path.
 __global__ void __launch_bounds__(256) k_gemv_t_stats(int nl, int k, const double *__restrict__ A, int lda, int parts,
-                                                      GtStat *__restrict__ out) {
+                                                      const VecSplitInfo *__restrict__ info, GtStat *__restrict__ out) {
     const int w = (int)(((int64_t)blockIdx.x * 256 + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     const int row = w / parts, part = w % parts;
     if (row >= nl) return;
     const double *a = A + (size_t)row * lda;
+    const int xbad = info->bad, xnz = info->nz;
     LazyStats rs;
     constexpr int kIn = 8;
     const int step = 32 * parts;
@@ -204,6 +208,7 @@ __global__ void __launch_bounds__(256) k_gemv_t_stats(int nl, int k, const doubl
         double v[kIn];
 #pragma unroll
         for (int u = 0; u < kIn; u++) v[u] = __ldg(a + i + u * step);
+        if (xbad || xnz > kGtLevels) return;  // uniform
 #pragma unroll
         for (int u = 0; u < kIn; u++) lazy_elem(rs, v[u]);
         lazy_sync(rs);
@@ -326,7 +331,8 @@ template <int WPR, int NB>
 __device__ __forceinline__ void gt_lines(int nl, int k, const double *__restrict__ A, int lda,
                                          const double *__restrict__ xs, int ldx, const VecSplitInfo &xi, int rho,
                                          int maxS, int sum_mode, int parts, const GtStat *__restrict__ stats,
-                                         double *__restrict__ yt, GemvTStatus *st, GtShared &sh) {
+                                         double *__restrict__ yt, GemvTStatus *st, int *__restrict__ deep_lines,
+                                         GtShared &sh) {
     auto &ps = sh.ps;
     auto &smx = sh.smx;
     auto &shm = sh.shm;
@@ -372,8 +378,9 @@ __device__ __forceinline__ void gt_lines(int nl, int k, const double *__restrict
     const bool nonfinite = !(mx <= 1.7976931348623157e308);
     const int tau0 = nonfinite ? 0 : tau_rule(mx);
     GtPlan pl = gt_predict(tau0, lb, rho, maxS, xi.glast);
-    bool bad = nonfinite || pl.bad || tau0 + xi.tau0 + ceil_log2_int((uint32_t)k) > 1000;
-    if (bad) pl.L = 0;
+    bool deep = nonfinite || pl.L > kGtLevels;
+    bool bad = !deep && (pl.bad || tau0 + xi.tau0 + ceil_log2_int((uint32_t)k) > 1000);
+    if (bad || deep) pl.L = 0;
     const int step = 32 * WPR;
 
     // ---- pass 2 ----
@@ -441,7 +448,7 @@ __device__ __forceinline__ void gt_lines(int nl, int k, const double *__restrict
                 proven = proven && h > thr(s);
             }
         }
-    if (!bad && !proven) {  // the exact chain, one pass per level, and the products again (x's slices from L2)
+    if (!bad && !deep && !proven) {  // the exact chain, one pass per level, and the products again (x's slices from L2)
         int z = maxS - 1, L = maxS;
         for (int s = 1;; s++) {
             uint64_t m = 0;
@@ -467,16 +474,15 @@ __device__ __forceinline__ void gt_lines(int nl, int k, const double *__restrict
             }
             if (s == maxS) break;
             const int tau = tau_rule(__longlong_as_double((long long)mm));
-            if (s == kGtLevels || rho + tau - 53 < -1000 || rho + tau - 53 + xi.glast < -1060) {
-                bad = true;
-                break;
-            }
+            deep = s == kGtLevels;
+            bad = !deep && (rho + tau - 53 < -1000 || rho + tau - 53 + xi.glast < -1060);
+            if (bad || deep) break;
 #pragma unroll
             for (int q = 0; q < kGtLevels; q++)
                 if (q == s) pl.sig[q] = 0.75 * pow2(rho + tau);
         }
         pl.z = z;
-        pl.L = bad ? 0 : L;
+        pl.L = bad || deep ? 0 : L;
 #pragma unroll
         for (int s = 0; s < kGtLevels; s++)
 #pragma unroll
@@ -491,12 +497,15 @@ __device__ __forceinline__ void gt_lines(int nl, int k, const double *__restrict
     double t = 0.0;
     gt_line_sum<WPR, NB>(P, pl.L, nB, sum_mode, ps, warp, lane, group, &t);
     if (live && sub == 0 && lane == 0) {
-        if (bad)
-            atomicOr(&st->declined, 1);
-        else
-            __stcg(yt + row, t);
         const int z = pl.z < maxS - 1 ? pl.z : maxS - 1;
-        if (z > __ldcg(&st->zmax)) atomicMax(&st->zmax, z);
+        if (deep)
+            deep_lines[atomicAdd(&st->ndeep, 1)] = row;
+        else if (bad)
+            atomicOr(&st->declined, 1);
+        else {
+            __stcg(yt + row, t);
+            if (z > __ldcg(&st->zmax)) atomicMax(&st->zmax, z);
+        }
     }
 }
 
@@ -504,7 +513,7 @@ template <int WPR>
 __global__ void __launch_bounds__(kGtThreads, 2)
     k_gemv_t(int nl, int k, const double *__restrict__ A, int lda, const double *__restrict__ xs, int ldx,
              const VecSplitInfo *__restrict__ info, int rho, int maxS, int sum_mode, int parts,
-             const GtStat *__restrict__ stats, double *__restrict__ yt, GemvTStatus *st) {
+             const GtStat *__restrict__ stats, double *__restrict__ yt, GemvTStatus *st, int *__restrict__ deep_lines) {
     const VecSplitInfo xi = *info;
     __shared__ __align__(16) GtShared sh;
     if (xi.bad || xi.nz > kGtLevels) {  // uniform over the grid
@@ -512,25 +521,109 @@ __global__ void __launch_bounds__(kGtThreads, 2)
         return;
     }
     if (xi.nz <= 4)
-        gt_lines<WPR, 4>(nl, k, A, lda, xs, ldx, xi, rho, maxS, sum_mode, parts, stats, yt, st, sh);
+        gt_lines<WPR, 4>(nl, k, A, lda, xs, ldx, xi, rho, maxS, sum_mode, parts, stats, yt, st, deep_lines, sh);
     else
-        gt_lines<WPR, 6>(nl, k, A, lda, xs, ldx, xi, rho, maxS, sum_mode, parts, stats, yt, st, sh);
+        gt_lines<WPR, 6>(nl, k, A, lda, xs, ldx, xi, rho, maxS, sum_mode, parts, stats, yt, st, deep_lines, sh);
 }
 
-// y, once it is known that every line has its sum.
-__global__ void k_gemv_t_write(int nl, const double *__restrict__ yt, const GemvTStatus *__restrict__ st, double alpha,
-                               double beta, double *__restrict__ y) {
+// A deep line: a block follows its true chain, the remainders in shared memory
+// (k doubles), and adds each level's products as it is cut.  What binds it is the
+// chain: a cut, a block maximum and nB block sums a level, some 2 us.  2000 lines
+// of 3000, one of them such: the call 156 us, all of them 351 (by the slice path
+// alone 627 and 680, after a declined pass over the lines 704 and 747).
+__global__ void __launch_bounds__(kGtThreads) k_gemv_t_deep(int k, const double *__restrict__ A, int lda,
+                                                            const double *__restrict__ xs, int ldx,
+                                                            const VecSplitInfo *__restrict__ info, int rho, int maxS,
+                                                            int sum_mode, const int *__restrict__ deep_lines,
+                                                            double *__restrict__ yt, GemvTStatus *st) {
+    extern __shared__ double rem[];
+    __shared__ double red[kGtThreads / 32], part[kGtLevels][kGtThreads / 32];
+    __shared__ double P[kMaxSplitDefault * kGtLevels], terms[kMaxSplitDefault * kGtLevels];
+    const VecSplitInfo xi = *info;
+    const int t = threadIdx.x, line = deep_lines[blockIdx.x], nB = xi.nz;
+    const double *a = A + (size_t)line * lda;
+    double mx = 0.0;
+    bool nonfinite = false;
+    for (int i = t; i < k; i += kGtThreads) {
+        const double v = a[i];
+        rem[i] = v;
+        mx = ref_max(mx, fabs(v));
+        nonfinite |= !isfinite(v);
+    }
+    nonfinite = __syncthreads_or(nonfinite);
+    mx = block_max_nonneg(mx, red);
+    // (no slice of x would make NaN of it)
+    bool bad = (nonfinite && nB == 0) || tau_rule(mx) + xi.tau0 + ceil_log2_int((uint32_t)k) > 1000;
+    int L = maxS, z = maxS - 1;
+    for (int s = 0; s < maxS && !bad; s++) {  // uniform
+        const int tau = tau_rule(mx);
+        bad = rho + tau > 1000 || rho + tau - 53 < -1000 || rho + tau - 53 + xi.glast < -1060;
+        if (bad) break;
+        const double sigma = 0.75 * pow2(rho + tau);
+        double acc[kGtLevels], nm = 0.0;
+#pragma unroll
+        for (int b = 0; b < kGtLevels; b++) acc[b] = 0.0;
+        for (int i = t; i < k; i += kGtThreads) {
+            double r = rem[i];
+            const double sl = (r + sigma) - sigma;
+            r = r - sl;
+            rem[i] = r;
+            nm = ref_max(nm, fabs(r));
+#pragma unroll
+            for (int b = 0; b < kGtLevels; b++)
+                if (b < nB) acc[b] = fma(sl, xs[(size_t)b * ldx + i], acc[b]);
+        }
+#pragma unroll
+        for (int b = 0; b < kGtLevels; b++) {
+            for (int o = 16; o > 0; o >>= 1) acc[b] += __shfl_xor_sync(0xffffffffu, acc[b], o);
+            if ((t & 31) == 0) part[b][t >> 5] = acc[b];
+        }
+        mx = block_max_nonneg(nm, red);  // synchronises: the parts are written
+        if (t < kGtLevels) {
+            double v = 0.0;
+            for (int w = 0; w < kGtThreads / 32; w++) v += part[t][w];
+            P[s * kGtLevels + t] = v;
+        }
+        if (mx == 0.0) {
+            L = s + 1;
+            z = s;
+            break;
+        }
+        __syncthreads();  // before the parts are written again
+    }
+    __syncthreads();
+    if (t != 0) return;
+    if (bad) {
+        atomicOr(&st->declined, 1);
+        return;
+    }
+    int np = 0;
+    for_each_pair(L, nB, L + nB - 2, [&](int ia, int ib) { terms[np++] = P[ia * kGtLevels + ib]; });
+    double sum = 0.0;
+    if (sum_mode == 1)
+        sum = nearsum(np, terms, 1);
+    else
+        for (int i = 0; i < np; i++) sum += terms[i];
+    yt[line] = sum;
+    atomicMax(&st->zmax, z);
+}
+
+// y, once it is known that every line has its sum (the first `ndeep` deep ones done).
+__global__ void k_gemv_t_write(int nl, const double *__restrict__ yt, const GemvTStatus *__restrict__ st, int ndeep,
+                               double alpha, double beta, double *__restrict__ y) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < nl && !st->declined) y[r] = fma(alpha, yt[r], beta * y[r]);
+    if (r < nl && !st->declined && st->ndeep == ndeep) y[r] = fma(alpha, yt[r], beta * y[r]);
 }
 
 // y = alpha A^T x + beta y over nl lines of length k (line l at A + l lda),
 // splitEpsMode 0 and the full pair set.  *done false (y untouched) when the
-// slice path must run.
+// slice path must run: then xs has x's slices where they were formed and the
+// arena has room beside them (they stay allocated), else null.
 int gemv_t_fused(cuozblasHandle_t *h, int nl, int k, const double *A, int lda, const double *x, double alpha,
-                 double beta, double *y, bool *done, int *nA, int *nB) {
+                 double beta, double *y, bool *done, int *nA, int *nB, VecSlices *kept) {
     State *st = state(h);
     *done = false;
+    *kept = VecSlices{};
     if (k < 1 || nl < 1 || k > kSplitOneMax) return CUOZBLAS_STATUS_SUCCESS;
     const int maxS = h->nSplitMax > 0 ? h->nSplitMax : kMaxSplitDefault;
     const int rho = rho_rule(k, 0);
@@ -538,7 +631,9 @@ int gemv_t_fused(cuozblasHandle_t *h, int nl, int k, const double *A, int lda, c
     Arena ar(h);
     const uint64_t mk = ar.mark();
     double *xs = ar.take<double>((uint64_t)maxS * ldx);
+    const uint64_t mk_xs = ar.mark();
     double *yt = ar.take<double>(nl);
+    int *deep_lines = ar.take<int>(nl);
     // parts of a line in pass 1: enough warps to keep the memory busy
     int parts = 1;
     while (parts < 8 && (int64_t)nl * parts < 48 * sm_count() && k > 512 * parts) parts *= 2;
@@ -555,7 +650,8 @@ int gemv_t_fused(cuozblasHandle_t *h, int nl, int k, const double *A, int lda, c
     OZB_CHECK(cudaMemsetAsync(blk, 0, sizeof(Block), st->stream));
     OZB_TRY(split_vector_one(h, k, x, rho, maxS, xs, ldx, &blk->info));
     counted(h);
-    k_gemv_t_stats<<<(unsigned)(((int64_t)nl * parts * 32 + 255) / 256), 256, 0, st->stream>>>(nl, k, A, lda, parts, stats);
+    k_gemv_t_stats<<<(unsigned)(((int64_t)nl * parts * 32 + 255) / 256), 256, 0, st->stream>>>(nl, k, A, lda, parts,
+                                                                                               &blk->info, stats);
     OZB_CHECK(cudaGetLastError());
     // Warps per line: the fewest rounds of the 16 resident warps per SM over (line part + its reductions).
     int wpr = 1;
@@ -572,19 +668,38 @@ int gemv_t_fused(cuozblasHandle_t *h, int nl, int k, const double *A, int lda, c
     counted(h);
     auto go = [&](auto kern) {
         kern<<<grid, kGtThreads, 0, st->stream>>>(nl, k, A, lda, xs, ldx, &blk->info, rho, maxS, h->sumMode, parts, stats,
-                                                  yt, &blk->st);
+                                                  yt, &blk->st, deep_lines);
     };
     wpr == 1 ? go(k_gemv_t<1>) : wpr == 2 ? go(k_gemv_t<2>) : wpr == 4 ? go(k_gemv_t<4>) : go(k_gemv_t<8>);
     OZB_CHECK(cudaGetLastError());
-    counted(h);
-    k_gemv_t_write<<<(nl + 255) / 256, 256, 0, st->stream>>>(nl, yt, &blk->st, alpha, beta, y);
-    OZB_CHECK(cudaGetLastError());
-    span_end(h);
     Block *hb = reinterpret_cast<Block *>(st->h_ints);
-    OZB_CHECK(cudaMemcpyAsync(hb, blk, sizeof(Block), cudaMemcpyDeviceToHost, st->stream));
-    OZB_CHECK(cudaStreamSynchronize(st->stream));
+    for (int ndeep = 0;; ndeep = hb->st.ndeep) {
+        if (ndeep > 0) {
+            static std::atomic<uint64_t> attr{0};
+            OZB_CHECK(smem_optin((const void *)k_gemv_t_deep, kSplitOneMax * (int)sizeof(double), attr));
+            counted(h);
+            k_gemv_t_deep<<<ndeep, kGtThreads, k * sizeof(double), st->stream>>>(
+                k, A, lda, xs, ldx, &blk->info, rho, maxS, h->sumMode, deep_lines, yt, &blk->st);
+            OZB_CHECK(cudaGetLastError());
+        }
+        counted(h);
+        k_gemv_t_write<<<(nl + 255) / 256, 256, 0, st->stream>>>(nl, yt, &blk->st, ndeep, alpha, beta, y);
+        OZB_CHECK(cudaGetLastError());
+        span_end(h);
+        OZB_CHECK(cudaMemcpyAsync(hb, blk, sizeof(Block), cudaMemcpyDeviceToHost, st->stream));
+        OZB_CHECK(cudaStreamSynchronize(st->stream));
+        if (hb->st.declined || hb->st.ndeep == ndeep) break;
+    }
     ar.release(mk);
-    if (hb->st.declined) return CUOZBLAS_STATUS_SUCCESS;
+    if (hb->st.declined) {
+        // x's slices for the slice path, if that has all the room it can need above them
+        const uint64_t most = sizeof(double) * ((uint64_t)maxS * nl * (k + 1) + 2 * (uint64_t)maxS * maxS * nl) + (1u << 20);
+        if (mk_xs + most <= h->workSizeBytes) {
+            ar.take<double>((uint64_t)maxS * ldx);
+            *kept = VecSlices{xs, ldx, hb->info.ns};
+        }
+        return CUOZBLAS_STATUS_SUCCESS;
+    }
     const int c = (hb->st.zmax < 1 ? 1 : hb->st.zmax) + 1;
     *nA = c < maxS ? c : maxS;
     *nB = hb->info.ns;

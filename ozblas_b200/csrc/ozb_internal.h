@@ -288,8 +288,12 @@ int sum_rows_if_launch(cuozblasHandle_t *h, int m, int nA, int nB, int maxlevel,
                        double beta, double *y, double *scratch, const int *flags, int open);
 int gemv_fused_n(cuozblasHandle_t *h, int m, int n, const double *A, int lda, const double *xs, int ldx, int nB,
                  int rho, int maxS, int fastMode, double alpha, double beta, double *y, int *nA_out);
+struct VecSlices {
+    double *xs = nullptr;  // ns slices of ld doubles
+    int ld = 0, ns = 0;
+};
 int gemv_t_fused(cuozblasHandle_t *h, int nl, int k, const double *A, int lda, const double *x, double alpha,
-                 double beta, double *y, bool *done, int *nA, int *nB);
+                 double beta, double *y, bool *done, int *nA, int *nB, VecSlices *kept);
 int gemv_rn_n(cuozblasHandle_t *h, int m, int n, const double *A, int lda, const double *x, double alpha, double beta,
               double *y, bool *done, int *nA, int *nB);
 
