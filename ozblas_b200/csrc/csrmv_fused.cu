@@ -1437,8 +1437,10 @@ int csrmv_fused(cuozblasHandle_t *h, int m, int n, double alpha, const double *v
             OZB_CHECK(cudaGetLastError());
             nagain = 0;
         } else {
-            int *again = ar.take<int>(nslow);
-            if (ar.ok) {
+            // Rows that one launch with terms in memory takes go there at once: a second launch for
+            // those the certified sum leaves open, be it a few, would take as long as the first.
+            int *again = nslow > kCsrSlowChunk ? ar.take<int>(nslow) : nullptr;
+            if (again) {
                 OZB_CHECK(cudaMemsetAsync(&sc->nslow, 0, sizeof(int), s));
                 counted(h);
                 k_csrmv_slow<2><<<grid, 128, 0, s>>>(nslow, slow, val, colind, rowptr, x, shift, h->splitEpsMode,
@@ -1447,7 +1449,7 @@ int csrmv_fused(cuozblasHandle_t *h, int m, int n, double alpha, const double *v
                 OZB_CHECK(cudaMemcpyAsync(&nagain, &sc->nslow, sizeof(int), cudaMemcpyDeviceToHost, s));
                 OZB_CHECK(cudaStreamSynchronize(s));
                 list = again;
-            } else {  // no room for the list: every row with its terms
+            } else {  // (or no room for the list)
                 ar.ok = true;
             }
         }
