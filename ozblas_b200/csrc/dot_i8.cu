@@ -281,8 +281,8 @@ __global__ void __launch_bounds__(kDiThreads, 1)
         const int wq = __shfl_sync(0xffffffffu, tq >> 5, 0);  // the warp within the group
         const bool lead = tc::elect_one();
         // job k of this group (i = quad + k * kDiQuads), elements in xv / yv;
-        // thread 0 of the group issues the group's MMAs once all its warps
-        // have written the stage (group barrier 1 + quad)
+        // the group's first warp issues the group's MMAs once all its warps
+        // have written the stage (its full barrier)
         auto produce = [&](int k, const double (&xv)[E], const double (&yv)[E]) -> bool {
             const int st = quad * kDiStagesPerQuad + (k & 1);
             // every lane leaves on the same job (the warp collectives below need all lanes)

@@ -705,7 +705,7 @@ int gemv_fused_n(cuozblasHandle_t *h, int m, int n, const double *A, int lda, co
         int *rstate = ar.take<int>((uint64_t)m);
         if (ar.ok) {
             const int rb = (m + 31) / 32, ctiles = (n + kGtCols - 1) / kGtCols;
-            // about eight blocks per SM in all, up to twelve where that fills the last wave
+            // about eight blocks per SM in all, up to fourteen where that fills the last wave
             // of two blocks per SM better (8192 rows: 256 x 8 blocks leave 1 % of it idle, x 5 14 %)
             const int sms = sm_count();
             int gy = (sms * 8 + rb - 1) / rb;
